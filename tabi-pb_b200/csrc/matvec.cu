@@ -2,14 +2,17 @@
 // treecode3d_pb.f:1130-1189) as four device steps:
 //
 //  1. moments   COMP_MS (treecode3d_pb.f:859-916) for every cluster some
-//               target accepts.  The 16 source charges of pb_kernel
-//               (main.f90:664-694) reduce to 4 distinct ones -- A*x2 and
-//               (n_d*A)*x1 -- so 4 raw moment sets are summed, then
-//               weighted by the integer part of der_cof (main.f90:380-399)
-//               into the 16 per-index sets the contraction reads.
-//  2. far       one thread per (target, accepted cluster): the generated
-//               COMP_TCOEFF + COMPP_TREE_PB evaluation (taylor_gen.cuh),
-//               cluster moments staged in shared memory.
+//               target accepts.  FP64: the coefficients of its two harmonic
+//               polynomials per degree (harmonic.cuh).  FP32: the 16 source
+//               charges of pb_kernel (main.f90:664-694) reduce to 4 distinct
+//               ones -- A*x2 and (n_d*A)*x1 -- so 4 raw moment sets are
+//               summed, then weighted by the integer part of der_cof
+//               (main.f90:380-399) into the 16 per-index sets the contraction
+//               reads.
+//  2. far       one thread per (target, accepted cluster), cluster moments
+//               staged in shared memory: COMP_TCOEFF + COMPP_TREE_PB in solid
+//               harmonics (FP64, harmonic.cuh) or as the generated Cartesian
+//               recurrence (FP32, taylor_gen.cuh).
 //  3. near      one thread per (target, near leaf): COMPP_DIRECT_PB
 //               (treecode3d_pb.f:919-1008) over the leaf's faces staged in
 //               shared memory; the target's own face is skipped, which is what
@@ -22,6 +25,8 @@
 #include <algorithm>
 
 #include "bie_kernels.cuh"
+#include "fast_exp.cuh"
+#include "harmonic.cuh"
 #include "reduce.cuh"
 #include "taylor_gen.cuh"
 #include "tabi_impl.cuh"
@@ -93,9 +98,9 @@ __global__ void mom_partial_kernel(const int4* __restrict__ chunks,
   if (own) mraw[((size_t)ch.w * 4 + set) * NT + term] = acc;
 }
 
-template <int P, typename TO>
+template <int P>
 __global__ void mom_final_kernel(const int2* __restrict__ mslot_chunks,
-                                 const double* __restrict__ mraw, TO* __restrict__ mw) {
+                                 const double* __restrict__ mraw, float* __restrict__ mw) {
   constexpr int NT = tabi_nterms(P);
   int slot = blockIdx.x;
   int2 cr = mslot_chunks[slot];
@@ -114,50 +119,216 @@ __global__ void mom_final_kernel(const int2* __restrict__ mslot_chunks,
     double w = 1.0;
     for (int m = 0; m < 3; ++m)
       for (int j = 1; j <= kk[idx][m]; ++j) w *= (double)(kv[m] + j);
-    mw[(size_t)slot * 16 * NT + q] = (TO)(sgn * w * raw);
+    mw[(size_t)slot * 16 * NT + q] = (float)(sgn * w * raw);
+  }
+}
+
+// FP64 moments.  One block per chunk of up to 256 sources of a cluster; a warp
+// takes 32 sources at a time, each thread evaluates one source's
+// contributions to the 2 (p+2)^2 sums into its row of the warp's tile, and the
+// lanes add up the tile's columns.  One evaluation serves all sums: the form
+// with a thread per sum and three staged power factors per source ran
+// 4 C(p+3,3) threads of 7 shared loads a source.
+constexpr int harm_warps(int p) { return p <= 4 ? 4 : 2; }
+constexpr size_t harm_mom_smem(int p) {
+  return sizeof(double) * harm_warps(p) * 32 * (harm_raw(p) + 1);
+}
+
+template <int P>
+__global__ void __launch_bounds__(32 * harm_warps(P)) harm_mom_kernel(
+    const int4* __restrict__ chunks, const int* __restrict__ mslot_node,
+    const double* __restrict__ nd_mid, const double* __restrict__ px,
+    const double* __restrict__ py, const double* __restrict__ pz, const double* __restrict__ nx,
+    const double* __restrict__ ny, const double* __restrict__ nz,
+    const double* __restrict__ area, const double* __restrict__ x, int n,
+    const HarmBeta<P> beta, double eps, double* __restrict__ mraw) {
+  constexpr int NC = harm_raw(P), PITCH = NC + 1, W = harm_warps(P);
+  constexpr int CPL = (NC + 31) / 32;  // columns per lane
+  extern __shared__ double hsm[];
+  const int4 ch = chunks[blockIdx.x];
+  const int node = mslot_node[ch.x];
+  const double mx = nd_mid[3 * node], my = nd_mid[3 * node + 1], mz = nd_mid[3 * node + 2];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double* tile = hsm + warp * 32 * PITCH;
+  double acc[CPL];
+#pragma unroll
+  for (int k = 0; k < CPL; ++k) acc[k] = 0.0;
+  for (int base = 32 * warp; base < ch.z; base += 32 * W) {
+    const int cnt = min(32, ch.z - base);
+    if (lane < cnt) {
+      const int i = ch.y + base + lane;
+      const double A = area[i], x1 = x[i], x2 = x[n + i];
+      // pb_kernel (main.f90:673-681): A*x2 and (n_d*A)*x1
+      harm_source<P>(px[i] - mx, py[i] - my, pz[i] - mz, A * x2, (nx[i] * A) * x1,
+                     (ny[i] * A) * x1, (nz[i] * A) * x1, beta, eps,
+                     tile + lane * PITCH);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < CPL; ++k) {
+      const int c = lane + 32 * k;
+      if (c < NC)
+        for (int q = 0; q < cnt; ++q) acc[k] += tile[q * PITCH + c];
+    }
+    __syncwarp();
+  }
+#pragma unroll
+  for (int k = 0; k < CPL; ++k)
+    if (lane + 32 * k < NC) tile[lane + 32 * k] = acc[k];
+  __syncthreads();
+  for (int c = threadIdx.x; c < NC; c += 32 * W) {
+    double v = hsm[c];
+#pragma unroll
+    for (int w = 1; w < W; ++w) v += hsm[w * 32 * PITCH + c];
+    mraw[(size_t)ch.w * NC + c] = v;
+  }
+}
+
+// one block per cluster: the chunks' sums in order, the constants of (l, m),
+// and the gradients' coefficients, in the order harm_eval reads them
+template <int P>
+__global__ void __launch_bounds__(128) harm_final_kernel(const int2* __restrict__ mslot_chunks,
+                                                         const double* __restrict__ mraw,
+                                                         double* __restrict__ mw) {
+  constexpr int NC = harm_raw(P), NE = (P + 2) * (P + 2);
+  __shared__ double c[NC], sa[(P + 2) * (P + 3) / 2];
+  const int2 cr = mslot_chunks[blockIdx.x];
+  auto degree = [](int e) {
+    int l = 0;
+    while ((l + 1) * (l + 1) <= e) ++l;
+    return l;
+  };
+  for (int q = threadIdx.x; q < (P + 2) * (P + 3) / 2; q += blockDim.x) {
+    int l = 0;
+    while ((l + 1) * (l + 2) / 2 <= q) ++l;
+    sa[q] = harm_a(l, q - l * (l + 1) / 2);
+  }
+  for (int q = threadIdx.x; q < NC; q += blockDim.x) {
+    double raw = 0.0;
+    for (int k = 0; k < cr.y; ++k) raw += mraw[(size_t)(cr.x + k) * NC + q];
+    const int e = q >> 1, l = degree(e), m = (e - l * l + 1) >> 1;
+    c[q] = raw * harm_scale(l, m, q & 1);
+  }
+  __syncthreads();
+  double* out = mw + (size_t)blockIdx.x * harm_size(P);
+  for (int q = threadIdx.x; q < 8 * NE; q += blockDim.x) {
+    const int e = q >> 3, f = q & 7, l = degree(e), r = e - l * l, m = (r + 1) >> 1;
+    const double a = sa[l * (l + 1) / 2 + m];
+    if (l <= P)
+      out[q] = a * (f < 2 ? c[2 * e + f]
+                          : harm_grad(c + (f < 5 ? 0 : 1), l, m, r > 0 && !(r & 1), (f - 2) % 3));
+    else if (f < 2)
+      out[8 * (P + 1) * (P + 1) + 2 * r + f] = a * c[2 * e + f];
   }
 }
 
 // ---- far field
-// T = double: the reference's arithmetic.  T = float (mixed precision): the
-// target-to-centre offset is formed in FP64 and rounded once, the Taylor
-// recurrences and the contraction run in FP32, the result is widened to FP64
-// for the per-target sum.  Order 3 is capped at 128 registers (8 blocks per
-// SM instead of 6 in FP64, for a few bytes of spill).
-template <int P, typename T>
+// FP64 (harmonic.cuh)
+template <int P>
+__global__ void __launch_bounds__(64) far_harm_kernel(
+    const WorkItem* __restrict__ work, const int2* __restrict__ ent,
+    const double* __restrict__ mw, const double* __restrict__ nd_mid,
+    const double* __restrict__ px, const double* __restrict__ py, const double* __restrict__ pz,
+    const double* __restrict__ nx, const double* __restrict__ ny, const double* __restrict__ nz,
+    double kappa, double inv_eps, double2* __restrict__ res) {
+  __shared__ __align__(16) double sm[harm_size(P)];
+  const WorkItem wi = work[blockIdx.x];
+  const double* src = mw + (size_t)wi.mslot * harm_size(P);
+  for (int q = threadIdx.x; q < harm_size(P); q += blockDim.x) sm[q] = src[q];
+  __syncthreads();
+  if ((int)threadIdx.x >= wi.count) return;
+  const int2 e = ent[wi.start + threadIdx.x];
+  const int t = e.x;
+  // COMP_TCOEFF :707-709: target - mid
+  double o1, o2;
+  harm_eval<P>(px[t] - nd_mid[3 * wi.node], py[t] - nd_mid[3 * wi.node + 1],
+               pz[t] - nd_mid[3 * wi.node + 2], nx[t], ny[t], nz[t], kappa, inv_eps, sm, o1, o2);
+  res[e.y] = make_double2(o1 * kOneOver4Pi, o2 * kOneOver4Pi);
+}
+
+// FP32 (mixed precision): the target-to-centre offset is formed in FP64 and
+// rounded once, the Taylor recurrences and the contraction run in FP32, the
+// result is widened to FP64 for the per-target sum.
+template <int P>
 __global__ void __launch_bounds__(64, P == 3 ? 8 : 1) far_kernel(const WorkItem* __restrict__ work,
                                                  const int2* __restrict__ ent,
-                                                 const T* __restrict__ mw,
+                                                 const float* __restrict__ mw,
                                                  const double* __restrict__ nd_mid,
                                                  const double* __restrict__ px,
                                                  const double* __restrict__ py,
                                                  const double* __restrict__ pz,
                                                  const double* __restrict__ nx,
                                                  const double* __restrict__ ny,
-                                                 const double* __restrict__ nz, T kappa,
-                                                 T eps, double2* __restrict__ res) {
+                                                 const double* __restrict__ nz, float kappa,
+                                                 float eps, double2* __restrict__ res) {
   constexpr int NT = tabi_nterms(P);
-  __shared__ T smw[16 * NT];
+  __shared__ float smw[16 * NT];
   WorkItem wi = work[blockIdx.x];
-  const T* src = mw + (size_t)wi.mslot * 16 * NT;
+  const float* src = mw + (size_t)wi.mslot * 16 * NT;
   for (int q = threadIdx.x; q < 16 * NT; q += blockDim.x) smw[q] = src[q];
   __syncthreads();
   if ((int)threadIdx.x >= wi.count) return;
   int2 e = ent[wi.start + threadIdx.x];
   int t = e.x;
   // COMP_TCOEFF :707-709: dx = target - mid
-  T dx = (T)(px[t] - nd_mid[3 * wi.node]);
-  T dy = (T)(py[t] - nd_mid[3 * wi.node + 1]);
-  T dz = (T)(pz[t] - nd_mid[3 * wi.node + 2]);
-  T o1, o2;
-  far_eval<P, T>(dx, dy, dz, kappa, smw, (T)nx[t], (T)ny[t], (T)nz[t], eps, T(1) / eps, o1, o2);
+  float dx = (float)(px[t] - nd_mid[3 * wi.node]);
+  float dy = (float)(py[t] - nd_mid[3 * wi.node + 1]);
+  float dz = (float)(pz[t] - nd_mid[3 * wi.node + 2]);
+  float o1, o2;
+  far_eval<P, float>(dx, dy, dz, kappa, smw, (float)nx[t], (float)ny[t], (float)nz[t], eps,
+                     1.f / eps, o1, o2);
   res[e.y] = make_double2((double)o1 * kOneOver4Pi, (double)o2 * kOneOver4Pi);
 }
 
 // ---- near field
+// FP64: one block per (leaf, up to 128/S of the targets that meet it), S
+// neighbouring threads per target, each over every S-th of the leaf's faces.
+// Bound by the FP64 pipe, so the four kernels are formed as sums over the
+// weighted sources (m = A x1 n, w = A x2, d = r - s, i = 1/|d|,
+// t = (1 + kappa r) e, e = e^{-kappa r}):
+//   y1: i (i^2 (m.d)(1 - eps t) + w (1 - e)),
+//   y2: i^3 ((m.v0 - 3 i^2 (m.d)(v0.d))(t - 1) - kappa^2 (m.d)(v0.d) e
+//            + w (v0.d)(1 - t/eps)),
+// times 1/(4 pi) at the end: 37 FP64 instructions beside the reciprocal root and
+// the exponential (fast_exp.cuh), against 45 of the factored form of each
+// kernel.  Only blocks in which a target meets its own leaf test for the own
+// face.
 constexpr int kNearThreads = 128;
 constexpr int kNearTile = 512;
 
+template <int S, bool OWN>
+__device__ __forceinline__ void near_tile(const double2 (*src)[4], const double* tab, int cnt,
+                                          int self, double tx, double ty, double tz, double vx,
+                                          double vy, double vz, double kappa, double eps,
+                                          double inv_eps, double& p1, double& p2) {
+  const double k2 = kappa * kappa;
+#pragma unroll 2
+  for (int q = (int)threadIdx.x % S; q < cnt; q += S) {
+    const double2 a = src[q][0], b = src[q][1], c = src[q][2], g = src[q][3];
+    double dx = a.x - tx, dy = a.y - ty, dz = b.x - tz;
+    double mx = c.x, my = c.y, mz = g.x, w = b.y;
+    if (OWN && q == self) {  // the own face: no contribution, and no 1/0
+      dx = 1.0;
+      mx = my = mz = w = 0.0;
+    }
+    const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+    const double i = rsqrt(r2), i2 = i * i;
+    const double kr = kappa * (r2 * i);
+    const double e = exp_neg(kr, tab);
+    const double t = fma(kr, e, e);
+    const double md = fma(mx, dx, fma(my, dy, mz * dz));
+    const double vd = fma(vx, dx, fma(vy, dy, vz * dz));
+    const double mv = fma(mx, vx, fma(my, vy, mz * vz));
+    p1 = fma(i, fma(i2 * md, fma(-eps, t, 1.0), fma(-e, w, w)), p1);
+    const double mvd = md * vd;
+    double s = fma(-3.0 * i2, mvd, mv) * (t - 1.0);
+    s = fma(-(k2 * e), mvd, s);
+    s = fma(w * vd, fma(-inv_eps, t, 1.0), s);
+    p2 = fma(i * i2, s, p2);
+  }
+}
+
+template <int S>
 __global__ void __launch_bounds__(kNearThreads) near_kernel(
     const WorkItem* __restrict__ work, const int2* __restrict__ ent,
     const int* __restrict__ nd_ibeg, const int* __restrict__ nd_num,
@@ -166,60 +337,48 @@ __global__ void __launch_bounds__(kNearThreads) near_kernel(
     const double* __restrict__ ny, const double* __restrict__ nz,
     const double* __restrict__ area, const double* __restrict__ x, int n, double kappa,
     double eps, double2* __restrict__ res) {
-  __shared__ double s_x[kNearTile], s_y[kNearTile], s_z[kNearTile];
-  __shared__ double s_nx[kNearTile], s_ny[kNearTile], s_nz[kNearTile];
-  __shared__ double s_w1[kNearTile], s_w2[kNearTile];
-  WorkItem wi = work[blockIdx.x];
-  int ib = nd_ibeg[wi.node], nsrc = nd_num[wi.node];
-  bool own = (int)threadIdx.x < wi.count;
-  int t = 0, slot = 0;
-  double tx = 0, ty = 0, tz = 0, vx = 0, vy = 0, vz = 0;
-  if (own) {
-    int2 e = ent[wi.start + threadIdx.x];
-    t = e.x;
-    slot = e.y;
-    tx = px[t];
-    ty = py[t];
-    tz = pz[t];
-    vx = nx[t];
-    vy = ny[t];
-    vz = nz[t];
-  }
+  // per face: (x, y), (z, A x2), (A x1 n_x, A x1 n_y), (A x1 n_z, -)
+  __shared__ double2 src[kNearTile][4];
+  __shared__ double tab[kExpTab];
+  exp_table_fill(tab);
+  const WorkItem wi = work[blockIdx.x];
+  const int ib = nd_ibeg[wi.node], nsrc = nd_num[wi.node];
+  const int k = (int)threadIdx.x / S;
+  const bool own = k < wi.count;
+  const int2 ent_k = ent[wi.start + min(k, wi.count - 1)];
+  const int t = ent_k.x;
+  const double tx = px[t], ty = py[t], tz = pz[t], vx = nx[t], vy = ny[t], vz = nz[t];
+  const bool meets_own = __syncthreads_or(t >= ib && t < ib + nsrc);
   const double inv_eps = 1.0 / eps;
   double p1 = 0.0, p2 = 0.0;
   for (int b0 = 0; b0 < nsrc; b0 += kNearTile) {
-    int cnt = min(kNearTile, nsrc - b0);
-    __syncthreads();
-    for (int q = threadIdx.x; q < cnt; q += blockDim.x) {
-      int j = ib + b0 + q;
-      s_x[q] = px[j];
-      s_y[q] = py[j];
-      s_z[q] = pz[j];
-      s_nx[q] = nx[j];
-      s_ny[q] = ny[j];
-      s_nz[q] = nz[j];
-      double A = area[j];
-      s_w1[q] = A * x[j];
-      s_w2[q] = A * x[n + j];
+    const int cnt = min(kNearTile, nsrc - b0);
+    if (b0 > 0) __syncthreads();
+    for (int q = threadIdx.x; q < cnt; q += kNearThreads) {
+      const int j = ib + b0 + q;
+      const double A = area[j], w1 = A * x[j];
+      src[q][0] = make_double2(px[j], py[j]);
+      src[q][1] = make_double2(pz[j], A * x[n + j]);
+      src[q][2] = make_double2(w1 * nx[j], w1 * ny[j]);
+      src[q][3] = make_double2(w1 * nz[j], 0.0);
     }
     __syncthreads();
     if (own) {
-      int self = t - (ib + b0);
-#pragma unroll 2
-      for (int q = 0; q < cnt; ++q) {
-        bool skip = (q == self);
-        double dx = s_x[q] - tx, dy = s_y[q] - ty, dz = s_z[q] - tz;
-        if (skip) dx = 1.0;  // keeps the skipped pair finite
-        double K1, K2, K3, K4;
-        bie4<double>(dx, dy, dz, vx, vy, vz, s_nx[q], s_ny[q], s_nz[q], kappa, eps, inv_eps, K1,
-                     K2, K3, K4);
-        double w1 = skip ? 0.0 : s_w1[q], w2 = skip ? 0.0 : s_w2[q];
-        p1 = fma(K1, w1, fma(K2, w2, p1));
-        p2 = fma(K3, w1, fma(K4, w2, p2));
-      }
+      if (meets_own)
+        near_tile<S, true>(src, tab, cnt, t - (ib + b0), tx, ty, tz, vx, vy, vz, kappa, eps,
+                           inv_eps, p1, p2);
+      else
+        near_tile<S, false>(src, tab, cnt, 0, tx, ty, tz, vx, vy, vz, kappa, eps, inv_eps, p1,
+                            p2);
     }
   }
-  if (own) res[slot] = make_double2(p1, p2);
+#pragma unroll
+  for (int o = S / 2; o > 0; o >>= 1) {
+    p1 += __shfl_xor_sync(0xffffffffu, p1, o);
+    p2 += __shfl_xor_sync(0xffffffffu, p2, o);
+  }
+  if (own && threadIdx.x % S == 0)
+    res[ent_k.y] = make_double2(p1 * kOneOver4Pi, p2 * kOneOver4Pi);
 }
 
 // Mixed-precision near field.  Each face's position relative to the centre of
@@ -346,22 +505,30 @@ void launch_moments(Handle& H, const double* x, bool f32, cudaStream_t s) {
   Tree& T = H.tree;
   constexpr int NT = tabi_nterms(P);
   if (T.nmslot == 0) return;
-  int nch = 0;
-  for (int k = 0; k < T.nmslot; ++k) nch += T.mslot_nchunk[k];
-  int threads = ((4 * NT + 31) / 32) * 32;
+  const int nch = T.mslot_chunk0.back() + T.mslot_nchunk.back();
+  if (f32) {
+    int threads = ((4 * NT + 31) / 32) * 32;
+    {
+      TABI_K(K_MOMENTS, s);
+      mom_partial_kernel<P><<<nch, threads, 0, s>>>(
+          T.d_mchunks.p, T.d_mslot_node.p, T.d_mid.p, H.d_x.p, H.d_y.p, H.d_z.p, H.d_nx.p,
+          H.d_ny.p, H.d_nz.p, H.d_area.p, x, H.n, H.d_mraw.p);
+    }
+    TABI_K(K_MOMENTS, s);
+    mom_final_kernel<P><<<T.nmslot, 256, 0, s>>>(T.d_mslot_chunks.p, H.d_mraw.p, H.d_mwf.p);
+    return;
+  }
+  if (harm_mom_smem(P) > 48 * 1024)
+    raise_smem_limit((const void*)harm_mom_kernel<P>, harm_mom_smem(P));
   {
     TABI_K(K_MOMENTS, s);
-    mom_partial_kernel<P><<<nch, threads, 0, s>>>(T.d_mchunks.p, T.d_mslot_node.p, T.d_mid.p,
-                                                  H.d_x.p, H.d_y.p, H.d_z.p, H.d_nx.p, H.d_ny.p,
-                                                  H.d_nz.p, H.d_area.p, x, H.n, H.d_mraw.p);
+    harm_mom_kernel<P><<<nch, 32 * harm_warps(P), harm_mom_smem(P), s>>>(
+        T.d_mchunks.p, T.d_mslot_node.p, T.d_mid.p, H.d_x.p, H.d_y.p, H.d_z.p, H.d_nx.p,
+        H.d_ny.p, H.d_nz.p, H.d_area.p, x, H.n, harm_beta<P>(H.prm.kappa),
+        H.prm.eps1 / H.prm.eps0, H.d_mraw.p);
   }
   TABI_K(K_MOMENTS, s);
-  if (f32)
-    mom_final_kernel<P, float><<<T.nmslot, 256, 0, s>>>(T.d_mslot_chunks.p, H.d_mraw.p,
-                                                          H.d_mwf.p);
-  else
-    mom_final_kernel<P, double><<<T.nmslot, 256, 0, s>>>(T.d_mslot_chunks.p, H.d_mraw.p,
-                                                           H.d_mw.p);
+  harm_final_kernel<P><<<T.nmslot, 128, 0, s>>>(T.d_mslot_chunks.p, H.d_mraw.p, H.d_mw.p);
 }
 
 template <int P>
@@ -374,13 +541,13 @@ void launch_far(Handle& H, bool f32, cudaStream_t s) {
   const double eps = H.prm.eps1 / H.prm.eps0;
   TABI_K(K_FAR, s);
   if (f32)
-    far_kernel<P, float><<<nw, 64, 0, s>>>(
+    far_kernel<P><<<nw, 64, 0, s>>>(
         fw, fe, H.d_mwf.p, T.d_mid.p, H.d_x.p, H.d_y.p, H.d_z.p,
         H.d_nx.p, H.d_ny.p, H.d_nz.p, (float)H.prm.kappa, (float)eps, H.d_res.p);
   else
-    far_kernel<P, double><<<nw, 64, 0, s>>>(
+    far_harm_kernel<P><<<nw, 64, 0, s>>>(
         fw, fe, H.d_mw.p, T.d_mid.p, H.d_x.p, H.d_y.p, H.d_z.p,
-        H.d_nx.p, H.d_ny.p, H.d_nz.p, H.prm.kappa, eps, H.d_res.p);
+        H.d_nx.p, H.d_ny.p, H.d_nz.p, H.prm.kappa, 1.0 / eps, H.d_res.p);
 }
 
 // FP32 copies of the faces relative to their leaf centres (once per tree)
@@ -433,6 +600,14 @@ double nrm2_dev(Handle& H, const double* a, int n, cudaStream_t s) {
   return sqrt(reduce_dev(H, 2, a, nullptr, n, s));
 }
 
+void alloc_moments(Handle& H, int nchunk) {
+  const int p = H.prm.order, nslot = H.tree.nmslot;
+  const bool mixed = H.prm.precision == TABI_PREC_MIXED;
+  H.d_mraw.alloc((size_t)nchunk * std::max(harm_raw(p), mixed ? 4 * tabi_nterms(p) : 0));
+  H.d_mw.alloc((size_t)nslot * harm_size(p));
+  if (mixed) H.d_mwf.alloc((size_t)nslot * 16 * tabi_nterms(p));
+}
+
 void matvec_dev(Handle& H, const double* x, double* y, cudaStream_t s, bool check_zero) {
   const int n = H.n;
   if (check_zero) {
@@ -446,10 +621,7 @@ void matvec_dev(Handle& H, const double* x, double* y, cudaStream_t s, bool chec
   }
   Tree& T = H.tree;
   const bool f32 = H.mv_prec == TABI_PREC_MIXED;
-  if (f32) {
-    prepare_f32(H, s);
-    if (T.nmslot > 0) H.d_mwf.alloc(H.d_mw.n);
-  }
+  if (f32) prepare_f32(H, s);
   TABI_PHASE(K_PHASE_MATVEC, s);
   // the near field runs on the handle's side stream, concurrently with the
   // moments + far field on s; both write disjoint result slots
@@ -483,10 +655,18 @@ void matvec_dev(Handle& H, const double* x, double* y, cudaStream_t s, bool chec
         (float)(H.prm.eps1 / H.prm.eps0), H.d_res.p);
   } else if (nnw > 0) {
     TABI_K(K_NEAR, sn);
-    near_kernel<<<nnw, kNearThreads, 0, sn>>>(
-        nwk, nent, T.d_ibeg.p, T.d_num.p, H.d_x.p, H.d_y.p, H.d_z.p,
-        H.d_nx.p, H.d_ny.p, H.d_nz.p, H.d_area.p, x, n, H.prm.kappa, H.prm.eps1 / H.prm.eps0,
-        H.d_res.p);
+    auto launch = [&](auto* kernel) {
+      kernel<<<nnw, kNearThreads, 0, sn>>>(
+          nwk, nent, T.d_ibeg.p, T.d_num.p, H.d_x.p, H.d_y.p, H.d_z.p, H.d_nx.p, H.d_ny.p,
+          H.d_nz.p, H.d_area.p, x, n, H.prm.kappa, H.prm.eps1 / H.prm.eps0, H.d_res.p);
+    };
+    switch (T.near_split) {
+      case 1: launch(near_kernel<1>); break;
+      case 2: launch(near_kernel<2>); break;
+      case 4: launch(near_kernel<4>); break;
+      case 8: launch(near_kernel<8>); break;
+      default: launch(near_kernel<16>); break;
+    }
   }
   switch (H.prm.order) {
     case 1: launch_far<1>(H, f32, s); break;

@@ -199,6 +199,7 @@ struct Tree {
   DBuf<int2> d_near_ent;       // (target, slot) grouped by leaf
   PinVec<WorkItem> far_work, near_work;  // page-locked: uploaded per tree
   DBuf<WorkItem> d_far_work, d_near_work;
+  int near_split = 1;  // threads per target of the FP64 near field (near_work's chunks)
   int nmslot = 0;
   std::vector<int> mslot_node;  // node id per moment slot
   DBuf<int> d_mslot_node;
@@ -351,8 +352,8 @@ struct Handle {
   Tree tree;
   // matvec scratch
   DBuf<double> d_mraw;    // moment partials
-  DBuf<double> d_mw;      // weighted moments, 16 x NT per slot
-  DBuf<float> d_mwf;      // the same in FP32 (mixed-precision far field)
+  DBuf<double> d_mw;      // per cluster the far field's harmonic coefficients (harmonic.cuh)
+  DBuf<float> d_mwf;      // weighted Cartesian moments, 16 x NT (mixed-precision far field)
   int mv_prec = TABI_PREC_FP64;  // arithmetic of the treecode operator
   DBuf<double2> d_res;    // per-slot interaction results
   DBuf<double2> d_dirpart;  // direct-sum partials (accuracy reference)
@@ -437,6 +438,8 @@ void energy_dev(Handle& H, int nchr, const double* chrpos, const double* atmchr,
 void build_tree(Handle& H, cudaStream_t s);
 void build_lists(Handle& H, cudaStream_t s);
 // matvec (matvec.cu)
+// moment scratch for the tree's nmslot clusters and nchunk source chunks
+void alloc_moments(Handle& H, int nchunk);
 void matvec_dev(Handle& H, const double* x, double* y, cudaStream_t s, bool check_zero);
 // restricts matvec_dev / msolve_dev to the leaf-aligned target range [t0, t1)
 // of the tree order (the whole range lifts the restriction)

@@ -665,7 +665,13 @@ void build_lists(Handle& H, cudaStream_t s) {
       T.d_rad.p, H.prm.theta, nullptr, nullptr, nullptr, T.d_slot_off.p, d_foff.p, d_noff.p,
       far_cnt.p, near_cnt.p, T.d_far_ent.p, T.d_near_ent.p, H.d_err.p); }
   // work items and moment slots
-  const int kFarChunk = 64, kNearChunk = 128, kMomChunk = 256;
+  const int kFarChunk = 64, kMomChunk = 256;
+  // threads per target of the FP64 near field, as few as give every SM 8 blocks
+  // of 128 threads (the FP32 one keeps a thread per target)
+  T.near_split = 1;
+  if (H.prm.precision == TABI_PREC_FP64)
+    while (T.near_split < 16 && tn * T.near_split < 148LL * 8 * 128) T.near_split *= 2;
+  const int near_chunk = 128 / T.near_split;
   T.far_work.clear();
   T.near_work.clear();
   T.mslot_node.clear();
@@ -685,11 +691,15 @@ void build_lists(Handle& H, cudaStream_t s) {
       for (int st = 0; st < hf[c]; st += kFarChunk)
         T.far_work.push_back({c, (int)(foff[c] + st), std::min(kFarChunk, hf[c] - st), slot});
     }
-    if (hn[c] > 0)
-      for (int st = 0; st < hn[c]; st += kNearChunk)
-        T.near_work.push_back({c, (int)(noff[c] + st), std::min(kNearChunk, hn[c] - st),
-                               T.ibeg[c]});
   }
+  // near field: largest leaves first, so that the last blocks to run are short
+  std::vector<int> by_size(T.leaves);
+  std::stable_sort(by_size.begin(), by_size.end(),
+                   [&](int a, int b) { return T.num[a] > T.num[b]; });
+  for (int c : by_size)
+    for (int st = 0; st < hn[c]; st += near_chunk)
+      T.near_work.push_back({c, (int)(noff[c] + st), std::min(near_chunk, hn[c] - st),
+                             T.ibeg[c]});
   T.nmslot = (int)T.mslot_node.size();
   T.d_far_work.alloc(std::max<size_t>(T.far_work.size(), 1));
   T.d_near_work.alloc(std::max<size_t>(T.near_work.size(), 1));
@@ -714,8 +724,7 @@ void build_lists(Handle& H, cudaStream_t s) {
   TABI_REQUIRE(herr == 0, TABI_ERR_LIMIT, "tree traversal stack overflow");
   // scratch sized for the lists
   H.d_res.alloc(std::max<int64_t>(T.n_slots, 1));
-  H.d_mraw.alloc(std::max<size_t>(mch.size(), 1) * 4 * 165);
-  H.d_mw.alloc(std::max(T.nmslot, 1) * (size_t)16 * 165);
+  alloc_moments(H, (int)mch.size());
 }
 
 }  // namespace tabi
