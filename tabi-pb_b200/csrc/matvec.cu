@@ -292,7 +292,9 @@ __global__ void __launch_bounds__(64, P == 3 ? 8 : 1) far_kernel(const WorkItem*
 // times 1/(4 pi) at the end: 37 FP64 instructions beside the reciprocal root and
 // the exponential (fast_exp.cuh), against 45 of the factored form of each
 // kernel.  Only blocks in which a target meets its own leaf test for the own
-// face.
+// face.  Measured beside the far field, 73.5 M pairs: 0.50 -> 0.32 ms; 193 M
+// pairs: 1.36 -> 0.90 ms; 0.55 M pairs (1,272 targets, one thread each gave 27
+// blocks): 49 -> 20 us.
 constexpr int kNearThreads = 128;
 constexpr int kNearTile = 512;
 
