@@ -1216,14 +1216,17 @@ __global__ void __launch_bounds__(NT, (NT <= 256 ? 4 : 1)) solve_kernel(
 // blocks of a well-resolved surface are strongly diagonal (the 2n x 2n blocks
 // of the benchmark molecule have condition numbers near 100 and no row
 // interchange at all), so the factorisation runs first without pivot
-// searches, as a right-looking blocked LU in 64-column steps:
-//   lu_np_diag_kernel   the 64 x 64 diagonal block of every leaf, factored in
-//                       shared memory, with the inverses of its L and U
-//                       (kept for the panels, and their 32 x 32 diagonal
-//                       blocks for the applies);
-//   lu_np_panel_kernel  L21 = A21 U11^{-1} by 64-row chunks and
-//                       U12 = L11^{-1} A12 by 64-column chunks;
-//   lu_gemm2_kernel     A22 -= L21 U12, 64 deep.
+// searches, right-looking in outer blocks of 256 columns, three launches each
+// over all leaves of a group:
+//   lu_np_block_kernel   the 256 x 256 diagonal block of every leaf, one CTA
+//                        each, in four 64-column steps, with the inverses of
+//                        the 64 x 64 diagonal blocks' L and U (and their
+//                        32 x 32 diagonal blocks for the applies);
+//   lu_np_border_kernel  the block's L21 = A21 U11^{-1} by 64-row chunks and
+//                        U12 = L11^{-1} A12 by 64-column chunks: each chunk's
+//                        four 64-deep steps depend on no other chunk, so one
+//                        CTA takes them all from shared memory;
+//   lu_gemm2_kernel      A22 -= L21 U12, 256 deep.
 // Every multiplier l is checked: |l| <= 1 - 2^-20 for all of them certifies
 // that partial pivoting (on these values or on the reference's, which differ
 // by rounding only) keeps the diagonal row at every column, so the factors
@@ -1231,54 +1234,109 @@ __global__ void __launch_bounds__(NT, (NT <= 256 ? 4 : 1)) solve_kernel(
 // near tie, a zero or non-finite pivot) is re-assembled and factored again by
 // the pivoted kernels above.
 constexpr int kNP = 64;    // step width
-constexpr int kNPT = 256;  // threads of the diagonal and panel kernels
-constexpr int kNPPitch = kNP + 1;
+constexpr int kNPT = 256;  // threads of the block and border kernels
+constexpr int kOB2 = 256;  // outer block
+constexpr int kPP = kNP + 4;  // pitch of a staged 64-double column
+constexpr int kNB2 = kNP * kPP;  // a staged 64 x 64 block
 constexpr double kNoPivBound = 1.0 - 1.0 / 1048576.0;
-constexpr size_t kNPDiagSmem = sizeof(double) * 3 * kNP * kNPPitch;
-constexpr size_t kNPPanelSmem = sizeof(double) * 2 * kNP * kNPPitch;
 
-// Per leaf (leaves[blockIdx.x]) with m > k0: D = A[k0:k0+d, k0:k0+d], d =
-// min(64, m - k0), factored in place without interchanges (DGETRF2's scaling:
-// multipliers times the pivot's reciprocal); scr receives L^{-1} (unit lower,
-// column-major) and U^{-1} (row-major) of D, 64 x 64 each with zeros outside
-// the triangle and from d on, and dinv the 32 x 32 diagonal blocks of both
-// (identity padded, the layout lu_diaginv_kernel writes).  The block, L^{-1}
-// and U^{-1} live in registers on a 16 x 16 thread grid; one loop of d
-// steps with one barrier each factors the block and forms both inverses
-// (the loop's comment gives the scheme).  Every entry of the factors takes
-// the same sequence of updates as in a column-by-column DGETF2 order.
-// one double into shared memory, asynchronously (zero when !valid)
-__device__ __forceinline__ void cp_async8(double* dst, const double* src, bool valid) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src),
-               "r"(valid ? 8 : 0));
+// FP64 tensor-core product of 8 x 8 x 4 (tcgen05 has no FP64 kind; this one runs
+// at the FP64 pipe's full rate, 37.05 TFLOP/s measured against 36.7 of a DFMA
+// loop, with an eighth of the instructions and shared loads).  Lane l holds
+// A[l / 4][l % 4], B[l % 4][l / 4] and C[l / 4][2 (l % 4) + {0, 1}].
+__device__ __forceinline__ void dmma884(double (&c)[2], double a, double b) {
+  asm volatile(
+      "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(c[0]), "+d"(c[1])
+      : "d"(a), "d"(b));
 }
 
-__global__ void __launch_bounds__(kNPT) lu_np_diag_kernel(
-    const int* __restrict__ leaves, int k0, const int2* __restrict__ leaf_rng,
-    const int64_t* __restrict__ blk_off, const int64_t* __restrict__ dinv_off,
-    double* __restrict__ lu, double* __restrict__ dinv, double* __restrict__ scr,
-    int* __restrict__ fail) {
-  extern __shared__ double nsm[];
-  chain_wait();  // the previous launch of the chain has finished
-  chain_signal();
-  double(*D)[kNPPitch] = reinterpret_cast<double(*)[kNPPitch]>(nsm);
-  double(*Li)[kNPPitch] = reinterpret_cast<double(*)[kNPPitch]>(nsm + kNP * kNPPitch);
-  double(*Ui)[kNPPitch] = reinterpret_cast<double(*)[kNPPitch]>(nsm + 2 * kNP * kNPPitch);
-  const int leaf = leaves[blockIdx.x];
-  const int m = 2 * leaf_rng[leaf].y;
-  const int d = min(kNP, m - k0);
-  double* A = lu + blk_off[leaf];
-  const int tid = threadIdx.x;
-  for (int e = tid; e < kNP * kNP; e += kNPT) {
-    const int c = e >> 6, r = e & 63;
-    cp_async8(&D[r][c], A + (size_t)(k0 + min(c, d - 1)) * m + k0 + min(r, d - 1),
-              r < d && c < d);
+// acc += A B for a warp's (8 MT) x (8 NT) tile over KD (a multiple of 4): A
+// k-major (row r, depth k at A[k * AP + r]), B by column (depth k, column c at
+// B[c * BP + k]).  A pitch of 4 modulo 16 doubles puts the 16 words of a
+// half-warp's fragment load on 16 different bank pairs.
+template <int MT, int NT, int AP, int BP, int KD>
+__device__ __forceinline__ void dmma_tile(double (&acc)[MT][NT][2], const double* A,
+                                          const double* B) {
+  static_assert(AP % 16 == 4 && BP % 16 == 4, "fragment loads on different banks");
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const double* a = A + t * AP + g;
+  const double* b = B + g * BP + t;
+#pragma unroll
+  for (int k = 0; k < KD; k += 4) {
+    double av[MT], bv[NT];
+#pragma unroll
+    for (int i = 0; i < MT; ++i) av[i] = a[k * AP + 8 * i];
+#pragma unroll
+    for (int i = 0; i < NT; ++i) bv[i] = b[8 * i * BP + k];
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+      for (int q = 0; q < NT; ++q) dmma884(acc[i][q], av[i], bv[q]);
   }
-  asm volatile("cp.async.commit_group;\n" ::);
-  __shared__ double s_rcp[kNP];  // reciprocal of each pivot
-  __shared__ double s_row[2][kNP], s_col[2][kNP], s_xrow[2][kNP], s_zcol[2][kNP];
-  asm volatile("cp.async.wait_group 0;\n" ::);
+}
+
+// Copies a block of 64 columns of 64 doubles (leading dimension ld, 16-byte
+// aligned columns) into shared memory at pitch kPP, zeros outside nr x nc (nr
+// even); the caller commits and waits.
+__device__ __forceinline__ void stage64(double* dst, const double* src, int ld, int nr, int nc) {
+#pragma unroll
+  for (int e = 0; e < kNP * kNP / 2 / kNPT; ++e) {
+    const int q = (int)threadIdx.x + kNPT * e, c = q >> 5, r = 2 * (q & 31);
+    const bool ok = c < nc && r < nr;
+    cp_async16(dst + c * kPP + r, ok ? src + (size_t)c * ld + r : src, ok);
+  }
+}
+
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
+}
+
+// A warp's 32 x 16 tile of a 64 x 64 product: rows tile_r0().., columns
+// tile_c0().., and f(r, c, entry) over the lane's entries of it
+__device__ __forceinline__ int tile_r0() { return 32 * ((int)(threadIdx.x >> 5) & 1); }
+__device__ __forceinline__ int tile_c0() { return 16 * (int)(threadIdx.x >> 6); }
+template <typename F>
+__device__ __forceinline__ void tile_each(double (&acc)[4][2][2], F&& f) {
+  const int r = tile_r0() + ((int)(threadIdx.x & 31) >> 2);
+  const int c = tile_c0() + 2 * ((int)threadIdx.x & 3);
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+      for (int b = 0; b < 2; ++b) f(r + 8 * i, c + 8 * q + b, acc[i][q][b]);
+}
+
+// The d x d (d <= 64) diagonal block at D (column-major, leading dimension m)
+// factored in place without interchanges (DGETRF2's scaling: multipliers
+// times the pivot's reciprocal).  li and ui (shared, pitch kPP) receive
+// L^{-1} (unit lower) and U^{-1}, column-major with zeros outside the triangle
+// and from d on; S the same at pitch 64; Di their 32 x 32 diagonal blocks
+// (identity padded, the layout lu_diaginv_kernel writes).  fb: shared scratch
+// of one staged block.  Every thread of the CTA; true if the certificate
+// failed in an entry of this thread.  The block, L^{-1} and U^{-1} live in
+// registers on a 16 x 16 thread grid; one loop of d steps with one barrier each
+// factors the block and forms both inverses.  Every entry of the factors takes
+// the same sequence of updates as in a column-by-column DGETF2 order.
+struct DiagShared {
+  double rcp[kNP];  // reciprocal of each pivot
+  double row[2][kNP], col[2][kNP], xrow[2][kNP], zcol[2][kNP];
+};
+
+__device__ bool lu_diag64(double* D, int m, int d, double* li, double* ui, double* fb,
+                          DiagShared& sh, double* S, double* Di) {
+  const int tid = threadIdx.x;
+  auto& s_rcp = sh.rcp;
+  auto& s_row = sh.row;
+  auto& s_col = sh.col;
+  auto& s_xrow = sh.xrow;
+  auto& s_zcol = sh.zcol;
+  stage64(fb, D, m, d, d);
+  cp_async_commit();
+  cp_async_wait<0>();
   __syncthreads();
   // Thread (tx, ty) of a 16 x 16 grid holds rows ty + 16p and columns
   // tx + 16q (p, q < 4) of the block in registers, and of X = L^{-1} and
@@ -1312,7 +1370,7 @@ __global__ void __launch_bounds__(kNPT) lu_np_diag_kernel(
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int i = ty + 16 * p, c = tx + 16 * q;
-      a[p][q] = D[i][c];
+      a[p][q] = fb[c * kPP + i];
       x[p][q] = z[p][q] = (i == c && i < d) ? 1.0 : 0.0;
     }
   auto pivot_rcp = [&](int j, double pk) {  // by the holder of entry (j, j)
@@ -1391,24 +1449,17 @@ __global__ void __launch_bounds__(kNPT) lu_np_diag_kernel(
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int i = ty + 16 * p, c = tx + 16 * q;
-      D[i][c] = a[p][q];
-      Li[i][c] = x[p][q];
-      Ui[i][c] = z[p][q];
+      fb[c * kPP + i] = a[p][q];
+      li[c * kPP + i] = x[p][q];
+      ui[c * kPP + i] = z[p][q];
     }
   __syncthreads();
-  // factors back
-  for (int e = tid; e < d * d; e += kNPT) {
-    const int c = e / d, r = e - c * d;
-    A[(size_t)(k0 + c) * m + k0 + r] = D[r][c];
-  }
-  if (__syncthreads_or(bad) && tid == 0) fail[leaf] = 1;
-  double* S = scr + (size_t)blockIdx.x * 2 * kNP * kNP;
   for (int e = tid; e < kNP * kNP; e += kNPT) {
-    const int hi = e / kNP, lo = e - hi * kNP;
-    S[e] = Li[lo][hi];            // column-major L^{-1}
-    S[kNP * kNP + e] = Ui[hi][lo];  // row-major U^{-1}
+    const int c = e >> 6, r = e & 63;
+    if (c < d && r < d) D[(size_t)c * m + r] = fb[c * kPP + r];
+    S[e] = li[c * kPP + r];
+    S[kNP * kNP + e] = ui[c * kPP + r];
   }
-  double* Di = dinv + dinv_off[leaf] + (size_t)(k0 / kDB) * 2 * kDB * kDB;
   for (int b = 0; b * kDB < d; ++b) {
     const int nb = min(kDB, d - b * kDB), o = b * kDB;
     double* Lb = Di + (size_t)b * 2 * kDB * kDB;
@@ -1416,172 +1467,284 @@ __global__ void __launch_bounds__(kNPT) lu_np_diag_kernel(
     for (int e = tid; e < kDB * kDB; e += kNPT) {
       const int c = e / kDB, r = e - c * kDB;
       const double id = r == c ? 1.0 : 0.0;
-      Lb[e] = (r < nb && c < nb) ? Li[o + r][o + c] : id;
-      Ub[e] = (r < nb && c < nb) ? Ui[o + r][o + c] : id;
+      Lb[e] = (r < nb && c < nb) ? li[(o + c) * kPP + o + r] : id;
+      Ub[e] = (r < nb && c < nb) ? ui[(o + c) * kPP + o + r] : id;
     }
   }
+  return bad;
 }
 
-// item = (leaf, slot, kind, off): kind 0, rows [off, off + 64) of the step's
-// column panel: L21 = A21 U11^{-1}, each multiplier checked; kind 1, columns
-// [off, off + 64) of its row panel: U12 = L11^{-1} A12.  slot = the leaf's
-// row in the diagonal kernel's launch (its scratch).  A 64 x 64 x 64 product
-// out = P Q from shared memory, 4 x 4 outputs per thread (rows tr + 16 a,
-// columns tc + 16 b: P loads on 16 consecutive rows, Q loads broadcast).
-__global__ void __launch_bounds__(kNPT) lu_np_panel_kernel(
-    const int4* __restrict__ items, int k0, const int2* __restrict__ leaf_rng,
-    const int64_t* __restrict__ blk_off, double* __restrict__ lu,
-    const double* __restrict__ scr, int* __restrict__ fail) {
-  extern __shared__ double nsm[];
+// Per leaf (leaves[blockIdx.x]) with m > K0: the diagonal block A[K0:K0+D,
+// K0:K0+D], D = min(256, m - K0), factored in place; scr and dinv receive the
+// inverses of its 64 x 64 diagonal blocks (see lu_diag64).  Step j: the
+// diagonal block, L_ij = A_ij U_jj^{-1} (multipliers checked), and per block
+// column k U_jk = L_jj^{-1} A_jk and A_ik -= L_ij U_jk, all as 64 x 64 x 64
+// products on the FP64 tensor cores from three staged blocks (104 KB, so two
+// CTAs, or one and an update's, share an SM and fill each other's waits).
+// One CTA for the whole block: the step's 64-column launches over all leaves
+// that it replaces (diagonal, panel, update: 50 + 60 + 70 us each, four per
+// outer block) streamed every leaf's 256 columns from HBM each time and left
+// the SMs waiting between them.
+constexpr size_t kNPBlockSmem = sizeof(double) * 3 * kNB2;
+
+__global__ void __launch_bounds__(kNPT, 2) lu_np_block_kernel(
+    const int* __restrict__ leaves, int K0, const int2* __restrict__ leaf_rng,
+    const int64_t* __restrict__ blk_off, const int64_t* __restrict__ dinv_off, double* lu,
+    double* __restrict__ dinv, double* __restrict__ scr, int* __restrict__ fail) {
+  extern __shared__ __align__(16) double nsm[];
+  __shared__ DiagShared sh;
   chain_wait();  // the previous launch of the chain has finished
   chain_signal();
-  double(*X)[kNPPitch] = reinterpret_cast<double(*)[kNPPitch]>(nsm);
-  double(*V)[kNPPitch] = reinterpret_cast<double(*)[kNPPitch]>(nsm + kNP * kNPPitch);
-  const int4 it = items[blockIdx.x];
-  const int leaf = it.x, kind = it.z, off = it.w;
-  const int m = 2 * leaf_rng[leaf].y;
-  const int d = min(kNP, m - k0);
-  const int cnt = min(kNP, m - off);
-  double* A = lu + blk_off[leaf];
-  const double* S = scr + (size_t)it.y * 2 * kNP * kNP + (kind == 0 ? kNP * kNP : 0);
-  const int tid = threadIdx.x, tr = tid & 15, tc = tid >> 4;
-  // V = the inverse as [row][col]: U^{-1} (row-major in scr) for kind 0,
-  // L^{-1} (column-major in scr) for kind 1; zeros outside d x d
-  for (int e = tid; e < kNP * kNP; e += kNPT) {
-    const int hi = e >> 6, lo = e & 63;
-    cp_async8(kind == 0 ? &V[hi][lo] : &V[lo][hi], S + e, true);
-  }
-  if (kind == 0) {  // X[i][q] = A[off + i, k0 + q]
-    for (int e = tid; e < kNP * kNP; e += kNPT) {
-      const int q = e >> 6, i = e & 63;
-      const bool ok = i < cnt && q < d;
-      cp_async8(&X[i][q], ok ? A + (size_t)(k0 + q) * m + off + i : A, ok);
-    }
-  } else {          // X[q][c] = A[k0 + q, off + c]
-    for (int e = tid; e < kNP * kNP; e += kNPT) {
-      const int c = e >> 6, q = e & 63;
-      const bool ok = c < cnt && q < d;
-      cp_async8(&X[q][c], ok ? A + (size_t)(off + c) * m + k0 + q : A, ok);
-    }
-  }
-  asm volatile("cp.async.commit_group;\n" ::);
-  asm volatile("cp.async.wait_group 0;\n" ::);
-  __syncthreads();
-  // kind 0: out = X V (P = X, Q = V); kind 1: out = V X (P = V, Q = X)
-  const double(*P)[kNPPitch] = kind == 0 ? X : V;
-  const double(*Q)[kNPPitch] = kind == 0 ? V : X;
-  double acc[4][4];
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b) acc[a][b] = 0.0;
-#pragma unroll 4
-  for (int q = 0; q < d; ++q) {
-    double pv[4], qv[4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a) pv[a] = P[tr + 16 * a][q];
-#pragma unroll
-    for (int b = 0; b < 4; ++b) qv[b] = Q[q][tc + 16 * b];
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) acc[a][b] = fma(pv[a], qv[b], acc[a][b]);
-  }
+  double* b0 = nsm;              // L_jj^{-1}
+  double* b1 = nsm + kNB2;       // U_jj^{-1}, then U_jk
+  double* b2 = nsm + 2 * kNB2;   // A_ij, then L_ij
+  const int leaf = leaves[blockIdx.x];
+  const int m = 2 * leaf_rng[leaf].y, D = min(kOB2, m - K0);
+  double* A = lu + blk_off[leaf] + (size_t)K0 * m + K0;
+  auto blk = [&](int i, int j) { return A + (size_t)(kNP * j) * m + kNP * i; };
+  const int tid = threadIdx.x;
   bool bad = false;
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      const int r = tr + 16 * a, c = tc + 16 * b;
-      if (kind == 0) {
-        if (r < cnt && c < d) {
-          if (!(fabs(acc[a][b]) <= kNoPivBound)) bad = true;
-          A[(size_t)(k0 + c) * m + off + r] = acc[a][b];
+  for (int j = 0; j * kNP < D; ++j) {
+    const int d = min(kNP, D - j * kNP);
+    bad |= lu_diag64(blk(j, j), m, d, b0, b1, b2, sh,
+                     scr + ((size_t)blockIdx.x * (kOB2 / kNP) + j) * 2 * kNP * kNP,
+                     dinv + dinv_off[leaf] + (size_t)((K0 + j * kNP) / kDB) * 2 * kDB * kDB);
+    const int nb = (D + kNP - 1) / kNP;
+    auto size = [&](int i) { return min(kNP, D - i * kNP); };
+    for (int i = j + 1; i < nb; ++i) {
+      __syncthreads();
+      stage64(b2, blk(i, j), m, size(i), kNP);
+      cp_async_commit();
+      cp_async_wait<0>();
+      __syncthreads();
+      double acc[4][2][2] = {};
+      dmma_tile<4, 2, kPP, kPP, kNP>(acc, b2 + tile_r0(), b1 + tile_c0() * kPP);
+      double* out = blk(i, j);
+      tile_each(acc, [&](int r, int c, double v) {
+        if (r < size(i)) {
+          if (!(fabs(v) <= kNoPivBound)) bad = true;
+          out[(size_t)c * m + r] = v;
         }
-      } else if (c < cnt && r < d) {
-        A[(size_t)(off + c) * m + k0 + r] = acc[a][b];
+      });
+    }
+    for (int k = j + 1; k < nb; ++k) {
+      __syncthreads();
+      stage64(b1, blk(j, k), m, kNP, size(k));
+      stage64(b2, blk(j + 1, j), m, size(j + 1), kNP);
+      cp_async_commit();
+      cp_async_wait<0>();
+      __syncthreads();
+      {
+        double acc[4][2][2] = {};
+        dmma_tile<4, 2, kPP, kPP, kNP>(acc, b0 + tile_r0(), b1 + tile_c0() * kPP);
+        __syncthreads();  // A_jk is read
+        double* out = blk(j, k);
+        tile_each(acc, [&](int r, int c, double v) {
+          b1[c * kPP + r] = v;
+          if (c < size(k)) out[(size_t)c * m + r] = v;
+        });
+      }
+      __syncthreads();
+      for (int i = j + 1; i < nb; ++i) {
+        double acc[4][2][2];
+        double* out = blk(i, k);
+        tile_each(acc, [&](int r, int c, double& v) {
+          v = r < size(i) && c < size(k) ? -out[(size_t)c * m + r] : 0.0;
+        });
+        if (i > j + 1) {
+          stage64(b2, blk(i, j), m, size(i), kNP);
+          cp_async_commit();
+          cp_async_wait<0>();
+          __syncthreads();
+        }
+        dmma_tile<4, 2, kPP, kPP, kNP>(acc, b2 + tile_r0(), b1 + tile_c0() * kPP);
+        tile_each(acc, [&](int r, int c, double v) {
+          if (r < size(i) && c < size(k)) out[(size_t)c * m + r] = -v;
+        });
+        if (i + 1 < nb) __syncthreads();  // b2 is read
       }
     }
+    __syncthreads();
+  }
   if (__syncthreads_or(bad) && tid == 0) fail[leaf] = 1;
 }
 
-// Updates of the unpivoted factorisation: item = (leaf, r0, c0, ends):
+// item = (leaf, slot, kind, off) of a leaf with m > K0 + 256: kind 0, rows
+// [off, off + 64) of L21; kind 1, columns [off, off + 64) of U12.  slot = the
+// leaf's position in the block kernel's launch (its scratch).  The chunk lies
+// in shared memory; the ten 64 x 64 blocks of the diagonal block's factors and
+// inverses stream through two buffers:
+//   kind 0: Y_j = Y_j U_jj^{-1}, then Y_i -= Y_j U_ji for i > j (columns by 64),
+//   kind 1: X_j = L_jj^{-1} X_j, then X_i -= L_ij X_j for i > j (rows by 64).
+constexpr int kTP1 = kOB2 + 4;  // kind 1: pitch of a column of 256
+constexpr size_t kNPBorderSmem = sizeof(double) * (kOB2 * kPP + 2 * kNB2);
+
+template <int KIND>
+__device__ __forceinline__ bool lu_border(double* T, double* ring, double* A, int m, int K0,
+                                          int off, const double* S) {
+  const int cnt = min(kNP, m - off);
+  double* chunk = KIND == 0 ? A + (size_t)K0 * m + off : A + (size_t)off * m + K0;
+  const double* F = A + (size_t)K0 * m + K0;  // the factored diagonal block
+  auto stage_factor = [&](int i, int j, int buf) {
+    double* dst = ring + buf * kNB2;
+    if (i == j)
+      stage64(dst, S + (size_t)j * 2 * kNP * kNP + (KIND == 0 ? kNP * kNP : 0), kNP, kNP, kNP);
+    else if (KIND == 0)
+      stage64(dst, F + (size_t)(kNP * i) * m + kNP * j, m, kNP, kNP);
+    else
+      stage64(dst, F + (size_t)(kNP * j) * m + kNP * i, m, kNP, kNP);
+    cp_async_commit();
+  };
+  if (KIND == 0) {
+#pragma unroll
+    for (int j = 0; j < kOB2 / kNP; ++j)
+      stage64(T + j * kNB2, chunk + (size_t)(j * kNP) * m, m, cnt, kNP);
+  } else {
+#pragma unroll
+    for (int e = 0; e < kNP * kOB2 / 2 / kNPT; ++e) {
+      const int q = (int)threadIdx.x + kNPT * e, c = q >> 7, r = 2 * (q & 127);
+      const bool ok = c < cnt;
+      cp_async16(T + c * kTP1 + r, ok ? chunk + (size_t)c * m + r : chunk, ok);
+    }
+  }
+  // entry (r, c) of block i of the chunk
+  auto at = [&](int i, int r, int c) -> double& {
+    return KIND == 0 ? T[i * kNB2 + c * kPP + r] : T[c * kTP1 + i * kNP + r];
+  };
+  auto multiply = [&](double (&acc)[4][2][2], int j, const double* f) {
+    if (KIND == 0)
+      dmma_tile<4, 2, kPP, kPP, kNP>(acc, T + j * kNB2 + tile_r0(), f + tile_c0() * kPP);
+    else
+      dmma_tile<4, 2, kPP, kTP1, kNP>(acc, f + tile_r0(), T + tile_c0() * kTP1 + j * kNP);
+  };
+  bool bad = false;
+  stage_factor(0, 0, 0);
+  int buf = 0;
+  for (int j = 0; j < kOB2 / kNP; ++j)
+    for (int i = j; i < kOB2 / kNP; ++i, buf ^= 1) {
+      cp_async_wait<0>();
+      __syncthreads();  // this factor has arrived, the other buffer is read
+      if (i + 1 < kOB2 / kNP)
+        stage_factor(i + 1, j, buf ^ 1);
+      else if (j + 1 < kOB2 / kNP)
+        stage_factor(j + 1, j + 1, buf ^ 1);
+      const double* f = ring + buf * kNB2;
+      double acc[4][2][2] = {};
+      if (i == j) {
+        multiply(acc, j, f);
+        __syncthreads();  // block j is read
+        tile_each(acc, [&](int r, int c, double v) {
+          if (KIND == 0 && !(fabs(v) <= kNoPivBound)) bad = true;
+          at(j, r, c) = v;
+        });
+      } else {
+        tile_each(acc, [&](int r, int c, double& v) { v = -at(i, r, c); });
+        multiply(acc, j, f);
+        tile_each(acc, [&](int r, int c, double v) { at(i, r, c) = -v; });
+      }
+    }
+  __syncthreads();
+  if (KIND == 0) {
+    for (int q = threadIdx.x; q < kOB2 * kNP; q += kNPT) {
+      const int c = q >> 6, r = q & 63;
+      if (r < cnt) chunk[(size_t)c * m + r] = T[c * kPP + r];
+    }
+  } else {
+    for (int q = threadIdx.x; q < kNP * kOB2; q += kNPT) {
+      const int c = q >> 8, r = q & 255;
+      if (c < cnt) chunk[(size_t)c * m + r] = T[c * kTP1 + r];
+    }
+  }
+  return bad;
+}
+
+__global__ void __launch_bounds__(kNPT, 1) lu_np_border_kernel(
+    const int4* __restrict__ items, int K0, const int2* __restrict__ leaf_rng,
+    const int64_t* __restrict__ blk_off, double* lu, const double* __restrict__ scr,
+    int* __restrict__ fail) {
+  extern __shared__ __align__(16) double nsm[];
+  chain_wait();  // the previous launch of the chain has finished
+  chain_signal();
+  const int4 it = items[blockIdx.x];
+  const int m = 2 * leaf_rng[it.x].y;
+  double* A = lu + blk_off[it.x];
+  const double* S = scr + (size_t)it.y * (kOB2 / kNP) * 2 * kNP * kNP;
+  double* ring = nsm + kOB2 * kPP;
+  const bool bad = it.z == 0 ? lu_border<0>(nsm, ring, A, m, K0, it.w, S)
+                             : lu_border<1>(nsm, ring, A, m, K0, it.w, S);
+  if (__syncthreads_or(bad) && threadIdx.x == 0) fail[it.x] = 1;
+}
+
+// Updates of the unpivoted factorisation: item = (leaf, r0, c0, -):
 // C = A[r0:r0+128, c0:c0+64] -= A[r0:, k0:k0+kd] A[k0:k0+kd, c0:] with
-// kd = min(kdepth, m - k0) (64 inside an outer block of kOB2 columns, kOB2
-// for the trailing matrix right of it), rows clipped at re and columns at ce,
-// packed as ends = (re << 16) | ce (0: both m).  256 threads, 8 x 4
-// outputs each: rows 2 tr + 32 a + {0, 1} (a = 0..3; each pair one 16-byte
-// shared load, eight lanes of a load phase on 32 distinct banks) and columns
-// 4 tc .. 4 tc + 3 (two 16-byte loads, broadcast within a phase).  C is loaded
-// into the accumulators and the products subtracted one k at a time
-// (fma(-l, u, c)), the order of the reference's DGEMM (C := C - A B,
-// dgetrf_dep.f), while the 32-deep slices of L (k-major) and U (by column,
-// pitch 34: conflict-free 16-byte stores, broadcast loads) arrive by cp.async
-// (zero-filled outside the tile: m, r0, c0, k0 and the depth are even, so a
-// 16-byte chunk is wholly inside or outside).
+// kd = min(kdepth, m - k0), rows and columns clipped at m.  FP64 tensor cores, a
+// 32 x 32 tile per warp: -C is loaded into the accumulators, the products are added
+// in order of k, and the negative of the sum is stored.  32-deep slices of L
+// (k-major) and U (by column) arrive by cp.async, double-buffered (zero-filled
+// outside the tile: m, r0, c0, k0 and the depth are even, so a 16-byte chunk is
+// wholly inside or outside).  The form with 8 x 4 outputs per thread on DFMA
+// was bound by its 12 shared-load words per 32 multiply-adds: 45-50 % of the
+// FP64 pipe.
 constexpr int kG2M = 128, kG2N = 64, kG2K = 32;
-constexpr int kG2UP = kG2K + 2;  // U slice by column: pitch of 34 doubles
-constexpr int kOB2 = 256;  // outer block of the unpivoted factorisation
-constexpr size_t kGemm2Smem = sizeof(double) * 2 * (kG2K * kG2M + kG2N * kG2UP);
+constexpr int kG2LP = kG2M + 4;  // L slice: pitch of a depth's 128 rows
+constexpr int kG2UP = kG2K + 4;  // U slice: pitch of a column's 32 depths
+constexpr size_t kGemm2Smem = sizeof(double) * 2 * (kG2K * kG2LP + kG2N * kG2UP);
 
 __global__ void __launch_bounds__(256, 2) lu_gemm2_kernel(const int4* __restrict__ items, int k0,
                                                           int kdepth,
                                                           const int2* __restrict__ leaf_rng,
                                                           const int64_t* __restrict__ blk_off,
                                                           double* __restrict__ lu) {
-  extern __shared__ double gsm2[];
+  extern __shared__ __align__(16) double gsm2[];
   chain_wait();  // the previous launch of the chain has finished
   chain_signal();
-  double* sL = gsm2;                      // [2][kG2K][kG2M]  L slice, k-major
-  double* sU = gsm2 + 2 * kG2K * kG2M;    // [2][kG2N][kG2UP] U slice, by column
+  double* sL = gsm2;                      // [2][kG2K][kG2LP]  L slice, k-major
+  double* sU = gsm2 + 2 * kG2K * kG2LP;   // [2][kG2N][kG2UP] U slice, by column
   const int4 it = items[blockIdx.x];
   const int leaf = it.x, r0 = it.y, c0 = it.z;
   const int m = 2 * leaf_rng[leaf].y;
-  const int re = it.w ? min(m, it.w >> 16) : m, ce = it.w ? min(m, it.w & 0xffff) : m;
   const int kd = min(kdepth, m - k0);
   double* A = lu + blk_off[leaf];
-  const int tid = threadIdx.x;
-  const int tr = tid & 15, tc = tid >> 4;
-  auto row_of = [&](int a) { return 2 * tr + 32 * (a >> 1) + (a & 1); };
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   auto load_slice = [&](int kc, int buf) {
     const int nbk = min(kG2K, kd - kc), kb = k0 + kc;
-    double* L = sL + buf * kG2K * kG2M;
+    double* L = sL + buf * kG2K * kG2LP;
     double* U = sU + buf * kG2N * kG2UP;
 #pragma unroll
     for (int e = 0; e < (kG2K * kG2M / 2) / 256; ++e) {
       const int q = tid + 256 * e;
       const int k = q / (kG2M / 2), rr = 2 * (q % (kG2M / 2));
-      const bool ok = k < nbk && r0 + rr < re;
-      cp_async16(L + k * kG2M + rr, ok ? A + (size_t)(kb + k) * m + r0 + rr : A, ok);
+      const bool ok = k < nbk && r0 + rr < m;
+      cp_async16(L + k * kG2LP + rr, ok ? A + (size_t)(kb + k) * m + r0 + rr : A, ok);
     }
     // U by column (the source's own layout): 16-byte chunks of 2 k
 #pragma unroll
     for (int e = 0; e < (kG2K * kG2N / 2) / 256; ++e) {
       const int q = tid + 256 * e;
       const int c = q / (kG2K / 2), kk = 2 * (q % (kG2K / 2));
-      const bool ok = kk < nbk && c0 + c < ce;
+      const bool ok = kk < nbk && c0 + c < m;
       cp_async16(U + c * kG2UP + kk, ok ? A + (size_t)(c0 + c) * m + kb + kk : A, ok);
     }
     asm volatile("cp.async.commit_group;\n" ::);
   };
   load_slice(0, 0);
   if (kG2K < kd) load_slice(kG2K, 1);
-  // C by row pairs: 16 lanes read 256 contiguous bytes of a column (rows and
-  // m are even, so a pair is wholly inside or outside)
-  double acc[8][4];
+  // this warp's tile, and the lane's row and column in it
+  const int wr = 32 * (warp & 3), wc = 32 * (warp >> 2);
+  const int rl = r0 + wr + (lane >> 2), cl = c0 + wc + 2 * (lane & 3);
+  double acc[4][4][2];
 #pragma unroll
-  for (int b = 0; b < 4; ++b) {
-    const int c = c0 + 4 * tc + b;
-    const double* cc = A + (size_t)min(c, m - 1) * m;
+  for (int q = 0; q < 4; ++q)
 #pragma unroll
-    for (int a = 0; a < 8; a += 2) {
-      const int r = r0 + row_of(a);
-      const double2 v = (c < ce && r < re) ? *reinterpret_cast<const double2*>(cc + r)
-                                           : make_double2(0.0, 0.0);
-      acc[a][b] = v.x;
-      acc[a + 1][b] = v.y;
+    for (int b = 0; b < 2; ++b) {
+      const int c = cl + 8 * q + b;
+      const double* cc = A + (size_t)min(c, m - 1) * m;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = rl + 8 * i;
+        acc[i][q][b] = (c < m && r < m) ? -cc[r] : 0.0;
+      }
     }
-  }
   for (int kc = 0, buf = 0; kc < kd; kc += kG2K, buf ^= 1) {
     if (kc + kG2K < kd) {
       asm volatile("cp.async.wait_group 1;\n" ::);
@@ -1589,56 +1752,27 @@ __global__ void __launch_bounds__(256, 2) lu_gemm2_kernel(const int4* __restrict
       asm volatile("cp.async.wait_group 0;\n" ::);
     }
     __syncthreads();
-    // all 32 k of the slice (zero-filled past the depth: fma(-0, 0, c) = c),
-    // the next k's operands loaded while this k's products run
-    const double* L = sL + buf * kG2K * kG2M + 2 * tr;
-    const double* U = sU + buf * kG2N * kG2UP + 4 * tc * kG2UP;
-    double2 lc[4];
-    double uc[4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a) lc[a] = *reinterpret_cast<const double2*>(L + 32 * a);
-#pragma unroll
-    for (int b = 0; b < 4; ++b) uc[b] = U[b * kG2UP];
-#pragma unroll
-    for (int k = 0; k < kG2K; ++k) {
-      double2 ln[4];
-      double un[4];
-      if (k + 1 < kG2K) {
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-          ln[a] = *reinterpret_cast<const double2*>(L + (k + 1) * kG2M + 32 * a);
-#pragma unroll
-        for (int b = 0; b < 4; ++b) un[b] = U[b * kG2UP + k + 1];
-      }
-      const double lv[8] = {lc[0].x, lc[0].y, lc[1].x, lc[1].y,
-                            lc[2].x, lc[2].y, lc[3].x, lc[3].y};
-#pragma unroll
-      for (int a = 0; a < 8; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] = fma(-lv[a], uc[b], acc[a][b]);
-      if (k + 1 < kG2K) {
-#pragma unroll
-        for (int a = 0; a < 4; ++a) lc[a] = ln[a];
-#pragma unroll
-        for (int b = 0; b < 4; ++b) uc[b] = un[b];
-      }
-    }
+    // all 32 k of the slice: zero-filled past the depth
+    dmma_tile<4, 4, kG2LP, kG2UP, kG2K>(acc, sL + buf * kG2K * kG2LP + wr,
+                                        sU + buf * kG2N * kG2UP + wc * kG2UP);
     if (kc + 2 * kG2K < kd) {  // buffer buf takes the slice two on
       __syncthreads();
       load_slice(kc + 2 * kG2K, buf);
     }
   }
 #pragma unroll
-  for (int b = 0; b < 4; ++b) {
-    const int c = c0 + 4 * tc + b;
-    if (c >= ce) continue;
-    double* cc = A + (size_t)c * m;
+  for (int q = 0; q < 4; ++q)
 #pragma unroll
-    for (int a = 0; a < 8; a += 2) {
-      const int r = r0 + row_of(a);
-      if (r < re) *reinterpret_cast<double2*>(cc + r) = make_double2(acc[a][b], acc[a + 1][b]);
+    for (int b = 0; b < 2; ++b) {
+      const int c = cl + 8 * q + b;
+      if (c >= m) continue;
+      double* cc = A + (size_t)c * m;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = rl + 8 * i;
+        if (r < m) cc[r] = -acc[i][q][b];
+      }
     }
-  }
 }
 
 // every leaf: no interchange (1-based local pivots i + 1) and the identity
@@ -1733,8 +1867,8 @@ void build_precond(Handle& H, cudaStream_t s) {
     T.d_dinv_off.alloc(nl);
     H.pc_h_dinv_off.assign(T.dinv_off.data(), nl);
     H.pc_h_dinv_off.upload(T.d_dinv_off, s);
-    raise_smem_limit((const void*)lu_np_diag_kernel, kNPDiagSmem);
-    raise_smem_limit((const void*)lu_np_panel_kernel, kNPPanelSmem);
+    raise_smem_limit((const void*)lu_np_block_kernel, kNPBlockSmem);
+    raise_smem_limit((const void*)lu_np_border_kernel, kNPBorderSmem);
     raise_smem_limit((const void*)lu_gemm2_kernel, kGemm2Smem);
     std::vector<int> grp[2];
     for (int l = 0; l < nl; ++l) grp[2 * rng[l].y > kLuSmallBlock ? 0 : 1].push_back(l);
@@ -1744,32 +1878,22 @@ void build_precond(Handle& H, cudaStream_t s) {
     TABI_CUDA(cudaEventRecord(H.ev_fork, s));
     TABI_CUDA(cudaStreamWaitEvent(H.lu_hi, H.ev_fork, 0));
     TABI_CUDA(cudaStreamWaitEvent(H.lu_small, H.ev_fork, 0));
-    // Two-level right-looking order (outer blocks of kOB2 columns, inner steps
-    // of 64).  Inside an outer block: the diagonal block of each inner step,
-    // its L21 for every row below and its U12 for the block's own columns, and
-    // the update of the block's own columns.  Then the columns right of the
-    // block: U12 = L11^{-1} A12 in four 64-row sub-steps (each applies the
-    // inner step's L^{-1}, then updates the block's rows below it), and the
-    // trailing matrix takes one kOB2-deep update.
+    // Right-looking order in outer blocks of kOB2 columns: the diagonal block of
+    // every leaf, its L21 and U12 chunks, the trailing update.
     //
-    // Look-ahead (the large-block group): the trailing update of an outer
-    // block is split by columns.  The next outer block's kOB2 columns, which
-    // its steps factor, are updated on the group's stream; the columns beyond
-    // it on the low-priority auxiliary stream, beside the next
-    // block's diagonal, panel and update launches, which touch only rows and
-    // columns of that block or its own columns below it.  The next block's
-    // columns right of it (rows of the block, columns beyond) wait for the
-    // auxiliary stream.  Every entry is updated by the same tile in the same
-    // k order as without the split, so the factors are the same bit for bit.
+    // Look-ahead: the trailing update of an outer block is split.  The next
+    // outer block's diagonal block, which is factored next, is updated on the
+    // group's stream; the rest on the middle-priority auxiliary stream, beside
+    // that factorisation.  The next block's chunks wait for the auxiliary
+    // stream.
     struct Launch {
-      // 0 diagonal, 1 panel, 2 update, 3 fork to the auxiliary stream,
-      // 4 wait for the auxiliary stream, 5 update on the auxiliary stream
+      // 0 diagonal block, 1 its chunks, 2 update, 3 fork to the auxiliary
+      // stream, 4 wait for the auxiliary stream, 5 update on the auxiliary stream
       int kind;
-      int k0, depth, off, cnt, scr_slot0;
+      int k0, off, cnt;
     };
     // one group's plan: item lists (uploaded on st) and its launches
-    auto plan_np = [&](const std::vector<int>& order, Handle::NpPlan& B, cudaStream_t st,
-                       bool la) {
+    auto plan_np = [&](const std::vector<int>& order, Handle::NpPlan& B, cudaStream_t st) {
       int gmax = 0;
       for (int l : order) gmax = std::max(gmax, 2 * rng[l].y);
       std::vector<Launch> plan;
@@ -1779,102 +1903,56 @@ void build_precond(Handle& H, cudaStream_t s) {
       dl.restart();
       pit.restart();
       git.restart();
-      const auto pack = [](int re, int ce) { return (re << 16) | ce; };
-      int max_slots = 1;
-      auto emit = [&](int kind, int k0, int depth, size_t before, size_t after, int slot0) {
-        if (after > before)
-          plan.push_back({kind, k0, depth, (int)before, (int)(after - before), slot0});
+      auto emit = [&](int kind, int k0, size_t before, size_t after) {
+        if (after > before) plan.push_back({kind, k0, (int)before, (int)(after - before)});
       };
       bool rest_pending = false;  // an update on the auxiliary stream not yet waited for
       for (int K0 = 0; K0 < gmax; K0 += kOB2) {
-        int nact = 0;
-        for (int l : order) nact += 2 * rng[l].y > K0;
-        max_slots = std::max(max_slots, nact);
-        // the leaves' rows in this outer block's diagonal launches: slot index
-        // = inner step * nact + position
-        for (int k0 = K0; k0 < std::min(gmax, K0 + kOB2); k0 += kNP) {
-          const int j = (k0 - K0) / kNP;
-          size_t d0 = dl.len, p0 = pit.len, g0 = git.len;
-          int slot = 0;
-          for (int l : order) {
-            const int m = 2 * rng[l].y;
-            if (m <= k0) continue;
-            dl.push(l);
-            const int d = std::min(kNP, m - k0), ce = std::min(m, K0 + kOB2);
-            for (int off = k0 + d; off < m; off += kNP)
-              pit.push(make_int4(l, j * nact + slot, 0, off));
-            for (int off = k0 + d; off < ce; off += kNP)
-              pit.push(make_int4(l, j * nact + slot, 1, off));
-            for (int r0 = k0 + d; r0 < m; r0 += kG2M)
-              for (int c0 = k0 + d; c0 < ce; c0 += kG2N)
-                git.push(make_int4(l, r0, c0, pack(m, ce)));
-            ++slot;
-          }
-          emit(0, k0, 0, d0, dl.len, j * nact);
-          emit(1, k0, 0, p0, pit.len, 0);
-          emit(2, k0, kNP, g0, git.len, 0);
-        }
-        // the columns right of the block (leaves with m > K0 + kOB2 have all
-        // four inner steps; their slot in inner step j is j * nact + the
-        // leaf's position among the active leaves)
-        const int Kend = K0 + kOB2;
-        if (rest_pending) {
-          plan.push_back({4, K0, 0, 0, 0, 0});
-          rest_pending = false;
-        }
-        for (int j = 0; j < kOB2 / kNP; ++j) {
-          const int k0 = K0 + j * kNP;
-          size_t p0 = pit.len, g0 = git.len;
-          int pos = 0;
-          for (int l : order) {
-            const int m = 2 * rng[l].y;
-            if (m <= K0) continue;
-            if (m > Kend) {
-              for (int off = Kend; off < m; off += kNP)
-                pit.push(make_int4(l, j * nact + pos, 1, off));
-              for (int r0 = k0 + kNP; r0 < Kend; r0 += kG2M)
-                for (int c0 = Kend; c0 < m; c0 += kG2N)
-                  git.push(make_int4(l, r0, c0, pack(Kend, m)));
-            }
-            ++pos;
-          }
-          emit(1, k0, 0, p0, pit.len, 0);
-          emit(2, k0, kNP, g0, git.len, 0);
-        }
-        // the trailing update: columns [Kend, Knext) here, the rest on the
-        // auxiliary stream (all of it here without look-ahead)
-        const int Knext = la ? Kend + kOB2 : INT_MAX;
-        size_t g0 = git.len;
+        const int Kend = K0 + kOB2, Knext = Kend + kOB2;
+        const size_t d0 = dl.len, p0 = pit.len, g0 = git.len;
+        int slot = 0;
         for (int l : order) {
           const int m = 2 * rng[l].y;
-          if (m <= Kend) continue;
-          for (int r0 = Kend; r0 < m; r0 += kG2M)
+          if (m <= K0) continue;
+          dl.push(l);
+          for (int off = Kend; off < m; off += kNP) {
+            pit.push(make_int4(l, slot, 0, off));
+            pit.push(make_int4(l, slot, 1, off));
+          }
+          for (int r0 = Kend; r0 < std::min(m, Knext); r0 += kG2M)
             for (int c0 = Kend; c0 < std::min(m, Knext); c0 += kG2N)
               git.push(make_int4(l, r0, c0, 0));
+          ++slot;
         }
         const size_t g1 = git.len;
         for (int l : order) {
           const int m = 2 * rng[l].y;
           if (m <= Knext) continue;
           for (int r0 = Kend; r0 < m; r0 += kG2M)
-            for (int c0 = Knext; c0 < m; c0 += kG2N) git.push(make_int4(l, r0, c0, 0));
+            for (int c0 = r0 < Knext ? Knext : Kend; c0 < m; c0 += kG2N)
+              git.push(make_int4(l, r0, c0, 0));
         }
-        // the fork before the look-ahead columns' launch (the auxiliary stream
+        emit(0, K0, d0, dl.len);
+        if (rest_pending) {
+          plan.push_back({4, K0, 0, 0});
+          rest_pending = false;
+        }
+        emit(1, K0, p0, pit.len);
+        // the fork before the look-ahead tiles' launch (the auxiliary stream
         // must not wait for it), the rest launched after it (earlier launches
         // are dispatched first)
         const bool rest = git.len > g1;
-        if (rest) plan.push_back({3, K0, 0, 0, 0, 0});
-        emit(2, K0, kOB2, g0, g1, 0);
+        if (rest) plan.push_back({3, K0, 0, 0});
+        emit(2, K0, g0, g1);
         if (rest) {
-          emit(5, K0, kOB2, g1, git.len, 0);
+          emit(5, K0, g1, git.len);
           rest_pending = true;
         }
       }
-      if (rest_pending) plan.push_back({4, gmax, 0, 0, 0, 0});
       dl.upload(B.dleaves, st);
       pit.upload(B.pitems, st);
       git.upload(B.gitems, st);
-      B.scr.alloc((size_t)max_slots * (kOB2 / kNP) * 2 * kNP * kNP);
+      B.scr.alloc(order.size() * (kOB2 / kNP) * 2 * kNP * kNP);
       return plan;
     };
     // Issues launch `at` of a group's plan.  Kernels follow kernels on the
@@ -1895,14 +1973,13 @@ void build_precond(Handle& H, cudaStream_t s) {
       {
         if (q.kind == 0) {
           TABI_K(K_LU, st);
-          launch_chained(chain, lu_np_diag_kernel, dim3(q.cnt), dim3(kNPT), kNPDiagSmem, st,
+          launch_chained(chain, lu_np_block_kernel, dim3(q.cnt), dim3(kNPT), kNPBlockSmem, st,
                          B.dleaves.p + q.off, q.k0, T.d_leaf_rng.p, T.d_blk_off.p,
-                         T.d_dinv_off.p, T.d_lu.p, T.d_dinv.p,
-                         B.scr.p + (size_t)q.scr_slot0 * 2 * kNP * kNP, d_fail.p);
+                         T.d_dinv_off.p, T.d_lu.p, T.d_dinv.p, B.scr.p, d_fail.p);
           chain = true;
         } else if (q.kind == 1) {
           TABI_K(K_LU_STRIP, st);
-          launch_chained(chain, lu_np_panel_kernel, dim3(q.cnt), dim3(kNPT), kNPPanelSmem, st,
+          launch_chained(chain, lu_np_border_kernel, dim3(q.cnt), dim3(kNPT), kNPBorderSmem, st,
                          B.pitems.p + q.off, q.k0, T.d_leaf_rng.p, T.d_blk_off.p, T.d_lu.p,
                          B.scr.p, d_fail.p);
           chain = true;
@@ -1918,7 +1995,7 @@ void build_precond(Handle& H, cudaStream_t s) {
           TABI_K(K_LU_UPDATE, gs);
           launch_chained(chain && q.kind == 2, lu_gemm2_kernel, dim3(q.cnt), dim3(256),
                          kGemm2Smem, gs,
-                         B.gitems.p + q.off, q.k0, q.depth, T.d_leaf_rng.p, T.d_blk_off.p,
+                         B.gitems.p + q.off, q.k0, kOB2, T.d_leaf_rng.p, T.d_blk_off.p,
                          T.d_lu.p);
           if (q.kind == 5) TABI_CUDA(cudaEventRecord(H.ev_rest, H.aux));
           else chain = true;
@@ -1932,8 +2009,8 @@ void build_precond(Handle& H, cudaStream_t s) {
     big.st = H.lu_hi;
     small.B = &H.pc_np[1];
     small.st = H.lu_small;
-    if (!grp[0].empty()) big.plan = plan_np(grp[0], H.pc_np[0], H.lu_hi, true);
-    if (!grp[1].empty()) small.plan = plan_np(grp[1], H.pc_np[1], H.lu_small, false);
+    if (!grp[0].empty()) big.plan = plan_np(grp[0], H.pc_np[0], H.lu_hi);
+    if (!grp[1].empty()) small.plan = plan_np(grp[1], H.pc_np[1], H.lu_small);
     while (big.at < big.plan.size() || small.at < small.plan.size()) {
       if (big.at < big.plan.size()) issue_one(big);
       if (small.at < small.plan.size()) issue_one(small);
