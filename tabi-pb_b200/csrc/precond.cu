@@ -1234,8 +1234,8 @@ __global__ void __launch_bounds__(NT, (NT <= 256 ? 4 : 1)) solve_kernel(
 // near tie, a zero or non-finite pivot) is re-assembled and factored again by
 // the pivoted kernels above.
 constexpr int kNP = 64;    // step width
-constexpr int kNPT = 256;  // threads of the block and border kernels
-constexpr int kOB2 = 256;  // outer block
+constexpr int kNPT = 256;  // threads of the block kernel
+constexpr int kOB2 = 128;  // outer block
 constexpr int kPP = kNP + 4;  // pitch of a staged 64-double column
 constexpr int kNB2 = kNP * kPP;  // a staged 64 x 64 block
 constexpr double kNoPivBound = 1.0 - 1.0 / 1048576.0;
@@ -1278,11 +1278,12 @@ __device__ __forceinline__ void dmma_tile(double (&acc)[MT][NT][2], const double
 
 // Copies a block of 64 columns of 64 doubles (leading dimension ld, 16-byte
 // aligned columns) into shared memory at pitch kPP, zeros outside nr x nc (nr
-// even); the caller commits and waits.
+// even); the caller commits and waits.  NT: threads of the CTA.
+template <int NT>
 __device__ __forceinline__ void stage64(double* dst, const double* src, int ld, int nr, int nc) {
 #pragma unroll
-  for (int e = 0; e < kNP * kNP / 2 / kNPT; ++e) {
-    const int q = (int)threadIdx.x + kNPT * e, c = q >> 5, r = 2 * (q & 31);
+  for (int e = 0; e < kNP * kNP / 2 / NT; ++e) {
+    const int q = (int)threadIdx.x + NT * e, c = q >> 5, r = 2 * (q & 31);
     const bool ok = c < nc && r < nr;
     cp_async16(dst + c * kPP + r, ok ? src + (size_t)c * ld + r : src, ok);
   }
@@ -1294,171 +1295,218 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
 }
 
-// A warp's 32 x 16 tile of a 64 x 64 product: rows tile_r0().., columns
-// tile_c0().., and f(r, c, entry) over the lane's entries of it
-__device__ __forceinline__ int tile_r0() { return 32 * ((int)(threadIdx.x >> 5) & 1); }
-__device__ __forceinline__ int tile_c0() { return 16 * (int)(threadIdx.x >> 6); }
-template <typename F>
-__device__ __forceinline__ void tile_each(double (&acc)[4][2][2], F&& f) {
-  const int r = tile_r0() + ((int)(threadIdx.x & 31) >> 2);
-  const int c = tile_c0() + 2 * ((int)threadIdx.x & 3);
+// f(r, c, entry) over the lane's entries of a warp's (8 MT) x (8 NT) tile
+template <int MT, int NT, typename F>
+__device__ __forceinline__ void tile_each(double (&acc)[MT][NT][2], F&& f) {
+  const int r = (int)(threadIdx.x & 31) >> 2, c = 2 * ((int)threadIdx.x & 3);
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < MT; ++i)
 #pragma unroll
-    for (int q = 0; q < 2; ++q)
+    for (int q = 0; q < NT; ++q)
 #pragma unroll
       for (int b = 0; b < 2; ++b) f(r + 8 * i, c + 8 * q + b, acc[i][q][b]);
 }
 
-// The d x d (d <= 64) diagonal block at D (column-major, leading dimension m)
-// factored in place without interchanges (DGETRF2's scaling: multipliers
-// times the pivot's reciprocal).  li and ui (shared, pitch kPP) receive
-// L^{-1} (unit lower) and U^{-1}, column-major with zeros outside the triangle
-// and from d on; S the same at pitch 64; Di their 32 x 32 diagonal blocks
-// (identity padded, the layout lu_diaginv_kernel writes).  fb: shared scratch
-// of one staged block.  Every thread of the CTA; true if the certificate
-// failed in an entry of this thread.  The block, L^{-1} and U^{-1} live in
-// registers on a 16 x 16 thread grid; one loop of d steps with one barrier each
-// factors the block and forms both inverses.  Every entry of the factors takes
-// the same sequence of updates as in a column-by-column DGETF2 order.
-struct DiagShared {
-  double rcp[kNP];  // reciprocal of each pivot
-  double row[2][kNP], col[2][kNP], xrow[2][kNP], zcol[2][kNP];
-};
+// 1/x to about an ulp for normal, finite x: one third-order Householder step
+// y (1 + e + e^2), e = 1 - x y, from the hardware's approximation (relative
+// error 2^-20); a chain of four operations after it, half the latency of a
+// division.
+__device__ __forceinline__ double fast_rcp(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
 
+// The CTA (256 threads, one element each): the 16 x 16 block at A (shared,
+// column-major, pitch kPP; rows and columns from d on are zero) factored in
+// place without interchanges (DGETRF2's scaling: multipliers times the pivot's
+// reciprocal); rcp receives the reciprocals of the pivots (0 from d on).  True
+// in threads whose entry fails the certificate; a pivot that is zero, subnormal
+// (where DGETRF2 divides instead) or not finite fails it too, and the leaf goes
+// to the pivoted kernels, which follow DGETRF2 there.  Step t reads row and
+// column t and writes only entries right of and below them, so one barrier a
+// step is enough.  One warp with eight entries a lane took 475 cycles a step
+// (its own 110 instructions), one entry a thread takes a third of that.
+__device__ __forceinline__ bool lu_diag16(double* A, int d, double* rcp) {
+  const int r = threadIdx.x & 15, c = threadIdx.x >> 4;
+  double a = A[c * kPP + r];
+#pragma unroll 1
+  for (int t = 0; t < d; ++t) {
+    const double rp = fast_rcp(A[t * kPP + t]);
+    const double l = A[t * kPP + r] * rp, u = A[c * kPP + t];
+    if (r > t) {
+      if (c > t) {
+        a = fma(-l, u, a);
+        A[c * kPP + r] = a;
+      } else if (c == t) {
+        a = l;
+      }
+    }
+    if (r == t && c == t) rcp[t] = rp;
+    __syncthreads();
+  }
+  bool bad = false;
+  if (r > c) {
+    A[c * kPP + r] = a;
+    bad = !(fabs(a) <= kNoPivBound);
+  } else if (r == c) {
+    if (r < d)
+      bad = !(fabs(a) >= 2.2250738585072014e-308 && fabs(a) <= 1.7976931348623157e308);
+    else
+      rcp[r] = 0.0;
+  }
+  return bad;
+}
+
+// One warp: li and ui (zero on entry) receive the inverses of the factored 16 x
+// 16 block at A, zero from d on.  Half h = 0 of the warp: column r of L^{-1} by
+// forward substitution; h = 1: column r of U^{-1} by backward substitution, the
+// same loop on reversed indices.
+__device__ __forceinline__ void lu_inv16(const double* A, int d, const double* rcp, double* li,
+                                         double* ui) {
+  const int lane = threadIdx.x & 31, r = lane & 15, h = lane >> 4;
+  const double* M = h == 0 ? A : A + 15 * kPP + 15;
+  const int sg = h == 0 ? 1 : -1, c = h == 0 ? r : 15 - r;
+  double x[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) x[i] = i == c && r < d ? 1.0 : 0.0;
+#pragma unroll
+  for (int q = 0; q < 16; ++q) {
+    if (h == 1) x[q] *= rcp[15 - q];
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      if (i > q) x[i] = fma(-M[sg * (q * kPP + i)], x[q], x[i]);
+  }
+  double* out = (h == 0 ? li : ui) + r * kPP;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) out[h == 0 ? i : 15 - i] = x[i];
+}
+
+// The d x d (d <= 64) diagonal block at D (column-major, leading dimension m)
+// factored in place; li and ui (shared, pitch kPP) receive L^{-1} (unit lower)
+// and U^{-1}, column-major with zeros outside the triangle and from d on; S the
+// same at pitch 64; Di their 32 x 32 diagonal blocks (identity padded, the
+// layout lu_diaginv_kernel writes).  fb: shared scratch of one staged block.
+// Every thread of the CTA; true if the certificate failed in an entry of this
+// thread.  Right-looking in four 16-column steps: the CTA factors the 16 x 16
+// block, a lane each substitutes a row of L or a column of U, and the update
+// is 16 x 16 x 16 tensor-core products, one warp each.  Then the inverses of the
+// four 16 x 16 blocks, one warp each, and from them by doubling those of 32 and
+// 64.  A loop over 64 columns with
+// one CTA barrier each, forming both inverses on the way, took 600 cycles a
+// column.
 __device__ bool lu_diag64(double* D, int m, int d, double* li, double* ui, double* fb,
-                          DiagShared& sh, double* S, double* Di) {
-  const int tid = threadIdx.x;
-  auto& s_rcp = sh.rcp;
-  auto& s_row = sh.row;
-  auto& s_col = sh.col;
-  auto& s_xrow = sh.xrow;
-  auto& s_zcol = sh.zcol;
-  stage64(fb, D, m, d, d);
+                          double* s_rcp, double* S, double* Di) {
+  const int tid = threadIdx.x, warp = tid >> 5;
+  constexpr int B = 16 * (kPP + 1);  // from one 16 x 16 diagonal block to the next
+  constexpr int C = 16 * kPP, NB = 4;
+  stage64<kNPT>(fb, D, m, d, d);
   cp_async_commit();
+  for (int e = tid; e < kNB2; e += kNPT) li[e] = ui[e] = 0.0;
   cp_async_wait<0>();
   __syncthreads();
-  // Thread (tx, ty) of a 16 x 16 grid holds rows ty + 16p and columns
-  // tx + 16q (p, q < 4) of the block in registers, and of X = L^{-1} and
-  // Z = U^{-1}.  The column loop runs as four rolled loops of 16 (one per
-  // band jp), so every register index and every band range is a compile-time
-  // constant; a short rolled loop also keeps the code that this
-  // once-per-launch kernel fetches small.  Entries of finished rows and
-  // columns within a band take a zero multiplier or row entry, which leaves
-  // them unchanged, so the updates need no predicates.
-  //
-  // Step j, one barrier (published vectors double-buffered by parity):
-  //  * the factorisation (DGETRF2's scaling): row j and column j, unscaled,
-  //    are published; every thread forms its rows' multipliers with the
-  //    pivot's reciprocal and updates its entries right of and below the
-  //    pivot.  The reciprocal of pivot j + 1 is formed during step j by the
-  //    thread that holds that entry, right after its update, and stored for
-  //    step j + 1.  A pivot that is zero, subnormal (where DGETRF2 divides
-  //    instead) or not finite fails the certificate, and the leaf goes to
-  //    the pivoted kernels, which follow DGETRF2 there.
-  //  * X by forward row operations, row i -= L[i][j] (row j of X), with row j
-  //    final at step j and L[i][j] the step's multiplier;
-  //  * Z by column operations, column j times the pivot's reciprocal, then
-  //    column c -= U[j][c] (column j of Z), with U[j][c] the step's row.
-  // X is lower and Z upper triangular, so step j changes X in rows of bands
-  // >= jp and columns of bands <= jp, Z the other way round.
-  const int tx = tid & 15, ty = tid >> 4;
   bool bad = false;
-  double a[4][4], x[4][4], z[4][4];
-#pragma unroll
-  for (int p = 0; p < 4; ++p)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int i = ty + 16 * p, c = tx + 16 * q;
-      a[p][q] = fb[c * kPP + i];
-      x[p][q] = z[p][q] = (i == c && i < d) ? 1.0 : 0.0;
-    }
-  auto pivot_rcp = [&](int j, double pk) {  // by the holder of entry (j, j)
-    if (!(fabs(pk) >= 2.2250738585072014e-308 && fabs(pk) <= 1.7976931348623157e308)) bad = true;
-    s_rcp[j] = 1.0 / pk;
+  auto put = [](double* dst, double (&acc)[2][2][2], double s) {
+    tile_each(acc, [&](int r, int c, double v) { dst[c * kPP + r] = s * v; });
   };
-  if (tid == 0) pivot_rcp(0, a[0][0]);
+  for (int j = 0; 16 * j < d; ++j) {
+    double* a = fb + j * B;
+    double* rcp = s_rcp + 16 * j;
+    bad |= lu_diag16(a, min(16, d - 16 * j), rcp);
+    __syncthreads();
+    // warps 0 and 1: row 16 + lane of L below the block; 2 and 3: column of U
+    // right of it
+    const int rem = NB - 1 - j, x0 = tid & 63;
+    if (tid < 128 && x0 < 16 * rem) {
+      double x[16];
+      if (tid < 64) {
+        double* p = a + 16 + x0;
 #pragma unroll
-  for (int jp = 0; jp < 4; ++jp) {
-#pragma unroll 1
-    for (int jt = 0; jt < 16; ++jt) {
-      const int j = 16 * jp + jt, b = j & 1;
-      if (j >= d) break;
-      if (ty == jt) {
+        for (int q = 0; q < 16; ++q) x[q] = p[q * kPP];
 #pragma unroll
-        for (int q = jp; q < 4; ++q) s_row[b][tx + 16 * q] = a[jp][q];
+        for (int q = 0; q < 16; ++q) {
+          x[q] *= rcp[q];
+          if (!(fabs(x[q]) <= kNoPivBound)) bad = true;
 #pragma unroll
-        for (int q = 0; q <= jp; ++q) s_xrow[b][tx + 16 * q] = x[jp][q];
+          for (int c = q + 1; c < 16; ++c) x[c] = fma(-x[q], a[c * kPP + q], x[c]);
+        }
+#pragma unroll
+        for (int q = 0; q < 16; ++q) p[q * kPP] = x[q];
+      } else {
+        double* p = a + (16 + x0) * kPP;
+#pragma unroll
+        for (int q = 0; q < 16; ++q) x[q] = p[q];
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+#pragma unroll
+          for (int i = q + 1; i < 16; ++i) x[i] = fma(-a[q * kPP + i], x[q], x[i]);
+        }
+#pragma unroll
+        for (int q = 0; q < 16; ++q) p[q] = x[q];
       }
-      if (tx == jt) {
-#pragma unroll
-        for (int p = jp; p < 4; ++p) s_col[b][ty + 16 * p] = a[p][jp];
-#pragma unroll
-        for (int p = 0; p <= jp; ++p) s_zcol[b][ty + 16 * p] = z[p][jp];
-      }
-      __syncthreads();
-      const double rcp = s_rcp[j];
-      double l[4], u[4], ux[4], zc[4];
-#pragma unroll
-      for (int p = jp; p < 4; ++p) {
-        const int i = ty + 16 * p;
-        l[p] = i > j ? s_col[b][i] * rcp : 0.0;
-      }
-#pragma unroll
-      for (int q = jp; q < 4; ++q) {
-        const int c = tx + 16 * q;
-        u[q] = c > j ? s_row[b][c] : 0.0;
-      }
-#pragma unroll
-      for (int q = 0; q <= jp; ++q) ux[q] = s_xrow[b][tx + 16 * q];
-#pragma unroll
-      for (int p = 0; p <= jp; ++p) zc[p] = s_zcol[b][ty + 16 * p] * rcp;
-      if (tx == jt) {  // the holders of column j: its multipliers, column j of Z scaled
-#pragma unroll
-        for (int p = jp; p < 4; ++p)
-          if (ty + 16 * p > j) {
-            if (!(fabs(l[p]) <= kNoPivBound)) bad = true;
-            a[p][jp] = l[p];
-          }
-#pragma unroll
-        for (int p = 0; p <= jp; ++p) z[p][jp] = zc[p];
-      }
-#pragma unroll
-      for (int p = jp; p < 4; ++p)
-#pragma unroll
-        for (int q = jp; q < 4; ++q) a[p][q] = fma(-l[p], u[q], a[p][q]);
-      // the next pivot's reciprocal, by its holder
-      if (tx == ty && tx == ((j + 1) & 15) && j + 1 < d) {
-        if (jt < 15)
-          pivot_rcp(j + 1, a[jp][jp]);
-        else if (jp < 3)
-          pivot_rcp(j + 1, a[jp < 3 ? jp + 1 : 3][jp < 3 ? jp + 1 : 3]);
-      }
-#pragma unroll
-      for (int p = jp; p < 4; ++p)
-#pragma unroll
-        for (int q = 0; q <= jp; ++q) x[p][q] = fma(-l[p], ux[q], x[p][q]);
-#pragma unroll
-      for (int p = 0; p <= jp; ++p)
-#pragma unroll
-        for (int q = jp; q < 4; ++q) z[p][q] = fma(-zc[p], u[q], z[p][q]);
     }
+    __syncthreads();
+    for (int w = warp; w < rem * rem; w += kNPT / 32) {
+      const int i = w % rem + 1, k = w / rem + 1;
+      double* t = a + 16 * i + k * C;
+      double acc[2][2][2];
+      tile_each(acc, [&](int r, int c, double& v) { v = -t[c * kPP + r]; });
+      dmma_tile<2, 2, kPP, kPP, 16>(acc, a + 16 * i, a + k * C);
+      put(t, acc, -1.0);
+    }
+    __syncthreads();
   }
-#pragma unroll
-  for (int p = 0; p < 4; ++p)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int i = ty + 16 * p, c = tx + 16 * q;
-      fb[c * kPP + i] = a[p][q];
-      li[c * kPP + i] = x[p][q];
-      ui[c * kPP + i] = z[p][q];
-    }
+  if (warp < NB && 16 * warp < d)
+    lu_inv16(fb + warp * B, d - 16 * warp, s_rcp + 16 * warp, li + warp * B, ui + warp * B);
   __syncthreads();
-  for (int e = tid; e < kNP * kNP; e += kNPT) {
-    const int c = e >> 6, r = e & 63;
-    if (c < d && r < d) D[(size_t)c * m + r] = fb[c * kPP + r];
-    S[e] = li[c * kPP + r];
-    S[kNP * kNP + e] = ui[c * kPP + r];
+  // the off-diagonal block of an inverse of twice the size, from the halves'
+  // inverses: -L22^{-1} (L21 L11^{-1}) and -(U11^{-1} U12) U22^{-1}; the product in
+  // brackets goes through the block's own place
+  if (warp < 4) {  // 32: two blocks of L^{-1}, two of U^{-1}, one warp each
+    const int o = 2 * (warp & 1) * B;
+    double* x = warp < 2 ? li + o + 16 : ui + o + C;
+    double acc[2][2][2] = {}, z[2][2][2] = {};
+    if (warp < 2)
+      dmma_tile<2, 2, kPP, kPP, 16>(acc, fb + o + 16, li + o);
+    else
+      dmma_tile<2, 2, kPP, kPP, 16>(acc, ui + o, fb + o + C);
+    put(x, acc, 1.0);
+    __syncwarp();
+    if (warp < 2)
+      dmma_tile<2, 2, kPP, kPP, 16>(z, li + o + B, x);
+    else
+      dmma_tile<2, 2, kPP, kPP, 16>(z, x, ui + o + B);
+    __syncwarp();
+    put(x, z, -1.0);
+  }
+  __syncthreads();
+  {  // 64: a 16 x 16 tile of the 32 x 32 block each, warps 0..3 of L^{-1}, 4..7 of U^{-1}
+    const int i = 16 * (warp & 1), k = (warp & 2) * (C / 2);
+    double* x = (warp < 4 ? li + 32 : ui + 2 * C) + i + k;
+    double acc[2][2][2] = {}, z[2][2][2] = {};
+    if (warp < 4)
+      dmma_tile<2, 2, kPP, kPP, 32>(acc, fb + 32 + i, li + k);
+    else
+      dmma_tile<2, 2, kPP, kPP, 32>(acc, ui + i, fb + 2 * C + k);
+    put(x, acc, 1.0);
+    __syncthreads();
+    if (warp < 4)
+      dmma_tile<2, 2, kPP, kPP, 32>(z, li + 2 * B + i, li + 32 + k);
+    else
+      dmma_tile<2, 2, kPP, kPP, 32>(z, ui + 2 * C + i, ui + 2 * B + k);
+    __syncthreads();
+    put(x, z, -1.0);
+  }
+  __syncthreads();
+  for (int e = tid; e < kNP * kNP / 2; e += kNPT) {
+    const int c = e >> 5, r = 2 * (e & 31), q = c * kPP + r;
+    const double2 *f2 = reinterpret_cast<const double2*>(fb + q),
+                  *l2 = reinterpret_cast<const double2*>(li + q),
+                  *u2 = reinterpret_cast<const double2*>(ui + q);
+    if (c < d && r < d) *reinterpret_cast<double2*>(D + (size_t)c * m + r) = *f2;
+    reinterpret_cast<double2*>(S)[e] = *l2;
+    reinterpret_cast<double2*>(S + kNP * kNP)[e] = *u2;
   }
   for (int b = 0; b * kDB < d; ++b) {
     const int nb = min(kDB, d - b * kDB), o = b * kDB;
@@ -1492,76 +1540,88 @@ __global__ void __launch_bounds__(kNPT, 2) lu_np_block_kernel(
     const int64_t* __restrict__ blk_off, const int64_t* __restrict__ dinv_off, double* lu,
     double* __restrict__ dinv, double* __restrict__ scr, int* __restrict__ fail) {
   extern __shared__ __align__(16) double nsm[];
-  __shared__ DiagShared sh;
+  __shared__ double s_rcp[kNP];  // reciprocal of each pivot
   chain_wait();  // the previous launch of the chain has finished
   chain_signal();
-  double* b0 = nsm;              // L_jj^{-1}
-  double* b1 = nsm + kNB2;       // U_jj^{-1}, then U_jk
-  double* b2 = nsm + 2 * kNB2;   // A_ij, then L_ij
+  double* b0 = nsm;              // L_jj^{-1}; then one of L_ij's two buffers
+  double* b1 = nsm + kNB2;       // U_jj^{-1}; one of A_jk's two buffers; U_jk
+  double* b2 = nsm + 2 * kNB2;   // A_ij; the other of A_jk's, of L_ij's buffers
   const int leaf = leaves[blockIdx.x];
   const int m = 2 * leaf_rng[leaf].y, D = min(kOB2, m - K0);
   double* A = lu + blk_off[leaf] + (size_t)K0 * m + K0;
   auto blk = [&](int i, int j) { return A + (size_t)(kNP * j) * m + kNP * i; };
-  const int tid = threadIdx.x;
+  auto size = [&](int i) { return min(kNP, D - i * kNP); };
+  const int tid = threadIdx.x, warp = tid >> 5;
+  // this warp's 32 x 16 tile of a product
+  const int r0 = 32 * (warp & 1), c0 = 16 * (warp >> 1);
+  const int nb = (D + kNP - 1) / kNP;
   bool bad = false;
-  for (int j = 0; j * kNP < D; ++j) {
-    const int d = min(kNP, D - j * kNP);
-    bad |= lu_diag64(blk(j, j), m, d, b0, b1, b2, sh,
+  for (int j = 0; j < nb; ++j) {
+    bad |= lu_diag64(blk(j, j), m, size(j), b0, b1, b2, s_rcp,
                      scr + ((size_t)blockIdx.x * (kOB2 / kNP) + j) * 2 * kNP * kNP,
                      dinv + dinv_off[leaf] + (size_t)((K0 + j * kNP) / kDB) * 2 * kDB * kDB);
-    const int nb = (D + kNP - 1) / kNP;
-    auto size = [&](int i) { return min(kNP, D - i * kNP); };
+    // L_ij = A_ij U_jj^{-1}
     for (int i = j + 1; i < nb; ++i) {
       __syncthreads();
-      stage64(b2, blk(i, j), m, size(i), kNP);
+      stage64<kNPT>(b2, blk(i, j), m, size(i), kNP);
       cp_async_commit();
       cp_async_wait<0>();
       __syncthreads();
       double acc[4][2][2] = {};
-      dmma_tile<4, 2, kPP, kPP, kNP>(acc, b2 + tile_r0(), b1 + tile_c0() * kPP);
+      dmma_tile<4, 2, kPP, kPP, kNP>(acc, b2 + r0, b1 + c0 * kPP);
       double* out = blk(i, j);
       tile_each(acc, [&](int r, int c, double v) {
-        if (r < size(i)) {
+        if (r0 + r < size(i)) {
           if (!(fabs(v) <= kNoPivBound)) bad = true;
-          out[(size_t)c * m + r] = v;
+          out[(size_t)(c0 + c) * m + r0 + r] = v;
         }
       });
     }
-    for (int k = j + 1; k < nb; ++k) {
-      __syncthreads();
-      stage64(b1, blk(j, k), m, kNP, size(k));
-      stage64(b2, blk(j + 1, j), m, size(j + 1), kNP);
+    // U_jk = L_jj^{-1} A_jk, A_jk one block ahead in b1 and b2
+    __syncthreads();
+    if (j + 1 < nb) {
+      stage64<kNPT>(b1, blk(j, j + 1), m, kNP, size(j + 1));
       cp_async_commit();
+    }
+    for (int k = j + 1; k < nb; ++k) {
       cp_async_wait<0>();
       __syncthreads();
-      {
-        double acc[4][2][2] = {};
-        dmma_tile<4, 2, kPP, kPP, kNP>(acc, b0 + tile_r0(), b1 + tile_c0() * kPP);
-        __syncthreads();  // A_jk is read
-        double* out = blk(j, k);
-        tile_each(acc, [&](int r, int c, double v) {
-          b1[c * kPP + r] = v;
-          if (c < size(k)) out[(size_t)c * m + r] = v;
-        });
+      if (k + 1 < nb) {
+        stage64<kNPT>((k - j) & 1 ? b2 : b1, blk(j, k + 1), m, kNP, size(k + 1));
+        cp_async_commit();
       }
-      __syncthreads();
-      for (int i = j + 1; i < nb; ++i) {
+      double acc[4][2][2] = {};
+      dmma_tile<4, 2, kPP, kPP, kNP>(acc, b0 + r0, ((k - j) & 1 ? b1 : b2) + c0 * kPP);
+      double* out = blk(j, k);
+      tile_each(acc, [&](int r, int c, double v) {
+        if (c0 + c < size(k)) out[(size_t)(c0 + c) * m + r0 + r] = v;
+      });
+    }
+    // A_ik -= L_ij U_jk, L_ij one block ahead in b0 and b2
+    __syncthreads();
+    int buf = 0;
+    for (int k = j + 1; k < nb; ++k) {
+      if (k > j + 1) __syncthreads();  // b1 is read
+      stage64<kNPT>(b1, blk(j, k), m, kNP, size(k));
+      if (k == j + 1) stage64<kNPT>(b0, blk(j + 1, j), m, size(j + 1), kNP);
+      cp_async_commit();
+      for (int i = j + 1; i < nb; ++i, buf ^= 1) {
         double acc[4][2][2];
         double* out = blk(i, k);
         tile_each(acc, [&](int r, int c, double& v) {
-          v = r < size(i) && c < size(k) ? -out[(size_t)c * m + r] : 0.0;
+          v = r0 + r < size(i) && c0 + c < size(k) ? -out[(size_t)(c0 + c) * m + r0 + r] : 0.0;
         });
-        if (i > j + 1) {
-          stage64(b2, blk(i, j), m, size(i), kNP);
+        cp_async_wait<0>();
+        __syncthreads();
+        const int in = i + 1 < nb ? i + 1 : j + 1;  // the next block of the cycle over i
+        if (i + 1 < nb || k + 1 < nb) {
+          stage64<kNPT>(buf ? b0 : b2, blk(in, j), m, size(in), kNP);
           cp_async_commit();
-          cp_async_wait<0>();
-          __syncthreads();
         }
-        dmma_tile<4, 2, kPP, kPP, kNP>(acc, b2 + tile_r0(), b1 + tile_c0() * kPP);
+        dmma_tile<4, 2, kPP, kPP, kNP>(acc, (buf ? b2 : b0) + r0, b1 + c0 * kPP);
         tile_each(acc, [&](int r, int c, double v) {
-          if (r < size(i) && c < size(k)) out[(size_t)c * m + r] = -v;
+          if (r0 + r < size(i) && c0 + c < size(k)) out[(size_t)(c0 + c) * m + r0 + r] = -v;
         });
-        if (i + 1 < nb) __syncthreads();  // b2 is read
       }
     }
     __syncthreads();
@@ -1569,69 +1629,70 @@ __global__ void __launch_bounds__(kNPT, 2) lu_np_block_kernel(
   if (__syncthreads_or(bad) && tid == 0) fail[leaf] = 1;
 }
 
-// item = (leaf, slot, kind, off) of a leaf with m > K0 + 256: kind 0, rows
+// item = (leaf, slot, kind, off) of a leaf with m > K0 + kOB2: kind 0, rows
 // [off, off + 64) of L21; kind 1, columns [off, off + 64) of U12.  slot = the
 // leaf's position in the block kernel's launch (its scratch).  The chunk lies
-// in shared memory; the ten 64 x 64 blocks of the diagonal block's factors and
-// inverses stream through two buffers:
+// in shared memory, the 64 x 64 blocks of the diagonal block's factors and
+// inverses pass through one buffer (104 KB together, so that two CTAs share
+// an SM and fill each other's waits):
 //   kind 0: Y_j = Y_j U_jj^{-1}, then Y_i -= Y_j U_ji for i > j (columns by 64),
 //   kind 1: X_j = L_jj^{-1} X_j, then X_i -= L_ij X_j for i > j (rows by 64).
-constexpr int kTP1 = kOB2 + 4;  // kind 1: pitch of a column of 256
-constexpr size_t kNPBorderSmem = sizeof(double) * (kOB2 * kPP + 2 * kNB2);
+constexpr int kTP1 = kOB2 + 4;  // kind 1: pitch of a column of the chunk
+constexpr size_t kNPBorderSmem = sizeof(double) * (kOB2 * kPP + kNB2);
 
 template <int KIND>
-__device__ __forceinline__ bool lu_border(double* T, double* ring, double* A, int m, int K0,
+__device__ __forceinline__ bool lu_border(double* T, double* f, double* A, int m, int K0,
                                           int off, const double* S) {
+  constexpr int NB = kOB2 / kNP;
   const int cnt = min(kNP, m - off);
   double* chunk = KIND == 0 ? A + (size_t)K0 * m + off : A + (size_t)off * m + K0;
   const double* F = A + (size_t)K0 * m + K0;  // the factored diagonal block
-  auto stage_factor = [&](int i, int j, int buf) {
-    double* dst = ring + buf * kNB2;
+  // this warp's 32 x 16 tile of a 64 x 64 product
+  const int r0 = 32 * ((int)(threadIdx.x >> 5) & 1), c0 = 16 * (int)(threadIdx.x >> 6);
+  auto stage_factor = [&](int i, int j) {
     if (i == j)
-      stage64(dst, S + (size_t)j * 2 * kNP * kNP + (KIND == 0 ? kNP * kNP : 0), kNP, kNP, kNP);
+      stage64<kNPT>(f, S + (size_t)j * 2 * kNP * kNP + (KIND == 0 ? kNP * kNP : 0), kNP, kNP,
+                    kNP);
     else if (KIND == 0)
-      stage64(dst, F + (size_t)(kNP * i) * m + kNP * j, m, kNP, kNP);
+      stage64<kNPT>(f, F + (size_t)(kNP * i) * m + kNP * j, m, kNP, kNP);
     else
-      stage64(dst, F + (size_t)(kNP * j) * m + kNP * i, m, kNP, kNP);
+      stage64<kNPT>(f, F + (size_t)(kNP * j) * m + kNP * i, m, kNP, kNP);
     cp_async_commit();
   };
   if (KIND == 0) {
 #pragma unroll
-    for (int j = 0; j < kOB2 / kNP; ++j)
-      stage64(T + j * kNB2, chunk + (size_t)(j * kNP) * m, m, cnt, kNP);
+    for (int j = 0; j < NB; ++j)
+      stage64<kNPT>(T + j * kNB2, chunk + (size_t)(j * kNP) * m, m, cnt, kNP);
   } else {
 #pragma unroll
     for (int e = 0; e < kNP * kOB2 / 2 / kNPT; ++e) {
-      const int q = (int)threadIdx.x + kNPT * e, c = q >> 7, r = 2 * (q & 127);
+      const int q = (int)threadIdx.x + kNPT * e, c = q / (kOB2 / 2), r = 2 * (q % (kOB2 / 2));
       const bool ok = c < cnt;
       cp_async16(T + c * kTP1 + r, ok ? chunk + (size_t)c * m + r : chunk, ok);
     }
   }
-  // entry (r, c) of block i of the chunk
+  // entry (r, c) of the warp's tile in block i of the chunk
   auto at = [&](int i, int r, int c) -> double& {
-    return KIND == 0 ? T[i * kNB2 + c * kPP + r] : T[c * kTP1 + i * kNP + r];
+    return KIND == 0 ? T[i * kNB2 + (c0 + c) * kPP + r0 + r]
+                     : T[(c0 + c) * kTP1 + i * kNP + r0 + r];
   };
-  auto multiply = [&](double (&acc)[4][2][2], int j, const double* f) {
+  auto multiply = [&](double (&acc)[4][2][2], int j) {
+    if ((KIND == 0 ? r0 : c0) >= cnt) return;  // past the chunk's edge
     if (KIND == 0)
-      dmma_tile<4, 2, kPP, kPP, kNP>(acc, T + j * kNB2 + tile_r0(), f + tile_c0() * kPP);
+      dmma_tile<4, 2, kPP, kPP, kNP>(acc, T + j * kNB2 + r0, f + c0 * kPP);
     else
-      dmma_tile<4, 2, kPP, kTP1, kNP>(acc, f + tile_r0(), T + tile_c0() * kTP1 + j * kNP);
+      dmma_tile<4, 2, kPP, kTP1, kNP>(acc, f + r0, T + c0 * kTP1 + j * kNP);
   };
   bool bad = false;
-  stage_factor(0, 0, 0);
-  int buf = 0;
-  for (int j = 0; j < kOB2 / kNP; ++j)
-    for (int i = j; i < kOB2 / kNP; ++i, buf ^= 1) {
+  for (int j = 0; j < NB; ++j)
+    for (int i = j; i < NB; ++i) {
+      if (i + j > 0) __syncthreads();  // the buffer is read, the chunk written
+      stage_factor(i, j);
       cp_async_wait<0>();
-      __syncthreads();  // this factor has arrived, the other buffer is read
-      if (i + 1 < kOB2 / kNP)
-        stage_factor(i + 1, j, buf ^ 1);
-      else if (j + 1 < kOB2 / kNP)
-        stage_factor(j + 1, j + 1, buf ^ 1);
-      const double* f = ring + buf * kNB2;
+      __syncthreads();
       double acc[4][2][2] = {};
       if (i == j) {
-        multiply(acc, j, f);
+        multiply(acc, j);
         __syncthreads();  // block j is read
         tile_each(acc, [&](int r, int c, double v) {
           if (KIND == 0 && !(fabs(v) <= kNoPivBound)) bad = true;
@@ -1639,26 +1700,20 @@ __device__ __forceinline__ bool lu_border(double* T, double* ring, double* A, in
         });
       } else {
         tile_each(acc, [&](int r, int c, double& v) { v = -at(i, r, c); });
-        multiply(acc, j, f);
+        multiply(acc, j);
         tile_each(acc, [&](int r, int c, double v) { at(i, r, c) = -v; });
       }
     }
   __syncthreads();
-  if (KIND == 0) {
-    for (int q = threadIdx.x; q < kOB2 * kNP; q += kNPT) {
-      const int c = q >> 6, r = q & 63;
-      if (r < cnt) chunk[(size_t)c * m + r] = T[c * kPP + r];
-    }
-  } else {
-    for (int q = threadIdx.x; q < kNP * kOB2; q += kNPT) {
-      const int c = q >> 8, r = q & 255;
-      if (c < cnt) chunk[(size_t)c * m + r] = T[c * kTP1 + r];
-    }
+  for (int q = threadIdx.x; q < kNP * kOB2; q += kNPT) {
+    const int c = KIND == 0 ? q / kNP : q / kOB2, r = KIND == 0 ? q % kNP : q % kOB2;
+    if (KIND == 0 ? r < cnt : c < cnt)
+      chunk[(size_t)c * m + r] = T[c * (KIND == 0 ? kPP : kTP1) + r];
   }
   return bad;
 }
 
-__global__ void __launch_bounds__(kNPT, 1) lu_np_border_kernel(
+__global__ void __launch_bounds__(kNPT, 2) lu_np_border_kernel(
     const int4* __restrict__ items, int K0, const int2* __restrict__ leaf_rng,
     const int64_t* __restrict__ blk_off, double* lu, const double* __restrict__ scr,
     int* __restrict__ fail) {
@@ -1669,9 +1724,9 @@ __global__ void __launch_bounds__(kNPT, 1) lu_np_border_kernel(
   const int m = 2 * leaf_rng[it.x].y;
   double* A = lu + blk_off[it.x];
   const double* S = scr + (size_t)it.y * (kOB2 / kNP) * 2 * kNP * kNP;
-  double* ring = nsm + kOB2 * kPP;
-  const bool bad = it.z == 0 ? lu_border<0>(nsm, ring, A, m, K0, it.w, S)
-                             : lu_border<1>(nsm, ring, A, m, K0, it.w, S);
+  double* f = nsm + kOB2 * kPP;
+  const bool bad = it.z == 0 ? lu_border<0>(nsm, f, A, m, K0, it.w, S)
+                             : lu_border<1>(nsm, f, A, m, K0, it.w, S);
   if (__syncthreads_or(bad) && threadIdx.x == 0) fail[it.x] = 1;
 }
 
@@ -1753,8 +1808,9 @@ __global__ void __launch_bounds__(256, 2) lu_gemm2_kernel(const int4* __restrict
     }
     __syncthreads();
     // all 32 k of the slice: zero-filled past the depth
-    dmma_tile<4, 4, kG2LP, kG2UP, kG2K>(acc, sL + buf * kG2K * kG2LP + wr,
-                                        sU + buf * kG2N * kG2UP + wc * kG2UP);
+    if (r0 + wr < m && c0 + wc < m)  // a warp past the edge leaves the pipe to the others
+      dmma_tile<4, 4, kG2LP, kG2UP, kG2K>(acc, sL + buf * kG2K * kG2LP + wr,
+                                          sU + buf * kG2N * kG2UP + wc * kG2UP);
     if (kc + 2 * kG2K < kd) {  // buffer buf takes the slice two on
       __syncthreads();
       load_slice(kc + 2 * kG2K, buf);
@@ -1881,11 +1937,11 @@ void build_precond(Handle& H, cudaStream_t s) {
     // Right-looking order in outer blocks of kOB2 columns: the diagonal block of
     // every leaf, its L21 and U12 chunks, the trailing update.
     //
-    // Look-ahead: the trailing update of an outer block is split.  The next
-    // outer block's diagonal block, which is factored next, is updated on the
-    // group's stream; the rest on the middle-priority auxiliary stream, beside
-    // that factorisation.  The next block's chunks wait for the auxiliary
-    // stream.
+    // Look-ahead (the large-block group): the trailing update of an outer block
+    // is split.  The next outer block's rows and columns are updated on the
+    // group's stream, the rest on the middle-priority auxiliary stream, beside
+    // the next block's factorisation and chunks, which need only the former.
+    // The next block's own update waits for the auxiliary stream.
     struct Launch {
       // 0 diagonal block, 1 its chunks, 2 update, 3 fork to the auxiliary
       // stream, 4 wait for the auxiliary stream, 5 update on the auxiliary stream
@@ -1893,7 +1949,8 @@ void build_precond(Handle& H, cudaStream_t s) {
       int k0, off, cnt;
     };
     // one group's plan: item lists (uploaded on st) and its launches
-    auto plan_np = [&](const std::vector<int>& order, Handle::NpPlan& B, cudaStream_t st) {
+    auto plan_np = [&](const std::vector<int>& order, Handle::NpPlan& B, cudaStream_t st,
+                       bool la) {
       int gmax = 0;
       for (int l : order) gmax = std::max(gmax, 2 * rng[l].y);
       std::vector<Launch> plan;
@@ -1908,7 +1965,7 @@ void build_precond(Handle& H, cudaStream_t s) {
       };
       bool rest_pending = false;  // an update on the auxiliary stream not yet waited for
       for (int K0 = 0; K0 < gmax; K0 += kOB2) {
-        const int Kend = K0 + kOB2, Knext = Kend + kOB2;
+        const int Kend = K0 + kOB2, Knext = la ? Kend + kOB2 : INT_MAX;
         const size_t d0 = dl.len, p0 = pit.len, g0 = git.len;
         int slot = 0;
         for (int l : order) {
@@ -1919,36 +1976,26 @@ void build_precond(Handle& H, cudaStream_t s) {
             pit.push(make_int4(l, slot, 0, off));
             pit.push(make_int4(l, slot, 1, off));
           }
-          for (int r0 = Kend; r0 < std::min(m, Knext); r0 += kG2M)
-            for (int c0 = Kend; c0 < std::min(m, Knext); c0 += kG2N)
+          for (int r0 = Kend; r0 < m; r0 += kG2M)
+            for (int c0 = Kend; c0 < m && (r0 < Knext || c0 < Knext); c0 += kG2N)
               git.push(make_int4(l, r0, c0, 0));
           ++slot;
         }
         const size_t g1 = git.len;
         for (int l : order) {
           const int m = 2 * rng[l].y;
-          if (m <= Knext) continue;
-          for (int r0 = Kend; r0 < m; r0 += kG2M)
-            for (int c0 = r0 < Knext ? Knext : Kend; c0 < m; c0 += kG2N)
-              git.push(make_int4(l, r0, c0, 0));
+          for (int r0 = Knext; la && r0 < m; r0 += kG2M)
+            for (int c0 = Knext; c0 < m; c0 += kG2N) git.push(make_int4(l, r0, c0, 0));
         }
         emit(0, K0, d0, dl.len);
-        if (rest_pending) {
-          plan.push_back({4, K0, 0, 0});
-          rest_pending = false;
-        }
         emit(1, K0, p0, pit.len);
-        // the fork before the look-ahead tiles' launch (the auxiliary stream
-        // must not wait for it), the rest launched after it (earlier launches
-        // are dispatched first)
-        const bool rest = git.len > g1;
-        if (rest) plan.push_back({3, K0, 0, 0});
+        if (git.len > g1) plan.push_back({3, K0, 0, 0});
+        if (rest_pending) plan.push_back({4, K0, 0, 0});
         emit(2, K0, g0, g1);
-        if (rest) {
-          emit(5, K0, g1, git.len);
-          rest_pending = true;
-        }
+        rest_pending = git.len > g1;
+        emit(5, K0, g1, git.len);
       }
+      if (rest_pending) plan.push_back({4, gmax, 0, 0});
       dl.upload(B.dleaves, st);
       pit.upload(B.pitems, st);
       git.upload(B.gitems, st);
@@ -2009,8 +2056,8 @@ void build_precond(Handle& H, cudaStream_t s) {
     big.st = H.lu_hi;
     small.B = &H.pc_np[1];
     small.st = H.lu_small;
-    if (!grp[0].empty()) big.plan = plan_np(grp[0], H.pc_np[0], H.lu_hi);
-    if (!grp[1].empty()) small.plan = plan_np(grp[1], H.pc_np[1], H.lu_small);
+    if (!grp[0].empty()) big.plan = plan_np(grp[0], H.pc_np[0], H.lu_hi, true);
+    if (!grp[1].empty()) small.plan = plan_np(grp[1], H.pc_np[1], H.lu_small, false);
     while (big.at < big.plan.size() || small.at < small.plan.size()) {
       if (big.at < big.plan.size()) issue_one(big);
       if (small.at < small.plan.size()) issue_one(small);
