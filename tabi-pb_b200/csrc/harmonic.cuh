@@ -36,6 +36,8 @@
 // 10.4 M, 4.59 -> 0.86 ms.
 #pragma once
 
+#include "fast_math.cuh"
+
 namespace tabi {
 
 // doubles per cluster: per element of degree <= p U, V and the gradients of
@@ -167,76 +169,90 @@ __device__ __forceinline__ double harm_grad(const double* c, int l, int k, bool 
   return 0.5 * (im ? -(low + re(k + 1)) : imc(k - 1) + imc(k + 1));
 }
 
-// out1 and out2 (before 1/(4 pi)) of a target at (x, y, z) from the cluster's
-// centre, unit normal (n0, n1, n2); M: the cluster's harm_size(P) coefficients,
-// 16-byte aligned, read in order.
-template <int P>
-__device__ __forceinline__ void harm_eval(double x, double y, double z, double n0, double n1,
-                                          double n2, double kappa, double inv_eps,
-                                          const double* __restrict__ M, double& out1,
-                                          double& out2) {
+// out1 and out2 (before 1/(4 pi)) of NT targets at (x, y, z) from the cluster's
+// centre, unit normals (n0, n1, n2); M: the cluster's harm_size(P) coefficients,
+// 16-byte aligned, read in order, once for the NT targets.
+template <int P, int NT>
+__device__ __forceinline__ void harm_eval(const double (&x)[NT], const double (&y)[NT],
+                                          const double (&z)[NT], const double (&n0)[NT],
+                                          const double (&n1)[NT], const double (&n2)[NT],
+                                          double kappa, double inv_eps,
+                                          const double* __restrict__ M, double (&out1)[NT],
+                                          double (&out2)[NT]) {
   constexpr int L = P + 1;
-  const double r2 = fma(x, x, fma(y, y, z * z));
-  const double ri = rsqrt(r2), ri2 = ri * ri;
-  const double kr = kappa * (r2 * ri), k2 = kappa * kappa;
-  const double ex = exp(-kr);
-  const double xn = fma(n0, x, fma(n1, y, n2 * z));
-  double c = ri, y0 = ex * ri, y1 = -fma(kr, ex, ex) * ri * ri2;  // c_l, y_l, y_{l+1}
-  double o1 = 0.0, o2 = 0.0, o2y = 0.0;
-  double za[L + 1], zb[L + 1], a[L + 1], b[L + 1];  // Z_{l-1}, Z_{l-2} and (x + iy)^m by m
-  a[0] = 1.0;
-  b[0] = 0.0;
+  const double k2 = kappa * kappa;
+  double r2[NT], ri2[NT], xn[NT], c[NT], y0[NT], y1[NT], o2y[NT];  // c_l, y_l, y_{l+1}
+  double za[NT][L + 1], zb[NT][L + 1], a[NT][L + 1], b[NT][L + 1];  // Z_{l-1}, Z_{l-2}, (x + iy)^m
+#pragma unroll
+  for (int k = 0; k < NT; ++k) {
+    r2[k] = fma(x[k], x[k], fma(y[k], y[k], z[k] * z[k]));
+    const double ri = fast_rsqrt(r2[k]);
+    ri2[k] = ri * ri;
+    const double kr = kappa * (r2[k] * ri);
+    const double ex = exp(-kr);
+    xn[k] = fma(n0[k], x[k], fma(n1[k], y[k], n2[k] * z[k]));
+    c[k] = ri;
+    y0[k] = ex * ri;
+    y1[k] = -fma(kr, ex, ex) * ri * ri2[k];
+    out1[k] = out2[k] = o2y[k] = 0.0;
+    a[k][0] = 1.0;
+    b[k][0] = 0.0;
+  }
 #pragma unroll
   for (int l = 0; l <= L; ++l) {
-    if (l > 0) {
-      a[l] = l == 1 ? x : fma(x, a[l - 1], -y * b[l - 1]);
-      b[l] = l == 1 ? y : fma(x, b[l - 1], y * a[l - 1]);
-    }
-    double su = 0.0, sv = 0.0, gu0 = 0.0, gu1 = 0.0, gu2 = 0.0, gv0 = 0.0, gv1 = 0.0, gv2 = 0.0;
+    // sums over the degree's elements: U, V, grad U_{l+1}, grad V_{l+1}
+    double s[NT][8] = {};
     const double* Ml = l <= P ? M + 8 * l * l : M + 8 * (P + 1) * (P + 1);
-    auto add = [&](int e, double s) {
-      if (l <= P) {
-        const double2* m2 = reinterpret_cast<const double2*>(Ml + 8 * e);
-        const double2 v0 = m2[0], v1 = m2[1], v2 = m2[2], v3 = m2[3];
-        su = fma(s, v0.x, su);
-        sv = fma(s, v0.y, sv);
-        gu0 = fma(s, v1.x, gu0);
-        gu1 = fma(s, v1.y, gu1);
-        gu2 = fma(s, v2.x, gu2);
-        gv0 = fma(s, v2.y, gv0);
-        gv1 = fma(s, v3.x, gv1);
-        gv2 = fma(s, v3.y, gv2);
-      } else {
-        const double2 v0 = *reinterpret_cast<const double2*>(Ml + 2 * e);
-        su = fma(s, v0.x, su);
-        sv = fma(s, v0.y, sv);
-      }
-    };
 #pragma unroll
     for (int m = 0; m <= l; ++m) {
-      const double zl = m == l       ? 1.0
-                        : m == l - 1 ? z
-                                     : fma(z, za[m], -(harm_b(l, m) * r2) * zb[m]);
-      if (m < l) zb[m] = za[m];
-      za[m] = zl;
-      add(m == 0 ? 0 : 2 * m - 1, m == 0 ? zl : m == l ? a[m] : zl * a[m]);
-      if (m > 0) add(2 * m, m == l ? b[m] : zl * b[m]);
+      double zl[NT];
+#pragma unroll
+      for (int k = 0; k < NT; ++k) {
+        if (m == l && l > 0) {
+          a[k][l] = l == 1 ? x[k] : fma(x[k], a[k][l - 1], -y[k] * b[k][l - 1]);
+          b[k][l] = l == 1 ? y[k] : fma(x[k], b[k][l - 1], y[k] * a[k][l - 1]);
+        }
+        zl[k] = m == l       ? 1.0
+                : m == l - 1 ? z[k]
+                             : fma(z[k], za[k][m], -(harm_b(l, m) * r2[k]) * zb[k][m]);
+        if (m < l) zb[k][m] = za[k][m];
+        za[k][m] = zl[k];
+      }
+#pragma unroll
+      for (int im = 0; im < (m > 0 ? 2 : 1); ++im) {
+        const int e = m == 0 ? 0 : 2 * m - 1 + im;
+        const double2* v = reinterpret_cast<const double2*>(Ml + (l <= P ? 8 : 2) * e);
+#pragma unroll
+        for (int q = 0; q < (l <= P ? 4 : 1); ++q) {
+          const double2 w = v[q];
+#pragma unroll
+          for (int k = 0; k < NT; ++k) {
+            const double t = im == 0 ? a[k][m] : b[k][m];
+            const double f = m == 0 ? zl[k] : m == l ? t : zl[k] * t;
+            s[k][2 * q] = fma(f, w.x, s[k][2 * q]);
+            s[k][2 * q + 1] = fma(f, w.y, s[k][2 * q + 1]);
+          }
+        }
+      }
     }
-    o1 = fma(c, su, fma(y0, sv, o1));
-    c *= -(double)(2 * l + 1) * ri2;
-    double tu = xn * su, tv = xn * sv;
-    if (l <= P) {
-      tu = fma(n0, gu0, fma(n1, gu1, fma(n2, gu2, tu)));
-      tv = fma(n0, gv0, fma(n1, gv1, fma(n2, gv2, tv)));
+#pragma unroll
+    for (int k = 0; k < NT; ++k) {
+      out1[k] = fma(c[k], s[k][0], fma(y0[k], s[k][1], out1[k]));
+      c[k] *= -(double)(2 * l + 1) * ri2[k];
+      double tu = xn[k] * s[k][0], tv = xn[k] * s[k][1];
+      if (l <= P) {
+        tu = fma(n0[k], s[k][2], fma(n1[k], s[k][3], fma(n2[k], s[k][4], tu)));
+        tv = fma(n0[k], s[k][5], fma(n1[k], s[k][6], fma(n2[k], s[k][7], tv)));
+      }
+      out2[k] = fma(c[k], tu, out2[k]);
+      o2y[k] = fma(y1[k], tv, o2y[k]);
+      const double yn = fma(k2, y0[k], -(double)(2 * l + 3) * y1[k]) * ri2[k];
+      y0[k] = y1[k];
+      y1[k] = yn;
     }
-    o2 = fma(c, tu, o2);
-    o2y = fma(y1, tv, o2y);
-    const double yn = fma(k2, y0, -(double)(2 * l + 3) * y1) * ri2;
-    y0 = y1;
-    y1 = yn;
   }
-  out1 = o1;
-  out2 = fma(inv_eps, o2y, o2);
+#pragma unroll
+  for (int k = 0; k < NT; ++k) out2[k] = fma(inv_eps, o2y[k], out2[k]);
 }
 
 }  // namespace tabi

@@ -25,7 +25,7 @@
 #include <algorithm>
 
 #include "bie_kernels.cuh"
-#include "fast_exp.cuh"
+#include "fast_math.cuh"
 #include "harmonic.cuh"
 #include "reduce.cuh"
 #include "taylor_gen.cuh"
@@ -223,9 +223,11 @@ __global__ void __launch_bounds__(128) harm_final_kernel(const int2* __restrict_
 }
 
 // ---- far field
-// FP64 (harmonic.cuh)
-template <int P>
-__global__ void __launch_bounds__(64) far_harm_kernel(
+// FP64 (harmonic.cuh): one block per (cluster, up to 64 NT of its targets), NT =
+// far_pair(P) targets per thread, which share every coefficient's shared load.
+
+template <int P, int NT>
+__global__ void __launch_bounds__(kFarThreads) far_harm_kernel(
     const WorkItem* __restrict__ work, const int2* __restrict__ ent,
     const double* __restrict__ mw, const double* __restrict__ nd_mid,
     const double* __restrict__ px, const double* __restrict__ py, const double* __restrict__ pz,
@@ -234,16 +236,31 @@ __global__ void __launch_bounds__(64) far_harm_kernel(
   __shared__ __align__(16) double sm[harm_size(P)];
   const WorkItem wi = work[blockIdx.x];
   const double* src = mw + (size_t)wi.mslot * harm_size(P);
-  for (int q = threadIdx.x; q < harm_size(P); q += blockDim.x) sm[q] = src[q];
+  for (int q = threadIdx.x; q < harm_size(P) / 2; q += kFarThreads)
+    reinterpret_cast<double2*>(sm)[q] = reinterpret_cast<const double2*>(src)[q];
+  const double mx = nd_mid[3 * wi.node], my = nd_mid[3 * wi.node + 1], mz = nd_mid[3 * wi.node + 2];
+  double x[NT], y[NT], z[NT], n0[NT], n1[NT], n2[NT], o1[NT], o2[NT];
+  int slot[NT];
+#pragma unroll
+  for (int k = 0; k < NT; ++k) {
+    // a thread past the end repeats the last target and writes nothing
+    const int2 e = ent[wi.start + min((int)threadIdx.x + kFarThreads * k, wi.count - 1)];
+    slot[k] = e.y;
+    // COMP_TCOEFF :707-709: target - mid
+    x[k] = px[e.x] - mx;
+    y[k] = py[e.x] - my;
+    z[k] = pz[e.x] - mz;
+    n0[k] = nx[e.x];
+    n1[k] = ny[e.x];
+    n2[k] = nz[e.x];
+  }
   __syncthreads();
-  if ((int)threadIdx.x >= wi.count) return;
-  const int2 e = ent[wi.start + threadIdx.x];
-  const int t = e.x;
-  // COMP_TCOEFF :707-709: target - mid
-  double o1, o2;
-  harm_eval<P>(px[t] - nd_mid[3 * wi.node], py[t] - nd_mid[3 * wi.node + 1],
-               pz[t] - nd_mid[3 * wi.node + 2], nx[t], ny[t], nz[t], kappa, inv_eps, sm, o1, o2);
-  res[e.y] = make_double2(o1 * kOneOver4Pi, o2 * kOneOver4Pi);
+  if ((int)(threadIdx.x & ~31u) >= wi.count) return;  // a warp without targets
+  harm_eval<P, NT>(x, y, z, n0, n1, n2, kappa, inv_eps, sm, o1, o2);
+#pragma unroll
+  for (int k = 0; k < NT; ++k)
+    if ((int)threadIdx.x + kFarThreads * k < wi.count)
+      res[slot[k]] = make_double2(o1[k] * kOneOver4Pi, o2[k] * kOneOver4Pi);
 }
 
 // FP32 (mixed precision): the target-to-centre offset is formed in FP64 and
@@ -267,8 +284,8 @@ __global__ void __launch_bounds__(64, P == 3 ? 8 : 1) far_kernel(const WorkItem*
   const float* src = mw + (size_t)wi.mslot * 16 * NT;
   for (int q = threadIdx.x; q < 16 * NT; q += blockDim.x) smw[q] = src[q];
   __syncthreads();
-  if ((int)threadIdx.x >= wi.count) return;
-  int2 e = ent[wi.start + threadIdx.x];
+  for (int k = threadIdx.x; k < wi.count; k += blockDim.x) {
+  int2 e = ent[wi.start + k];
   int t = e.x;
   // COMP_TCOEFF :707-709: dx = target - mid
   float dx = (float)(px[t] - nd_mid[3 * wi.node]);
@@ -278,6 +295,7 @@ __global__ void __launch_bounds__(64, P == 3 ? 8 : 1) far_kernel(const WorkItem*
   far_eval<P, float>(dx, dy, dz, kappa, smw, (float)nx[t], (float)ny[t], (float)nz[t], eps,
                      1.f / eps, o1, o2);
   res[e.y] = make_double2((double)o1 * kOneOver4Pi, (double)o2 * kOneOver4Pi);
+  }
 }
 
 // ---- near field
@@ -290,33 +308,34 @@ __global__ void __launch_bounds__(64, P == 3 ? 8 : 1) far_kernel(const WorkItem*
 //   y2: i^3 ((m.v0 - 3 i^2 (m.d)(v0.d))(t - 1) - kappa^2 (m.d)(v0.d) e
 //            + w (v0.d)(1 - t/eps)),
 // times 1/(4 pi) at the end: 37 FP64 instructions beside the reciprocal root and
-// the exponential (fast_exp.cuh), against 45 of the factored form of each
-// kernel.  Only blocks in which a target meets its own leaf test for the own
-// face.  Measured beside the far field, 73.5 M pairs: 0.50 -> 0.32 ms; 193 M
+// the exponential (fast_math.cuh), against 45 of the factored form of each
+// kernel.  Only blocks in which a target meets its own leaf, or kappa times a
+// distance may leave the exponential's table, test for either in the loop.
+// Measured beside the far field, 73.5 M pairs: 0.50 -> 0.32 ms; 193 M
 // pairs: 1.36 -> 0.90 ms; 0.55 M pairs (1,272 targets, one thread each gave 27
 // blocks): 49 -> 20 us.
 constexpr int kNearThreads = 128;
-constexpr int kNearTile = 512;
+constexpr int kNearTile = 256;
 
-template <int S, bool OWN>
+template <int S, bool CHECK>
 __device__ __forceinline__ void near_tile(const double2 (*src)[4], const double* tab, int cnt,
                                           int self, double tx, double ty, double tz, double vx,
                                           double vy, double vz, double kappa, double eps,
                                           double inv_eps, double& p1, double& p2) {
   const double k2 = kappa * kappa;
-#pragma unroll 2
+#pragma unroll 4
   for (int q = (int)threadIdx.x % S; q < cnt; q += S) {
     const double2 a = src[q][0], b = src[q][1], c = src[q][2], g = src[q][3];
     double dx = a.x - tx, dy = a.y - ty, dz = b.x - tz;
     double mx = c.x, my = c.y, mz = g.x, w = b.y;
-    if (OWN && q == self) {  // the own face: no contribution, and no 1/0
+    if (CHECK && q == self) {  // the own face: no contribution, and no 1/0
       dx = 1.0;
       mx = my = mz = w = 0.0;
     }
     const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
-    const double i = rsqrt(r2), i2 = i * i;
+    const double i = fast_rsqrt(r2), i2 = i * i;
     const double kr = kappa * (r2 * i);
-    const double e = exp_neg(kr, tab);
+    const double e = exp_neg<CHECK>(kr, tab);
     const double t = fma(kr, e, e);
     const double md = fma(mx, dx, fma(my, dy, mz * dz));
     const double vd = fma(vx, dx, fma(vy, dy, vz * dz));
@@ -331,9 +350,10 @@ __device__ __forceinline__ void near_tile(const double2 (*src)[4], const double*
 }
 
 template <int S>
-__global__ void __launch_bounds__(kNearThreads) near_kernel(
+__global__ void __launch_bounds__(kNearThreads, 5) near_kernel(
     const WorkItem* __restrict__ work, const int2* __restrict__ ent,
     const int* __restrict__ nd_ibeg, const int* __restrict__ nd_num,
+    const double* __restrict__ nd_mid, const double* __restrict__ nd_rad,
     const double* __restrict__ px, const double* __restrict__ py,
     const double* __restrict__ pz, const double* __restrict__ nx,
     const double* __restrict__ ny, const double* __restrict__ nz,
@@ -350,7 +370,13 @@ __global__ void __launch_bounds__(kNearThreads) near_kernel(
   const int2 ent_k = ent[wi.start + min(k, wi.count - 1)];
   const int t = ent_k.x;
   const double tx = px[t], ty = py[t], tz = pz[t], vx = nx[t], vy = ny[t], vz = nz[t];
-  const bool meets_own = __syncthreads_or(t >= ib && t < ib + nsrc);
+  const double far_end =
+      sqrt((tx - nd_mid[3 * wi.node]) * (tx - nd_mid[3 * wi.node]) +
+           (ty - nd_mid[3 * wi.node + 1]) * (ty - nd_mid[3 * wi.node + 1]) +
+           (tz - nd_mid[3 * wi.node + 2]) * (tz - nd_mid[3 * wi.node + 2])) +
+      nd_rad[wi.node];  // no face of the leaf is further from the target
+  const bool check = __syncthreads_or((t >= ib && t < ib + nsrc) ||
+                                      !(kappa * far_end < 0.99 * kExpTabEnd));
   const double inv_eps = 1.0 / eps;
   double p1 = 0.0, p2 = 0.0;
   for (int b0 = 0; b0 < nsrc; b0 += kNearTile) {
@@ -366,7 +392,7 @@ __global__ void __launch_bounds__(kNearThreads) near_kernel(
     }
     __syncthreads();
     if (own) {
-      if (meets_own)
+      if (check)
         near_tile<S, true>(src, tab, cnt, t - (ib + b0), tx, ty, tz, vx, vy, vz, kappa, eps,
                            inv_eps, p1, p2);
       else
@@ -547,7 +573,7 @@ void launch_far(Handle& H, bool f32, cudaStream_t s) {
         fw, fe, H.d_mwf.p, T.d_mid.p, H.d_x.p, H.d_y.p, H.d_z.p,
         H.d_nx.p, H.d_ny.p, H.d_nz.p, (float)H.prm.kappa, (float)eps, H.d_res.p);
   else
-    far_harm_kernel<P><<<nw, 64, 0, s>>>(
+    far_harm_kernel<P, far_pair(P)><<<nw, kFarThreads, 0, s>>>(
         fw, fe, H.d_mw.p, T.d_mid.p, H.d_x.p, H.d_y.p, H.d_z.p,
         H.d_nx.p, H.d_ny.p, H.d_nz.p, H.prm.kappa, 1.0 / eps, H.d_res.p);
 }
@@ -659,8 +685,8 @@ void matvec_dev(Handle& H, const double* x, double* y, cudaStream_t s, bool chec
     TABI_K(K_NEAR, sn);
     auto launch = [&](auto* kernel) {
       kernel<<<nnw, kNearThreads, 0, sn>>>(
-          nwk, nent, T.d_ibeg.p, T.d_num.p, H.d_x.p, H.d_y.p, H.d_z.p, H.d_nx.p, H.d_ny.p,
-          H.d_nz.p, H.d_area.p, x, n, H.prm.kappa, H.prm.eps1 / H.prm.eps0, H.d_res.p);
+          nwk, nent, T.d_ibeg.p, T.d_num.p, T.d_mid.p, T.d_rad.p, H.d_x.p, H.d_y.p, H.d_z.p,
+          H.d_nx.p, H.d_ny.p, H.d_nz.p, H.d_area.p, x, n, H.prm.kappa, H.prm.eps1 / H.prm.eps0, H.d_res.p);
     };
     switch (T.near_split) {
       case 1: launch(near_kernel<1>); break;

@@ -18,7 +18,7 @@
 #include <optional>
 #include <climits>
 
-#include "bie_kernels.cuh"
+#include "fast_math.cuh"
 #include "tabi_impl.cuh"
 
 namespace tabi {
@@ -27,44 +27,64 @@ namespace {
 
 constexpr int kAsmCols = 8;
 
-// grid: one block per (leaf, 8-column tile); tiles given as (leaf, j0)
+// The four kernels of one pair times -A_j (d = r_j - r_i, m = A_j v_j; the near
+// field's forms, see matvec.cu), 1/(4 pi) included in A_j.
+__device__ __forceinline__ void asm_pair(double dx, double dy, double dz, double vx, double vy,
+                                         double vz, double mx, double my, double mz, double A,
+                                         double kappa, double eps, double inv_eps,
+                                         const double* tab, double& K1, double& K2, double& K3,
+                                         double& K4) {
+  const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+  const double i = fast_rsqrt(r2), i2 = i * i, i3 = i * i2;
+  const double kr = kappa * (r2 * i);
+  const double e = exp_neg(kr, tab);
+  const double t = fma(kr, e, e);
+  const double md = fma(mx, dx, fma(my, dy, mz * dz));
+  const double vd = fma(vx, dx, fma(vy, dy, vz * dz));
+  const double mv = fma(mx, vx, fma(my, vy, mz * vz));
+  const double mvd = md * vd;
+  K1 = -(i3 * md) * fma(-eps, t, 1.0);
+  K2 = -(i * A) * (1.0 - e);
+  K3 = -i3 * fma(-(kappa * kappa) * e, mvd, fma(-3.0 * i2, mvd, mv) * (t - 1.0));
+  K4 = -(i3 * A) * vd * fma(-inv_eps, t, 1.0);
+}
+
+// One block per (leaf, 8 columns), tiles given as (leaf, j0).  A warp takes 32
+// rows of one column at a time, so that leaves of any size keep the block's
+// warps busy (with a thread per row the mean leaf of 160 left 96 of 256
+// idle).
 __global__ void __launch_bounds__(256) assemble_kernel(
     const int2* __restrict__ tiles, const int2* __restrict__ leaf_rng,
     const int64_t* __restrict__ blk_off, const double* __restrict__ px,
     const double* __restrict__ py, const double* __restrict__ pz, const double* __restrict__ nx,
     const double* __restrict__ ny, const double* __restrict__ nz,
     const double* __restrict__ area, double kappa, double eps, double* __restrict__ lu) {
-  int2 tl = tiles[blockIdx.x];
-  int2 lr = leaf_rng[tl.x];
-  int ib = lr.x, n = lr.y, m = 2 * n;
+  __shared__ double tab[kExpTab];
+  exp_table_fill(tab);
+  __syncthreads();
+  const int2 tl = tiles[blockIdx.x];
+  const int2 lr = leaf_rng[tl.x];
+  const int ib = lr.x, n = lr.y, m = 2 * n;
   double* A = lu + blk_off[tl.x];
   const double pre1 = 0.5 * (1.0 + eps), pre2 = 0.5 * (1.0 + 1.0 / eps);
   const double inv_eps = 1.0 / eps;
-  for (int jj = 0; jj < kAsmCols; ++jj) {
-    int j = tl.y + jj;
-    if (j >= n) break;
-    double sx = px[ib + j], sy = py[ib + j], sz = pz[ib + j];
-    double vx = nx[ib + j], vy = ny[ib + j], vz = nz[ib + j];
-    double Aj = area[ib + j];
+  const int lane = threadIdx.x & 31, cols = min(kAsmCols, n - tl.y);
+  for (int q = threadIdx.x >> 5; q < cols * ((n + 31) >> 5); q += 8) {
+    const int j = tl.y + q % cols, i = 32 * (q / cols) + lane;
+    if (i >= n) continue;
     double* c1 = A + (size_t)j * m;        // column j
     double* c2 = A + (size_t)(j + n) * m;  // column j + n
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      if (i == j) {
-        c1[i] = pre1;
-        c1[i + n] = 0.0;
-        c2[i] = 0.0;
-        c2[i + n] = pre2;
-        continue;
-      }
-      int t = ib + i;
-      double K1, K2, K3, K4;
-      bie4<double>(sx - px[t], sy - py[t], sz - pz[t], nx[t], ny[t], nz[t], vx, vy, vz, kappa,
-                   eps, inv_eps, K1, K2, K3, K4);
-      c1[i] = -K1 * Aj;
-      c1[i + n] = -K2 * Aj;
-      c2[i] = -K3 * Aj;
-      c2[i + n] = -K4 * Aj;
+    double K1 = pre1, K2 = 0.0, K3 = 0.0, K4 = pre2;
+    if (i != j) {
+      const int t = ib + i, s = ib + j;
+      const double Aj = area[s] * kOneOver4Pi;
+      asm_pair(px[s] - px[t], py[s] - py[t], pz[s] - pz[t], nx[t], ny[t], nz[t], Aj * nx[s],
+               Aj * ny[s], Aj * nz[s], Aj, kappa, eps, inv_eps, tab, K1, K2, K3, K4);
     }
+    c1[i] = K1;
+    c1[i + n] = K2;
+    c2[i] = K3;
+    c2[i + n] = K4;
   }
 }
 

@@ -12,6 +12,7 @@
 #include <cmath>
 #include <vector>
 
+#include "fast_math.cuh"
 #include "tabi_impl.cuh"
 
 namespace tabi {
@@ -40,6 +41,18 @@ __device__ __forceinline__ double heron(double aa, double bb, double cc) {
   double p = __dmul_rn(__dmul_rn(__dmul_rn(s, __dsub_rn(s, aa)), __dsub_rn(s, bb)),
                        __dsub_rn(s, cc));
   return __dsqrt_rn(p);
+}
+
+// b1 and b2 of one (face, atom) pair before the factors 1/(4 pi) and 1/eps0:
+// q/rs and q (v0.d)/rs^3, 20 FP64 instructions
+__device__ __forceinline__ void rhs_pair(double4 a, const double* r0, const double* v0,
+                                         double& b1, double& b2) {
+  const double dx = a.x - r0[0], dy = a.y - r0[1], dz = a.z - r0[2];
+  const double inv = fast_rsqrt(fma(dx, dx, fma(dy, dy, dz * dz)));
+  const double vd = fma(v0[0], dx, fma(v0[1], dy, v0[2] * dz));
+  const double t = a.w * inv;
+  b1 += t;
+  b2 = fma(t * (inv * inv), vd, b2);
 }
 
 // atoms4: (x, y, z, q) per atom
@@ -76,7 +89,6 @@ __global__ void __launch_bounds__(kFaceThreads) form_matrix_kernel(
     oarea[i] = heron(dist_rn(r[0], r[1]), dist_rn(r[0], r[2]), dist_rn(r[1], r[2]));
   }
   double b1 = 0.0, b2 = 0.0;
-  const double inv4pi = kOneOver4Pi;
   for (int a0 = 0; a0 < nchr; a0 += kAtomTile) {
     int cnt = min(kAtomTile, nchr - a0);
     __syncthreads();
@@ -86,21 +98,12 @@ __global__ void __launch_bounds__(kFaceThreads) form_matrix_kernel(
     }
     __syncthreads();
     if (own)
-      for (int q = 0; q < cnt; ++q) {
-        double4 a = sa[q];
-        double dx = a.x - r0[0], dy = a.y - r0[1], dz = a.z - r0[2];
-        double rs2 = fma(dx, dx, fma(dy, dy, dz * dz));
-        double inv = rsqrt(rs2);
-        double G0 = inv4pi * inv;                                          // 1/(4 pi rs)
-        double cosr = fma(v0[0], dx, fma(v0[1], dy, v0[2] * dz)) * inv;    // cos_theta
-        double G1 = cosr * inv * inv * inv4pi;                             // cos/rs^2/(4 pi)
-        b1 = fma(a.w, G0, b1);
-        b2 = fma(a.w, G1, b2);
-      }
+#pragma unroll 4
+      for (int q = 0; q < cnt; ++q) rhs_pair(sa[q], r0, v0, b1, b2);
   }
   if (own) {
-    b[i] = b1 / eps0;
-    b[nface + i] = b2 / eps0;
+    b[i] = b1 * kOneOver4Pi / eps0;
+    b[nface + i] = b2 * kOneOver4Pi / eps0;
   }
 }
 
@@ -135,31 +138,30 @@ __global__ void __launch_bounds__(kFaceThreads) rhs_kernel(const double* __restr
     }
     __syncthreads();
     if (own)
-      for (int q = 0; q < cnt; ++q) {
-        double4 a = sa[q];
-        double dx = a.x - r0[0], dy = a.y - r0[1], dz = a.z - r0[2];
-        double inv = rsqrt(fma(dx, dx, fma(dy, dy, dz * dz)));
-        double cosr = fma(v0[0], dx, fma(v0[1], dy, v0[2] * dz)) * inv;
-        b1 = fma(a.w, kOneOver4Pi * inv, b1);
-        b2 = fma(a.w, cosr * inv * inv * kOneOver4Pi, b2);
-      }
+#pragma unroll 4
+      for (int q = 0; q < cnt; ++q) rhs_pair(sa[q], r0, v0, b1, b2);
   }
   if (own) {
-    b[i] = b1 / eps0;
-    b[nface + i] = b2 / eps0;
+    b[i] = b1 * kOneOver4Pi / eps0;
+    b[nface + i] = b2 * kOneOver4Pi / eps0;
   }
 }
 
 constexpr int kEA = 8;  // atoms per energy block
 constexpr int kET = 256;
 
-// potential_molecule (main.f90:614-657) for kEA atoms per block
+// potential_molecule (main.f90:614-657) for kEA atoms per block, bound by the
+// FP64 pipe: 34 instructions per (face, atom) with the kernels formed as sums
+// over the weighted source (as in the near field) and the table exponential
 __global__ void __launch_bounds__(kET) energy_kernel(
     const double* __restrict__ px, const double* __restrict__ py, const double* __restrict__ pz,
     const double* __restrict__ nx, const double* __restrict__ ny, const double* __restrict__ nz,
     const double* __restrict__ area, const double* __restrict__ x, int n,
     const double* __restrict__ atoms4, int nchr, double kappa, double eps,
     double* __restrict__ ptl) {
+  __shared__ double tab[kExpTab];
+  exp_table_fill(tab);
+  __syncthreads();
   int a0 = blockIdx.x * kEA;
   double ax[kEA], ay[kEA], az[kEA], acc[kEA];
 #pragma unroll
@@ -171,25 +173,20 @@ __global__ void __launch_bounds__(kET) energy_kernel(
     acc[k] = 0.0;
   }
   for (int j = blockIdx.y * blockDim.x + threadIdx.x; j < n; j += gridDim.y * blockDim.x) {
-    double rx = px[j], ry = py[j], rz = pz[j];
-    double vx = nx[j], vy = ny[j], vz = nz[j];
-    double A = area[j];
-    double w1 = A * x[j], w2 = A * x[n + j];
+    const double rx = px[j], ry = py[j], rz = pz[j];
+    const double A = area[j], w1 = A * x[j], w = A * x[n + j];
+    const double mx = w1 * nx[j], my = w1 * ny[j], mz = w1 * nz[j];
 #pragma unroll
     for (int k = 0; k < kEA; ++k) {
-      double dx = rx - ax[k], dy = ry - ay[k], dz = rz - az[k];
-      double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
-      double inv = rsqrt(r2);
-      double rs = r2 * inv;
-      double G0 = kOneOver4Pi * inv;
-      double kr = kappa * rs;
-      double e = exp(-kr);
-      double c = fma(vx, dx, fma(vy, dy, vz * dz)) * inv;
-      double tp1 = G0 * inv;
-      double tp2 = (1.0 + kr) * e;
-      double H1 = (c * tp1) * fma(-eps, tp2, 1.0);  // G1 - eps G2
-      double H2 = G0 * (1.0 - e);                   // G0 - Gk
-      acc[k] = fma(H1, w1, fma(H2, w2, acc[k]));
+      const double dx = rx - ax[k], dy = ry - ay[k], dz = rz - az[k];
+      const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+      const double i = fast_rsqrt(r2);
+      const double kr = kappa * (r2 * i);
+      const double e = exp_neg(kr, tab);
+      const double t = fma(kr, e, e);
+      const double md = fma(mx, dx, fma(my, dy, mz * dz));
+      // (G1 - eps G2) w1 + (G0 - Gk) w without 1/(4 pi)
+      acc[k] = fma(i, fma(i * i * md, fma(-eps, t, 1.0), fma(-e, w, w)), acc[k]);
     }
   }
   __shared__ double s[kEA][kET / 32];
@@ -204,7 +201,7 @@ __global__ void __launch_bounds__(kET) energy_kernel(
   if (threadIdx.x < kEA && a0 + (int)threadIdx.x < nchr) {
     double t = 0.0;
     for (int q = 0; q < kET / 32; ++q) t += s[threadIdx.x][q];
-    ptl[(size_t)blockIdx.y * nchr + a0 + threadIdx.x] = t;
+    ptl[(size_t)blockIdx.y * nchr + a0 + threadIdx.x] = t * kOneOver4Pi;
   }
 }
 

@@ -152,6 +152,13 @@ struct PinVec {
   PinVec& operator=(const PinVec&) = delete;
 };
 
+// Threads of a far-field block and, in the FP64 one, targets per thread: two
+// from order 6 on, where the contraction's shared loads weigh most (operator
+// apply with one and two: order 3 461 and 461 us, order 6 1,813 and 1,777,
+// order 8 627 and 569), one below, where the second only costs registers.
+constexpr int kFarThreads = 64;
+__host__ __device__ constexpr int far_pair(int order) { return order >= 6 ? 2 : 1; }
+
 // Work item of the interaction kernels: node and a chunk of its entry list.
 struct WorkItem {
   int node;

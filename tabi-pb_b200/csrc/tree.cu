@@ -665,7 +665,8 @@ void build_lists(Handle& H, cudaStream_t s) {
       T.d_rad.p, H.prm.theta, nullptr, nullptr, nullptr, T.d_slot_off.p, d_foff.p, d_noff.p,
       far_cnt.p, near_cnt.p, T.d_far_ent.p, T.d_near_ent.p, H.d_err.p); }
   // work items and moment slots
-  const int kFarChunk = 64, kMomChunk = 256;
+  const int kMomChunk = 256;
+  const int far_chunk = kFarThreads * far_pair(H.prm.order);
   // threads per target of the FP64 near field, as few as give every SM 8 blocks
   // of 128 threads: below that the SMs idle (1,272 targets: 49 us with one, 20
   // with 16), above it more threads only stage the same leaf more often.  The
@@ -690,8 +691,8 @@ void build_lists(Handle& H, cudaStream_t s) {
         mch.push_back(make_int4(slot, T.ibeg[c] + st, std::min(kMomChunk, T.num[c] - st),
                                 (int)mch.size()));
       T.mslot_nchunk.push_back((int)mch.size() - T.mslot_chunk0.back());
-      for (int st = 0; st < hf[c]; st += kFarChunk)
-        T.far_work.push_back({c, (int)(foff[c] + st), std::min(kFarChunk, hf[c] - st), slot});
+      for (int st = 0; st < hf[c]; st += far_chunk)
+        T.far_work.push_back({c, (int)(foff[c] + st), std::min(far_chunk, hf[c] - st), slot});
     }
   }
   // near field: largest leaves first, so that the last blocks to run are short
