@@ -1,4 +1,5 @@
-"""Generates taylor_gen.cuh: straight-line far-field evaluation per Taylor order.
+"""Generates taylor_gen.cuh: straight-line far-field evaluation per Taylor order
+(the mixed-precision operator's; the FP64 one is harmonic.cuh).
 
 The reference evaluates a particle-cluster interaction (treecode3d_pb.f:439-486
 COMPP_TREE_PB) by filling the Taylor-coefficient arrays a(i,j,k), b(i,j,k) of
@@ -16,7 +17,9 @@ This script emits, for each order P, a device function that
     the moments pre-weighted by the integer part of der_cof (the 16 index
     sums fold into 8 accumulators, one per distinct target charge),
   * drops every b term for kappa = 0 (there b(0,0,0) = 1 is only ever
-    multiplied by kappa = 0, and all other b vanish).
+    multiplied by kappa = 0, and all other b vanish),
+  * reads the moments in the order it uses them, four per 16-byte shared load;
+    tabi_mpos gives the place of moment (index, term) in that order.
 Output: the two potentials of COMPP_TREE_PB before the 1/(4 pi) factor.
 
 Usage: python gen_taylor.py [max_order]   (writes taylor_gen.cuh beside itself)
@@ -183,6 +186,22 @@ def formulas(i, j, k, kap):
     return (b if kap else None), a
 
 
+def moment_order(p):
+    """(index, term) of the 16 x NT moments in the order the passes use them."""
+    tl = terms(p)
+    tindex = {t: n for n, t in enumerate(tl)}
+    out = []
+    for n in range(p + 3):
+        for k3 in range(n + 1):
+            for k2 in range(n - k3 + 1):
+                k = (n - k3 - k2, k2, k3)
+                for idx, kk in enumerate(KK):
+                    m = tuple(a - b for a, b in zip(k, kk))
+                    if min(m) >= 0 and sum(m) <= p:
+                        out.append((idx, tindex[m]))
+    return out
+
+
 def gen_pass(p, kap, pre):
     """One kappa pass: declarations, recurrence, contraction into acc{pre}_idx."""
     tl = terms(p)
@@ -197,6 +216,7 @@ def gen_pass(p, kap, pre):
     for name in ACC_NAMES:
         out.append(f"    T {pre}{name} = T(0);")
     out.append("    {")
+    pos = 0
     for n in range(top + 1):
         if n > 0 and BARRIER:
             out.append("    asm volatile(\"\" ::: \"memory\");  // keep moment loads in their shell")
@@ -212,7 +232,10 @@ def gen_pass(p, kap, pre):
                     if min(m) < 0 or sum(m) > p:
                         continue
                     acc = pre + ACC_OF[idx]
-                    out.append(f"    {acc} = fma(a_{k1}_{k2}_{k3}, Mw[{idx * nt + tindex[m]}], {acc});")
+                    if pos % 4 == 0:
+                        out.append(f"    const float4 m{pos // 4} = Mw[{pos // 4}];")
+                    out.append(f"    {acc} = fma(a_{k1}_{k2}_{k3}, m{pos // 4}.{'xyzw'[pos % 4]}, {acc});")
+                    pos += 1
     out.append("    }")
     return out
 
@@ -226,7 +249,7 @@ def gen_order(p):
     for kap, pre, fn in ((False, "u", "far_pass0"), (True, "v", "far_pass1")):
         L += ["template <typename T>",
               f"__device__ __noinline__ TabiFar4<T> {fn}_p{p}(T dx, T dy, T dz, T kappa,",
-              "                                             const T* __restrict__ Mw, T n0, T n1, T n2) {",
+              "                                             const float4* __restrict__ Mw, T n0, T n1, T n2) {",
               "  const T ddx = T(2) * dx, ddy = T(2) * dy, ddz = T(2) * dz;",
               "  T dist = dx * dx + dy * dy + dz * dz;",
               "  const T fac = T(1) / dist;",
@@ -242,7 +265,7 @@ def gen_order(p):
               "  return r;",
               "}", ""]
     L += ["template <typename T>",
-          f"__device__ __forceinline__ void far_eval_p{p}(T dx, T dy, T dz, T kappa, const T* __restrict__ Mw,",
+          f"__device__ __forceinline__ void far_eval_p{p}(T dx, T dy, T dz, T kappa, const float4* __restrict__ Mw,",
           "                                               T n0, T n1, T n2, T eps, T inv_eps,",
           "                                               T& out1, T& out2) {",
           f"  const TabiFar4<T> c = far_pass0_p{p}<T>(dx, dy, dz, T(0), Mw, n0, n1, n2);",
@@ -267,6 +290,29 @@ def main():
         L.append(f"__device__ __constant__ const signed char tabi_terms_p{p}[{len(tl)}][3] = {{"
                  + ", ".join("{%d,%d,%d}" % t for t in tl) + "};")
     L.append("")
+    L.append("// place of moment (index, term) = [index * NT + term] in the order the passes read,")
+    L.append("// and its weight")
+    for p in range(1, maxp + 1):
+        nt = len(terms(p))
+        pos = [0] * (16 * nt)
+        for n, (idx, t) in enumerate(moment_order(p)):
+            pos[idx * nt + t] = n
+        L.append(f"__device__ const unsigned short tabi_mpos_p{p}[{16 * nt}] = {{"
+                 + ", ".join(map(str, pos)) + "};")
+        # der_cof without 1/(4 pi) (main.f90:380-399): prod (k + 1)..(k + kk), and
+        # the sign of the dipole sets' target gradient (idx >= 7)
+        wt = []
+        for idx, kk in enumerate(KK):
+            for t in terms(p):
+                w = -1 if idx >= 7 else 1
+                for a, b in zip(t, kk):
+                    for j in range(1, b + 1):
+                        w *= a + j
+                wt.append(w)
+        assert max(map(abs, wt)) < 128
+        L.append(f"__device__ const signed char tabi_mwgt_p{p}[{16 * nt}] = {{"
+                 + ", ".join(map(str, wt)) + "};")
+    L.append("")
     L.append("__host__ __device__ constexpr int tabi_nterms(int p) { return (p + 1) * (p + 2) * (p + 3) / 6; }")
     L.append("")
     L.append("// Per-pass results: P (index 1), G (2-4), n.F (5-7), n.H (8-16).")
@@ -278,13 +324,22 @@ def main():
     for p in range(1, maxp + 1):
         L += gen_order(p)
     L.append("template <int P, typename T>")
-    L.append("__device__ __forceinline__ void far_eval(T dx, T dy, T dz, T kappa, const T* __restrict__ Mw,")
+    L.append("__device__ __forceinline__ void far_eval(T dx, T dy, T dz, T kappa, const float4* __restrict__ Mw,")
     L.append("                                         T n0, T n1, T n2, T eps, T inv_eps, T& o1, T& o2) {")
     for p in range(1, maxp + 1):
         kw = "if" if p == 1 else "else if"
         L.append(f"  {kw} constexpr (P == {p}) far_eval_p{p}<T>(dx, dy, dz, kappa, Mw, n0, n1, n2, eps, inv_eps, o1, o2);")
     L.append("}")
     L.append("")
+    for fn, ty in (("mpos", "unsigned short"), ("mwgt", "signed char")):
+        L.append("template <int P>")
+        L.append(f"__device__ __forceinline__ const {ty}* tabi_{fn}() {{")
+        for p in range(1, maxp + 1):
+            kw = "if" if p == 1 else "else if"
+            L.append(f"  {kw} constexpr (P == {p}) return tabi_{fn}_p{p};")
+        L.append("  else return nullptr;")
+        L.append("}")
+        L.append("")
     L.append("template <int P>")
     L.append("__device__ __forceinline__ const signed char (*tabi_terms())[3] {")
     for p in range(1, maxp + 1):

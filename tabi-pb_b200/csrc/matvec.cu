@@ -36,90 +36,107 @@ namespace tabi {
 namespace {
 
 // ---- moments
+// Cartesian moments of the mixed-precision far field, summed in FP64.  A group
+// of G threads takes a chunk of up to 256 sources of a cluster, a thread one
+// term of the 4 raw sets: the powers of 64 sources at a time and the 4 charges
+// lie in shared memory, and 7 shared words serve 4 sums (a thread per (set,
+// term) read 4 words for each of its own).  Every sum runs over its chunk's
+// sources in order.
 template <int P>
-__global__ void mom_partial_kernel(const int4* __restrict__ chunks,
-                                   const int* __restrict__ mslot_node,
-                                   const double* __restrict__ nd_mid,
-                                   const double* __restrict__ px, const double* __restrict__ py,
-                                   const double* __restrict__ pz, const double* __restrict__ nx,
-                                   const double* __restrict__ ny, const double* __restrict__ nz,
-                                   const double* __restrict__ area,
-                                   const double* __restrict__ x, int n,
-                                   double* __restrict__ mraw) {
-  constexpr int NT = tabi_nterms(P);
-  constexpr int TILE = 128;
-  constexpr int W = 3 * (P + 1) + 4;
-  __shared__ double st[TILE][W];
-  int4 ch = chunks[blockIdx.x];
-  int node = mslot_node[ch.x];
-  double mx = nd_mid[3 * node], my = nd_mid[3 * node + 1], mz = nd_mid[3 * node + 2];
-  int t = threadIdx.x;
-  int set = t / NT, term = t - set * NT;
-  bool own = t < 4 * NT;
-  int k1 = 0, k2 = 0, k3 = 0;
-  if (own) {
-    const signed char(*tt)[3] = tabi_terms<P>();
-    k1 = tt[term][0];
-    k2 = tt[term][1];
-    k3 = tt[term][2];
-  }
-  double acc = 0.0;
-  for (int base = 0; base < ch.z; base += TILE) {
-    int cnt = min(TILE, ch.z - base);
-    __syncthreads();
-    for (int q = threadIdx.x; q < cnt; q += blockDim.x) {
-      int i = ch.y + base + q;
-      // COMP_MS :876-889: dx = x - mid, powers by repeated multiplication
-      double dx = px[i] - mx, dy = py[i] - my, dz = pz[i] - mz;
-      double a = 1.0, b = 1.0, c = 1.0;
-#pragma unroll
-      for (int p = 0; p <= P; ++p) {
-        st[q][p] = a;
-        st[q][P + 1 + p] = b;
-        st[q][2 * (P + 1) + p] = c;
-        a *= dx;
-        b *= dy;
-        c *= dz;
-      }
-      double A = area[i], x1 = x[i], x2 = x[n + i];
-      // pb_kernel (main.f90:673-681): A*x2 and (n_d*A)*x1
-      st[q][3 * (P + 1) + 0] = A * x2;
-      st[q][3 * (P + 1) + 1] = (nx[i] * A) * x1;
-      st[q][3 * (P + 1) + 2] = (ny[i] * A) * x1;
-      st[q][3 * (P + 1) + 3] = (nz[i] * A) * x1;
-    }
-    __syncthreads();
-    if (own)
-      for (int q = 0; q < cnt; ++q) {
-        double txyz = st[q][k1] * st[q][P + 1 + k2] * st[q][2 * (P + 1) + k3];
-        acc = fma(st[q][3 * (P + 1) + set], txyz, acc);
-      }
-  }
-  if (own) mraw[((size_t)ch.w * 4 + set) * NT + term] = acc;
-}
+struct MomShape {
+  static constexpr int NT = tabi_nterms(P), W = 3 * (P + 1) + 4, TILE = 64;
+  static constexpr int G = (NT + 31) / 32 * 32, CPB = G >= 128 ? 1 : 128 / G;
+  static constexpr int PITCH = (W + 1) / 2 * 2;  // 16-byte aligned rows
+};
 
 template <int P>
-__global__ void mom_final_kernel(const int2* __restrict__ mslot_chunks,
-                                 const double* __restrict__ mraw, float* __restrict__ mw) {
+__global__ void __launch_bounds__(MomShape<P>::G* MomShape<P>::CPB) mom_partial_kernel(
+    const int4* __restrict__ chunks, int nchunk, const int* __restrict__ mslot_node,
+    const double* __restrict__ nd_mid, const double* __restrict__ px,
+    const double* __restrict__ py, const double* __restrict__ pz, const double* __restrict__ nx,
+    const double* __restrict__ ny, const double* __restrict__ nz,
+    const double* __restrict__ area, const double* __restrict__ x, int n,
+    double* __restrict__ mraw) {
+  using M = MomShape<P>;
+  constexpr int NT = M::NT, TILE = M::TILE, G = M::G;
+  __shared__ __align__(16) double stage[M::CPB][TILE][M::PITCH];
+  const int g = threadIdx.x / G, term = threadIdx.x % G;
+  const int c = blockIdx.x * M::CPB + g;
+  const int4 ch = c < nchunk ? chunks[c] : make_int4(0, 0, 0, 0);
+  const int node = mslot_node[ch.x];
+  const double mx = nd_mid[3 * node], my = nd_mid[3 * node + 1], mz = nd_mid[3 * node + 2];
+  double(*st)[M::PITCH] = stage[g];
+  int k1 = 0, k2 = 0, k3 = 0;
+  if (term < NT) {
+    const signed char(*tt)[3] = tabi_terms<P>();
+    k1 = 4 + tt[term][0];
+    k2 = 4 + P + 1 + tt[term][1];
+    k3 = 4 + 2 * (P + 1) + tt[term][2];
+  }
+  double acc[4] = {};
+  for (int base = 0; base < 256; base += TILE) {
+    const int cnt = min(TILE, ch.z - base);
+    if (__syncthreads_and(cnt <= 0)) break;
+    for (int q = term; q < cnt; q += G) {
+      const int i = ch.y + base + q;
+      // COMP_MS :876-889: dx = x - mid, powers by repeated multiplication
+      const double dx = px[i] - mx, dy = py[i] - my, dz = pz[i] - mz;
+      double a = 1.0, b = 1.0, d = 1.0;
+#pragma unroll
+      for (int p = 0; p <= P; ++p) {
+        st[q][4 + p] = a;
+        st[q][4 + P + 1 + p] = b;
+        st[q][4 + 2 * (P + 1) + p] = d;
+        a *= dx;
+        b *= dy;
+        d *= dz;
+      }
+      const double A = area[i], x1 = x[i], x2 = x[n + i];
+      // pb_kernel (main.f90:673-681): A*x2 and (n_d*A)*x1
+      st[q][0] = A * x2;
+      st[q][1] = (nx[i] * A) * x1;
+      st[q][2] = (ny[i] * A) * x1;
+      st[q][3] = (nz[i] * A) * x1;
+    }
+    __syncthreads();
+    if (term < NT)
+#pragma unroll 4
+      for (int q = 0; q < cnt; ++q) {
+        const double2 s0 = *reinterpret_cast<const double2*>(&st[q][0]);
+        const double2 s1 = *reinterpret_cast<const double2*>(&st[q][2]);
+        const double txyz = st[q][k1] * st[q][k2] * st[q][k3];
+        acc[0] = fma(s0.x, txyz, acc[0]);
+        acc[1] = fma(s0.y, txyz, acc[1]);
+        acc[2] = fma(s1.x, txyz, acc[2]);
+        acc[3] = fma(s1.y, txyz, acc[3]);
+      }
+  }
+  if (c < nchunk && term < NT)
+#pragma unroll
+    for (int set = 0; set < 4; ++set) mraw[((size_t)ch.w * 4 + set) * NT + term] = acc[set];
+}
+
+// the 16 weighted sets (kk and der_cof, main.f90:358-399) in the order the far
+// field reads them, from the chunks' sums in order
+template <int P>
+__global__ void __launch_bounds__(256) mom_final_kernel(const int2* __restrict__ mslot_chunks,
+                                                        const double* __restrict__ mraw,
+                                                        float* __restrict__ mw) {
   constexpr int NT = tabi_nterms(P);
-  int slot = blockIdx.x;
-  int2 cr = mslot_chunks[slot];
-  const signed char(*tt)[3] = tabi_terms<P>();
-  // kk (main.f90:358-376) and the source set / sign of each of the 16 indices
-  const int kk[16][3] = {{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {0, 0, 1}, {1, 0, 0}, {0, 1, 0},
-                         {0, 0, 1}, {2, 0, 0}, {1, 1, 0}, {1, 0, 1}, {1, 1, 0}, {0, 2, 0},
-                         {0, 1, 1}, {1, 0, 1}, {0, 1, 1}, {0, 0, 2}};
+  __shared__ double raw[4 * NT];
+  const int2 cr = mslot_chunks[blockIdx.x];
+  for (int q = threadIdx.x; q < 4 * NT; q += blockDim.x) {
+    double v = 0.0;
+    for (int c = 0; c < cr.y; ++c) v += mraw[(size_t)(cr.x + c) * 4 * NT + q];
+    raw[q] = v;
+  }
+  __syncthreads();
+  const unsigned short* mpos = tabi_mpos<P>();
+  const signed char* mwgt = tabi_mwgt<P>();
   for (int q = threadIdx.x; q < 16 * NT; q += blockDim.x) {
-    int idx = q / NT, term = q - idx * NT;
-    int set = (idx == 0) ? 0 : (idx <= 3) ? idx : (idx <= 6) ? 0 : 1 + (idx - 7) / 3;
-    double sgn = (idx >= 7) ? -1.0 : 1.0;
-    double raw = 0.0;
-    for (int c = 0; c < cr.y; ++c) raw += mraw[((size_t)(cr.x + c) * 4 + set) * NT + term];
-    int kv[3] = {tt[term][0], tt[term][1], tt[term][2]};
-    double w = 1.0;
-    for (int m = 0; m < 3; ++m)
-      for (int j = 1; j <= kk[idx][m]; ++j) w *= (double)(kv[m] + j);
-    mw[(size_t)slot * 16 * NT + q] = (float)(sgn * w * raw);
+    const int idx = q / NT, term = q - idx * NT;
+    const int set = idx == 0 ? 0 : idx <= 3 ? idx : idx <= 6 ? 0 : 1 + (idx - 7) / 3;
+    mw[(size_t)blockIdx.x * 16 * NT + mpos[q]] = (float)((double)mwgt[q] * raw[set * NT + term]);
   }
 }
 
@@ -265,9 +282,15 @@ __global__ void __launch_bounds__(kFarThreads) far_harm_kernel(
 
 // FP32 (mixed precision): the target-to-centre offset is formed in FP64 and
 // rounded once, the Taylor recurrences and the contraction run in FP32, the
-// result is widened to FP64 for the per-target sum.
+// result is widened to FP64 for the per-target sum.  Bound by the latency of
+// its straight-line code at a few warps per SM, so the register cap is where
+// more warps stop paying for the spills: far field at orders 3, 4, 5, 6 and 8
+// 232 -> 212, 575 -> 389, 967 -> 723, 1,239 -> 1,131 and 2,092 -> 1,493 us;
+// order 7 is fastest without one (863, 919 at 168 registers).
+constexpr int far_blocks(int p) { return p == 3 ? 12 : p == 4 || p == 5 ? 8 : p == 6 || p == 8 ? 6 : 1; }
+
 template <int P>
-__global__ void __launch_bounds__(64, P == 3 ? 8 : 1) far_kernel(const WorkItem* __restrict__ work,
+__global__ void __launch_bounds__(64, far_blocks(P)) far_kernel(const WorkItem* __restrict__ work,
                                                  const int2* __restrict__ ent,
                                                  const float* __restrict__ mw,
                                                  const double* __restrict__ nd_mid,
@@ -279,10 +302,10 @@ __global__ void __launch_bounds__(64, P == 3 ? 8 : 1) far_kernel(const WorkItem*
                                                  const double* __restrict__ nz, float kappa,
                                                  float eps, double2* __restrict__ res) {
   constexpr int NT = tabi_nterms(P);
-  __shared__ float smw[16 * NT];
+  __shared__ float4 smw[4 * NT];
   WorkItem wi = work[blockIdx.x];
-  const float* src = mw + (size_t)wi.mslot * 16 * NT;
-  for (int q = threadIdx.x; q < 16 * NT; q += blockDim.x) smw[q] = src[q];
+  const float4* src = reinterpret_cast<const float4*>(mw + (size_t)wi.mslot * 16 * NT);
+  for (int q = threadIdx.x; q < 4 * NT; q += blockDim.x) smw[q] = src[q];
   __syncthreads();
   for (int k = threadIdx.x; k < wi.count; k += blockDim.x) {
   int2 e = ent[wi.start + k];
@@ -531,15 +554,14 @@ __global__ void reduce_kernel(const int64_t* __restrict__ slot_off,
 template <int P>
 void launch_moments(Handle& H, const double* x, bool f32, cudaStream_t s) {
   Tree& T = H.tree;
-  constexpr int NT = tabi_nterms(P);
   if (T.nmslot == 0) return;
   const int nch = T.mslot_chunk0.back() + T.mslot_nchunk.back();
   if (f32) {
-    int threads = ((4 * NT + 31) / 32) * 32;
+    using M = MomShape<P>;
     {
       TABI_K(K_MOMENTS, s);
-      mom_partial_kernel<P><<<nch, threads, 0, s>>>(
-          T.d_mchunks.p, T.d_mslot_node.p, T.d_mid.p, H.d_x.p, H.d_y.p, H.d_z.p, H.d_nx.p,
+      mom_partial_kernel<P><<<ceil_div(nch, M::CPB), M::G * M::CPB, 0, s>>>(
+          T.d_mchunks.p, nch, T.d_mslot_node.p, T.d_mid.p, H.d_x.p, H.d_y.p, H.d_z.p, H.d_nx.p,
           H.d_ny.p, H.d_nz.p, H.d_area.p, x, H.n, H.d_mraw.p);
     }
     TABI_K(K_MOMENTS, s);
