@@ -377,23 +377,19 @@ int tabi_create(tabi_h* h, const tabi_params* p) {
     nh->H.prm = *p;
     nh->H.mv_prec = p->precision;
     TABI_CUDA(cudaGetDevice(&nh->H.device));
-    TABI_CUDA(cudaStreamCreateWithFlags(&nh->H.stream, cudaStreamNonBlocking));
-    TABI_CUDA(cudaStreamCreateWithFlags(&nh->H.side, cudaStreamNonBlocking));
-    TABI_CUDA(cudaEventCreateWithFlags(&nh->H.ev_fork, cudaEventDisableTiming));
-    TABI_CUDA(cudaEventCreateWithFlags(&nh->H.ev_join, cudaEventDisableTiming));
-    int prio_lo = 0, prio_hi = 0;
-    TABI_CUDA(cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi));
-    // the large-block chain first; the trailing updates beside it (the chain
-    // waits for them one outer block later) and the small-block group (a
-    // shorter chain of its own) share the SMs the chain leaves free
-    const int prio_mid = (prio_lo + prio_hi) / 2;
-    TABI_CUDA(cudaStreamCreateWithPriority(&nh->H.lu_hi, cudaStreamNonBlocking, prio_hi));
-    TABI_CUDA(cudaStreamCreateWithPriority(&nh->H.aux, cudaStreamNonBlocking, prio_mid));
-    TABI_CUDA(cudaStreamCreateWithPriority(&nh->H.lu_small, cudaStreamNonBlocking, prio_mid));
-    TABI_CUDA(cudaEventCreateWithFlags(&nh->H.ev_la, cudaEventDisableTiming));
-    TABI_CUDA(cudaEventCreateWithFlags(&nh->H.ev_rest, cudaEventDisableTiming));
-    TABI_CUDA(cudaEventCreateWithFlags(&nh->H.ev_lu_join, cudaEventDisableTiming));
-    TABI_CUDA(cudaMallocHost(&nh->H.h_pinned, sizeof(double) * 256));
+    Handle& H = nh->H;
+    H.res = HandleRes::get(H.device);
+    H.stream = H.res.stream;
+    H.side = H.res.side;
+    H.lu_hi = H.res.lu_hi;
+    H.aux = H.res.aux;
+    H.lu_small = H.res.lu_small;
+    H.ev_fork = H.res.ev_fork;
+    H.ev_join = H.res.ev_join;
+    H.ev_la = H.res.ev_la;
+    H.ev_rest = H.res.ev_rest;
+    H.ev_lu_join = H.res.ev_lu_join;
+    H.h_pinned = H.res.h_pinned;
   });
   if (rc != TABI_OK) {
     if (nh) tabi_destroy(nh);
@@ -406,18 +402,11 @@ int tabi_create(tabi_h* h, const tabi_params* p) {
 int tabi_destroy(tabi_h h) {
   if (!h) return TABI_OK;
   cudaSetDevice(h->H.device);
-  if (h->H.stream) cudaStreamSynchronize(h->H.stream);
-  if (h->H.h_pinned) cudaFreeHost(h->H.h_pinned);
-  if (h->H.side) cudaStreamSynchronize(h->H.side);
-  for (cudaStream_t x : {h->H.aux, h->H.lu_hi, h->H.lu_small})
-    if (x) cudaStreamSynchronize(x);
-  cudaStream_t st[] = {h->H.stream, h->H.side, h->H.aux, h->H.lu_hi, h->H.lu_small};
-  cudaEvent_t ev[] = {h->H.ev_fork, h->H.ev_join, h->H.ev_la, h->H.ev_rest, h->H.ev_lu_join};
+  MemPool::Idle idle;  // all work on the handle's buffers, on any stream, is done
+  HandleRes res = h->H.res;
+  const int device = h->H.device;
   delete h;
-  for (cudaStream_t x : st)
-    if (x) cudaStreamDestroy(x);
-  for (cudaEvent_t x : ev)
-    if (x) cudaEventDestroy(x);
+  res.put(device, idle.ok);
   return TABI_OK;
 }
 
@@ -894,6 +883,7 @@ int tabi_ws_create(tabi_ws* w, int hidden, int layers, unsigned long long seed) 
 
 int tabi_ws_destroy(tabi_ws w) {
   if (!w) return TABI_ERR_ARG;
+  MemPool::Idle idle;
   delete w->net;
   delete w;
   return TABI_OK;
@@ -1047,6 +1037,10 @@ int tabi_batch_run_dev(const tabi_params* p, int nmol, const tabi_mol_dev* mols,
             st[10] = w;
             st[11] = H.prm.maxparnode;
           }
+        }
+        if (own) {
+          MemPool::Idle idle;
+          own.reset();
         }
       } catch (const Error& e) {
         errs[w] = e.what();

@@ -43,13 +43,48 @@ struct Error : std::runtime_error {
     if (!(cond)) throw ::tabi::Error((code), (msg));    \
   } while (0)
 
-// Device buffer owned by the handle (freed on reset / destroy).
+// Cache of device and page-locked memory blocks (pool.cu), shared by all
+// handles and threads.  A block goes back when the GPU is done with it: put
+// waits for the device, as cudaFree does, unless the thread holds an Idle,
+// which has waited once for a whole object's blocks.
+struct MemPool {
+  struct Block {
+    void* p = nullptr;
+    size_t bytes = 0;
+    int device = -1;  // -1: page-locked
+  };
+  static Block get(size_t bytes, bool pinned);
+  static void put(Block b);
+  struct Idle {
+    bool ok;
+    Idle();
+    ~Idle();
+    Idle(const Idle&) = delete;
+    Idle& operator=(const Idle&) = delete;
+  };
+};
+
+// Streams, events and a small page-locked scratch of one handle, kept for the
+// next handle of the device.
+struct HandleRes {
+  cudaStream_t stream = nullptr, side = nullptr, lu_hi = nullptr, aux = nullptr,
+               lu_small = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_la = nullptr, ev_rest = nullptr,
+              ev_lu_join = nullptr;
+  double* h_pinned = nullptr;
+  static HandleRes get(int device);
+  void put(int device, bool idle);  // idle: the device has finished the streams' work
+  void destroy();
+};
+
+// Device buffer owned by the handle (given back on regrowth / destroy).
 template <typename T>
 struct DBuf {
   T* p = nullptr;
   size_t n = 0;
+  MemPool::Block blk;
   // Grows only.  A buffer that has to grow again gets 1.5x the request: every
-  // cudaFree synchronises the whole device, which stalls the other handles'
+  // release waits for the whole device, which stalls the other handles'
   // work (batch workers share the GPU), so regrowth should be rare.
   void alloc(size_t count) {
     if (count <= n && p) return;
@@ -57,29 +92,30 @@ struct DBuf {
     release();
     if (count == 0) return;
     if (regrow) count += count / 2;
-    TABI_CUDA(cudaMalloc(&p, count * sizeof(T)));
-    n = count;
+    blk = MemPool::get(count * sizeof(T), false);
+    p = static_cast<T*>(blk.p);
+    n = blk.bytes / sizeof(T);
   }
   void release() {
-    if (p) cudaFree(p);
+    MemPool::put(blk);
+    blk = MemPool::Block();
     p = nullptr;
     n = 0;
+  }
+  void swap(DBuf& o) {
+    std::swap(p, o.p);
+    std::swap(n, o.n);
+    std::swap(blk, o.blk);
   }
   ~DBuf() { release(); }
   DBuf() = default;
   DBuf(const DBuf&) = delete;
   DBuf& operator=(const DBuf&) = delete;
-  DBuf(DBuf&& o) noexcept : p(o.p), n(o.n) {
-    o.p = nullptr;
-    o.n = 0;
-  }
+  DBuf(DBuf&& o) noexcept { swap(o); }
   DBuf& operator=(DBuf&& o) noexcept {
     if (this != &o) {
       release();
-      p = o.p;
-      n = o.n;
-      o.p = nullptr;
-      o.n = 0;
+      swap(o);
     }
     return *this;
   }
@@ -92,12 +128,12 @@ struct DBuf {
 // GPU ran; from page-locked memory the copy returns at once.  `upload`
 // records an event after the copy and `restart` waits for it, so the contents
 // are never rewritten under a pending copy.  Grows only (by doubling, keeping
-// the contents); freeing page-locked memory synchronises the device, so
-// growth should be rare.
+// the contents).
 template <typename T>
 struct PinVec {
   T* p = nullptr;
   size_t len = 0, cap = 0;
+  MemPool::Block blk;
   cudaEvent_t done = nullptr;
   // starts a new fill (after the last copy out of the buffer has finished)
   void restart() {
@@ -115,12 +151,14 @@ struct PinVec {
   const T* end() const { return p + len; }
   void grow(size_t need) {
     const size_t nc = std::max<size_t>(std::max<size_t>(need, 2 * cap), 256);
-    T* q = nullptr;
-    TABI_CUDA(cudaMallocHost(&q, nc * sizeof(T)));
+    const MemPool::Block nb = MemPool::get(nc * sizeof(T), true);
+    T* q = static_cast<T*>(nb.p);
     if (len) std::memcpy(q, p, len * sizeof(T));
-    if (p) cudaFreeHost(p);
+    if (done) cudaEventSynchronize(done);
+    MemPool::put(blk);
+    blk = nb;
     p = q;
-    cap = nc;
+    cap = nb.bytes / sizeof(T);
   }
   void push(const T& v) {
     if (__builtin_expect(len == cap, 0)) grow(len + 1);
@@ -145,7 +183,7 @@ struct PinVec {
       cudaEventSynchronize(done);
       cudaEventDestroy(done);
     }
-    if (p) cudaFreeHost(p);
+    MemPool::put(blk);
   }
   PinVec() = default;
   PinVec(const PinVec&) = delete;
@@ -332,14 +370,15 @@ struct Handle {
   tabi_params prm{};
   Prof prof;
   std::string err;
+  HandleRes res;  // owns the streams, events and scratch named below
   cudaStream_t stream = nullptr;
   cudaStream_t side = nullptr;           // second stream of the matvec (near field)
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   // Streams of the leaf LU, forked from the caller's stream and joined back:
   // the large-block group's chain at the highest priority; the trailing
-  // updates' columns beyond the next outer block (throughput work beside the
-  // chain) and the small-block group below it, so that the block scheduler
-  // gives freed SMs to the chain first.
+  // updates beside it (the chain waits for them one outer block later) and the
+  // small-block group (a shorter chain of its own) below it, so that the block
+  // scheduler gives freed SMs to the chain first.
   cudaStream_t lu_hi = nullptr, lu_small = nullptr, aux = nullptr;
   // the leaf factorisation's phase timer, from its first launch
   // (build_precond) to the join of its streams (finish_precond)

@@ -415,16 +415,11 @@ void build_tree(Handle& H, cudaStream_t s) {
       TABI_CUDA(cudaMemcpyAsync(nu2.p, numd.p, sizeof(int) * cap, cudaMemcpyDeviceToDevice, s));
       TABI_CUDA(cudaStreamSynchronize(s));
     }
-    std::swap(bb.p, bb2.p);
-    std::swap(bb.n, bb2.n);
-    std::swap(mid.p, mid2.p);
-    std::swap(mid.n, mid2.n);
-    std::swap(rad.p, rad2.p);
-    std::swap(rad.n, rad2.n);
-    std::swap(split.p, sp2.p);
-    std::swap(split.n, sp2.n);
-    std::swap(numd.p, nu2.p);
-    std::swap(numd.n, nu2.n);
+    bb.swap(bb2);
+    mid.swap(mid2);
+    rad.swap(rad2);
+    split.swap(sp2);
+    numd.swap(nu2);
     cap = nc;
   };
   ensure(1);

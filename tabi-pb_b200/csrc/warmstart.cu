@@ -787,7 +787,8 @@ WsNet::WsNet(int hidden, int layers, unsigned long long seed) : H(hidden), L(lay
     fill(y.Wb2, H, H, 0.5 / std::sqrt((double)H));
   }
   TABI_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
-  TABI_CUDA(cudaMallocHost(&h_stats, sizeof(double) * 16));
+  h_blk = MemPool::get(sizeof(double) * 16, true);
+  h_stats = static_cast<double*>(h_blk.p);
   theta.alloc(np);
   wbf.alloc(np);
   grad.alloc(np);
@@ -807,7 +808,7 @@ WsNet::~WsNet() {
     cudaStreamSynchronize(stream);
     cudaStreamDestroy(stream);
   }
-  if (h_stats) cudaFreeHost(h_stats);
+  MemPool::put(h_blk);
 }
 
 std::unique_ptr<WsNet> WsNet::clone() const {

@@ -45,6 +45,7 @@ struct WsNet {
   std::vector<Layer> lay;
   int64_t adam_t = 0;
   cudaStream_t stream = nullptr;
+  MemPool::Block h_blk;
   double* h_stats = nullptr;  // pinned
 
   DBuf<float> theta, grad, m, v;
