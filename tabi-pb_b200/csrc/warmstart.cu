@@ -29,6 +29,7 @@
 #include <cmath>
 #include <cstring>
 #include <random>
+#include <type_traits>
 
 #include "tabi_impl.cuh"
 #include "warmstart.cuh"
@@ -44,7 +45,18 @@ constexpr int kF = kWsF;      // node features
 constexpr int kRedB = 592;    // blocks of the fixed-grid reductions
 constexpr int kWsBlocks = 592;
 
-__device__ __forceinline__ float sigm(float x) { return 1.f / (1.f + __expf(-x)); }
+// 1/y for y >= 1, rounded to nearest: the hardware's approximation (within an
+// ulp) and one multiply-add of its residual, which rounds correctly (Markstein,
+// IBM J. Res. Dev. 34 (1990)) -- the bits of 1.f / y without the division's
+// branch.  y above 3e38 gives 0.
+__device__ __forceinline__ float rcp_rn(float y) {
+  float r;
+  y = fminf(y, 3e38f);
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
+  return fmaf(r, fmaf(-y, r, 1.f), r);
+}
+
+__device__ __forceinline__ float sigm(float x) { return rcp_rn(1.f + __expf(-x)); }
 __device__ __forceinline__ float silu(float x) { return x * sigm(x); }
 __device__ __forceinline__ float dsilu(float x) {
   const float s = sigm(x);
@@ -339,64 +351,97 @@ __global__ void ws_node_kernel(int n, const float4* __restrict__ pos, const floa
 
 // ---------------------------------------------------------------- dense layers
 // C (M x N) = A (M x Kd, FP32, row-major) * B, B in bfloat16: B(k, c) = W[k*ldw + c]
-// (TB = false) or W[c*ldw + k] (TB = true, i.e. A * W^T).  64 x 64 tiles,
-// 16-deep k steps, 4 x 4 outputs per thread.  Epilogues:
+// (TB = false) or W[c*ldw + k] (TB = true, i.e. A * W^T).  Epilogues:
 //   0: C = acc            1: C = acc + bias          2: C += acc
 //   3: P = acc + bias, C = silu(P)
 //   4: P = P_in + acc, C = R + silu(P)  (second half of z = h Wb1 + a Wb2 + bb,
 //      P_in = h Wb1 + bb; R the residual input h)
-constexpr int kGM = 64, kGN = 64, kGK = 16;
+// A block takes 64 rows and 16 T columns -- all of them up to a width of 160 --
+// in 16-deep k steps, 4 x T outputs per thread (one 16-byte and T/2 8-byte shared
+// loads for 4 T multiply-adds), the next step's operands in registers
+// meanwhile; three blocks per SM where the epilogue reads two more matrices,
+// else two with the accumulators' registers unspilled.  Each output is one
+// chain of multiply-adds in order of k, so the tile shape does not change it.
+// Bound by issue and shared loads.  77,594 x 160 x 160, A W: 160 -> 129 us, with
+// epilogue 4 197 -> 195; the 64 x 64 tiles of 4 x 4 outputs wasted a sixth of
+// their columns and waited for every step's loads.
+constexpr int kGM = 64, kGK = 16;
 
-template <bool TB, int EPI>
-__global__ void __launch_bounds__(256) ws_gemm_kernel(int M, int N, int Kd,
+template <int T, bool TB, int EPI>
+__global__ void __launch_bounds__(256, EPI <= 1 ? 2 : 3) ws_gemm_kernel(int M, int N, int Kd,
                                                       const float* __restrict__ A, int lda,
                                                       const __nv_bfloat16* __restrict__ W,
                                                       int ldw, const float* __restrict__ bias,
                                                       float* __restrict__ C, int ldc,
                                                       float* __restrict__ P,
                                                       const float* __restrict__ Rin) {
-  __shared__ float As[kGK][kGM + 4];
-  __shared__ float Bs[kGK][kGN + 4];
+  constexpr int BN = 16 * T;
+  __shared__ __align__(16) float As[kGK][kGM + 4];
+  __shared__ __align__(8) float Bs[kGK][BN + 2];
   const int tid = threadIdx.x;
   const int tr = tid / 16, tc = tid % 16;
-  const int row0 = blockIdx.x * kGM, col0 = blockIdx.y * kGN;
-  float acc[4][4] = {};
-  for (int k0 = 0; k0 < Kd; k0 += kGK) {
+  const int row0 = blockIdx.x * kGM, col0 = blockIdx.y * BN;
+  const int ar = tid / 4, ak = 4 * (tid % 4);  // this thread's 4 elements of an A step
+  float av[4];
+  __nv_bfloat16 bv[T];
+  auto fetch = [&](int k0) {
+    const int gr = row0 + ar;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int e = tid + q * 256;  // 0..1023
-      const int r = e / kGK, k = e % kGK;
-      const int gr = row0 + r, gk = k0 + k;
-      As[k][r] = (gr < M && gk < Kd) ? A[(size_t)gr * lda + gk] : 0.f;
-      const int bk = e / kGN, bc = e % kGN;
-      const int gbk = k0 + bk, gbc = col0 + bc;
-      float w = 0.f;
-      if (gbk < Kd && gbc < N)
-        w = __bfloat162float(TB ? W[(size_t)gbc * ldw + gbk] : W[(size_t)gbk * ldw + gbc]);
-      Bs[bk][bc] = w;
+    for (int q = 0; q < 4; ++q)
+      av[q] = gr < M && k0 + ak + q < Kd ? A[(size_t)gr * lda + k0 + ak + q] : 0.f;
+#pragma unroll
+    for (int q = 0; q < T; ++q) {
+      const int e = tid + q * 256;
+      const int bk = TB ? e % kGK : e / BN, bc = TB ? e / kGK : e % BN;
+      const int gk = k0 + bk, gc = col0 + bc;
+      bv[q] = gk < Kd && gc < N ? (TB ? W[(size_t)gc * ldw + gk] : W[(size_t)gk * ldw + gc])
+                                : __float2bfloat16(0.f);
+    }
+  };
+  float acc[4][T] = {};
+  fetch(0);
+  for (int k0 = 0; k0 < Kd; k0 += kGK) {
+    if (k0 > 0) __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 4; ++q) As[ak + q][ar] = av[q];
+#pragma unroll
+    for (int q = 0; q < T; ++q) {
+      const int e = tid + q * 256;
+      Bs[TB ? e % kGK : e / BN][TB ? e / kGK : e % BN] = __bfloat162float(bv[q]);
     }
     __syncthreads();
+    if (k0 + kGK < Kd) fetch(k0 + kGK);
 #pragma unroll
     for (int k = 0; k < kGK; ++k) {
-      float a[4], b[4];
+      const float4 a = *reinterpret_cast<const float4*>(&As[k][tr * 4]);
+      float b[T];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[k][tr * 4 + i];
+      for (int j = 0; j < T; j += 2) {
+        if (j + 1 < T) {
+          const float2 v = *reinterpret_cast<const float2*>(&Bs[k][2 * tc + 16 * j]);
+          b[j] = v.x;
+          b[j + 1] = v.y;
+        } else {
+          b[j] = Bs[k][tc + 16 * j];
+        }
+      }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[k][tc * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+      for (int j = 0; j < T; ++j) {
+        acc[0][j] = fmaf(a.x, b[j], acc[0][j]);
+        acc[1][j] = fmaf(a.y, b[j], acc[1][j]);
+        acc[2][j] = fmaf(a.z, b[j], acc[2][j]);
+        acc[3][j] = fmaf(a.w, b[j], acc[3][j]);
+      }
     }
-    __syncthreads();
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int r = row0 + tr * 4 + i;
     if (r >= M) continue;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int c = col0 + tc * 4 + j;
+    for (int j = 0; j < T; ++j) {
+      // columns in pairs (the last of an odd T alone), as they were read
+      const int c = col0 + (j + 1 < T || (j & 1) ? 2 * tc + 16 * (j & ~1) + (j & 1) : tc + 16 * j);
       if (c >= N) continue;
       const size_t o = (size_t)r * ldc + c;
       const float v = acc[i][j];
@@ -417,64 +462,101 @@ __global__ void __launch_bounds__(256) ws_gemm_kernel(int M, int N, int Kd,
   }
 }
 
-// Weight gradient partials: part[chunk] (Kd x N) = A[rows of chunk]^T * D[rows of chunk]
-constexpr int kDWChunk = 4096;
-__global__ void __launch_bounds__(256) ws_dw_kernel(int M, int Kd, int N,
+// Weight gradient partials: part[chunk] (Kd x N) = A[rows of chunk]^T * D[rows of
+// chunk].  A block takes 16 T x 16 T outputs, T x T per thread (T 8-byte shared
+// loads for T^2 multiply-adds); the chunks are short enough to give every SM two
+// blocks.  77,594 rows, 160 x 160: 583 us with 64 x 64 tiles over 4,096 rows (171
+// blocks of 4 x 4 outputs per thread) -> 101 us.
+template <int T>
+__global__ void __launch_bounds__(256) ws_dw_kernel(int M, int Kd, int N, int chunk,
                                                     const float* __restrict__ A, int lda,
                                                     const float* __restrict__ D, int ldd,
                                                     float* __restrict__ part) {
-  __shared__ float As[kGK][kGM + 4];
-  __shared__ float Ds[kGK][kGN + 4];
+  constexpr int BT = 16 * T;
+  __shared__ __align__(8) float As[kGK][BT], Ds[kGK][BT];
+  // outputs in pairs (the last of an odd T alone)
+  auto at = [](int t, int q) {
+    return q + 1 < T || (q & 1) ? 2 * t + 16 * (q & ~1) + (q & 1) : t + 16 * q;
+  };
   const int tid = threadIdx.x;
   const int tr = tid / 16, tc = tid % 16;
-  const int k0 = blockIdx.x * kGM, c0 = blockIdx.y * kGN;
-  const int m0 = blockIdx.z * kDWChunk, m1 = min(M, m0 + kDWChunk);
-  float acc[4][4] = {};
+  const int k0 = blockIdx.x * BT, c0 = blockIdx.y * BT;
+  const int m0 = blockIdx.z * chunk, m1 = min(M, m0 + chunk);
+  float av[T], dv[T];
+  auto fetch = [&](int mb) {
+#pragma unroll
+    for (int q = 0; q < T; ++q) {
+      const int e = tid + q * 256, r = e / BT, c = e % BT, gm = mb + r;
+      av[q] = gm < m1 && k0 + c < Kd ? A[(size_t)gm * lda + k0 + c] : 0.f;
+      dv[q] = gm < m1 && c0 + c < N ? D[(size_t)gm * ldd + c0 + c] : 0.f;
+    }
+  };
+  float acc[T][T] = {};
+  fetch(m0);
   for (int mb = m0; mb < m1; mb += kGK) {
+    if (mb > m0) __syncthreads();
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < T; ++q) {
       const int e = tid + q * 256;
-      const int r = e / kGM, c = e % kGM;  // r: row within the 16-row step
-      const int gm = mb + r;
-      As[r][c] = (gm < m1 && k0 + c < Kd) ? A[(size_t)gm * lda + k0 + c] : 0.f;
-      Ds[r][c] = (gm < m1 && c0 + c < N) ? D[(size_t)gm * ldd + c0 + c] : 0.f;
+      As[e / BT][e % BT] = av[q];
+      Ds[e / BT][e % BT] = dv[q];
     }
     __syncthreads();
-#pragma unroll
+    if (mb + kGK < m1) fetch(mb + kGK);
+#pragma unroll 4
     for (int r = 0; r < kGK; ++r) {
-      float a[4], d[4];
+      float a[T], d[T];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[r][tr * 4 + i];
+      for (int i = 0; i < T; i += 2) {
+        if (i + 1 < T) {
+          const float2 v = *reinterpret_cast<const float2*>(&As[r][at(tr, i)]);
+          const float2 w = *reinterpret_cast<const float2*>(&Ds[r][at(tc, i)]);
+          a[i] = v.x;
+          a[i + 1] = v.y;
+          d[i] = w.x;
+          d[i + 1] = w.y;
+        } else {
+          a[i] = As[r][at(tr, i)];
+          d[i] = Ds[r][at(tc, i)];
+        }
+      }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) d[j] = Ds[r][tc * 4 + j];
+      for (int i = 0; i < T; ++i)
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], d[j], acc[i][j]);
+        for (int j = 0; j < T; ++j) acc[i][j] = fmaf(a[i], d[j], acc[i][j]);
     }
-    __syncthreads();
   }
   float* out = part + (size_t)blockIdx.z * Kd * N;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int k = k0 + tr * 4 + i;
+  for (int i = 0; i < T; ++i) {
+    const int k = k0 + at(tr, i);
     if (k >= Kd) continue;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int c = c0 + tc * 4 + j;
+    for (int j = 0; j < T; ++j) {
+      const int c = c0 + at(tc, j);
       if (c < N) out[(size_t)k * N + c] = acc[i][j];
     }
   }
 }
 
-// g[e] = sum over chunks of part[chunk][e], in chunk order
-__global__ void ws_sum_parts_kernel(const float* __restrict__ part, int nchunk, int64_t len,
-                                    float* __restrict__ g) {
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < len;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    float s = 0.f;
-    for (int c = 0; c < nchunk; ++c) s += part[(size_t)c * len + e];
-    g[e] = s;
+// g[e] = sum over chunks of part[chunk][e]: 32 elements per block, 8 threads
+// each over every 8th chunk in order, their sums added in order in FP64
+__global__ void __launch_bounds__(256) ws_sum_parts_kernel(const float* __restrict__ part,
+                                                           int nchunk, int64_t len,
+                                                           float* __restrict__ g) {
+  __shared__ double sm[8][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t e = blockIdx.x * (int64_t)32 + lane;
+  double s = 0.0;
+  if (e < len)
+#pragma unroll 4
+    for (int c = w; c < nchunk; c += 8) s += part[(size_t)c * len + e];
+  sm[w][lane] = s;
+  __syncthreads();
+  if (w == 0 && e < len) {
+#pragma unroll
+    for (int q = 1; q < 8; ++q) s += sm[q][lane];
+    g[e] = (float)s;
   }
 }
 
@@ -499,139 +581,227 @@ __global__ void ws_dsilu_kernel(int64_t len, const float* __restrict__ g,
 }
 
 // ---------------------------------------------------------------- aggregation
-// a_i = 1/K sum_k silu(e_ik Wf + bf) * u_{nbr(i,k)}; one thread per channel,
-// kWsNodes panels per block.
-constexpr int kWsNodes = 8;
+// a_i = 1/K sum_k silu(e_ik Wf + bf) * u_{nbr(i,k)}.  A block of H threads takes
+// kGrp panels at a time, H/4 threads per panel and 4 channels per thread: an
+// edge's 12 padded features are three 16-byte shared loads for 44
+// multiply-adds, and the neighbour's channels one 16-byte load (one channel
+// per thread read 11 words for 11 multiply-adds).  Every panel's sums run in
+// the order of its edges.  Bound by the latency of the gate's exponential and
+// reciprocal.  77,594 panels, H = 160: 400 -> 242 us.
+constexpr int kGrp = 4;
+constexpr int kWsNodes = 16;  // panels per block of the forward and du kernels
 
-__global__ void ws_agg_fwd_kernel(int n, int H, const float4* __restrict__ pos,
+struct EdgeStage {
+  float4 e[kGrp][kK][3];
+  int j[kGrp][kK];
+};
+
+// the weights of 4 channels
+struct Chan4 {
+  float4 w[kE], b;
+  __device__ __forceinline__ void load(const __nv_bfloat16* Wf, const float* bf, int H, int c) {
+#pragma unroll
+    for (int q = 0; q < kE; ++q) {
+      const __nv_bfloat16* p = Wf + (size_t)q * H + c;
+      w[q] = make_float4(__bfloat162float(p[0]), __bfloat162float(p[1]), __bfloat162float(p[2]),
+                         __bfloat162float(p[3]));
+    }
+    b = make_float4(bf[c], bf[c + 1], bf[c + 2], bf[c + 3]);
+  }
+  __device__ __forceinline__ float4 pre(const float (&e)[12]) const {
+    float4 v = b;
+#pragma unroll
+    for (int q = 0; q < kE; ++q) {
+      v.x = fmaf(e[q], w[q].x, v.x);
+      v.y = fmaf(e[q], w[q].y, v.y);
+      v.z = fmaf(e[q], w[q].z, v.z);
+      v.w = fmaf(e[q], w[q].w, v.w);
+    }
+    return v;
+  }
+};
+
+__device__ __forceinline__ void edge_unpack(const float4 (&s)[3], float (&e)[12]) {
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    const float4 v = s[q];
+    e[4 * q] = v.x;
+    e[4 * q + 1] = v.y;
+    e[4 * q + 2] = v.z;
+    e[4 * q + 3] = v.w;
+  }
+}
+
+__device__ __forceinline__ void edge_stage(float4 (&dst)[3], const float4 pi, const float4 ni,
+                                           const float4 pj, const float4 nj, float dbar) {
+  static_assert(kE <= 12, "an edge's features are three float4");
+  float e[12] = {};
+  float f[kE];
+  edge_feat(pi, ni, pj, nj, dbar, f);
+#pragma unroll
+  for (int q = 0; q < kE; ++q) e[q] = f[q];
+#pragma unroll
+  for (int q = 0; q < 3; ++q)
+    dst[q] = make_float4(e[4 * q], e[4 * q + 1], e[4 * q + 2], e[4 * q + 3]);
+}
+
+// the edges of panels i0 .. i0 + kGrp (below iend) into shared memory
+__device__ __forceinline__ void stage_panels(EdgeStage& S, int i0, int iend, const float4* pos,
+                                             const float4* nrm, const float* dbar,
+                                             const int* nbr) {
+  for (int q = threadIdx.x; q < kGrp * kK; q += blockDim.x) {
+    const int g = q / kK, k = q % kK, i = i0 + g;
+    if (i >= iend) continue;
+    const int j = nbr[(size_t)i * kK + k];
+    S.j[g][k] = j;
+    edge_stage(S.e[g][k], pos[i], nrm[i], pos[j], nrm[j], dbar[i]);
+  }
+}
+
+__global__ void __launch_bounds__(256, 3) ws_agg_fwd_kernel(int n, int H, const float4* __restrict__ pos,
                                   const float4* __restrict__ nrm, const float* __restrict__ dbar,
                                   const int* __restrict__ nbr,
                                   const __nv_bfloat16* __restrict__ Wf,
                                   const float* __restrict__ bfv, const float* __restrict__ u,
                                   float* __restrict__ a) {
-  __shared__ float es[kK][kE];
-  __shared__ int js[kK];
-  const int c = threadIdx.x;
-  float w[kE];
-#pragma unroll
-  for (int q = 0; q < kE; ++q) w[q] = __bfloat162float(Wf[(size_t)q * H + c]);
-  const float bc = bfv[c];
-  for (int t = 0; t < kWsNodes; ++t) {
-    const int i = blockIdx.x * kWsNodes + t;
-    if (i >= n) break;
+  __shared__ EdgeStage S;
+  const int g = threadIdx.x / (H / 4), c = 4 * (threadIdx.x % (H / 4));
+  Chan4 ch;
+  ch.load(Wf, bfv, H, c);
+  for (int t = 0; t < kWsNodes; t += kGrp) {
+    const int i0 = blockIdx.x * kWsNodes + t, i = i0 + g;
+    if (i0 >= n) break;
     __syncthreads();
-    if (c < kK) {
-      const int j = nbr[(size_t)i * kK + c];
-      js[c] = j;
-      float e[kE];
-      edge_feat(pos[i], nrm[i], pos[j], nrm[j], dbar[i], e);
-#pragma unroll
-      for (int q = 0; q < kE; ++q) es[c][q] = e[q];
-    }
+    stage_panels(S, i0, n, pos, nrm, dbar, nbr);
     __syncthreads();
-    float acc = 0.f;
+    if (i >= n) continue;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 4
     for (int k = 0; k < kK; ++k) {
-      float pr = bc;
-#pragma unroll
-      for (int q = 0; q < kE; ++q) pr = fmaf(es[k][q], w[q], pr);
-      acc = fmaf(silu(pr), u[(size_t)js[k] * H + c], acc);
+      float e[12];
+      edge_unpack(S.e[g][k], e);
+      const float4 uj = *reinterpret_cast<const float4*>(u + (size_t)S.j[g][k] * H + c);
+      const float4 pr = ch.pre(e);
+      acc.x = fmaf(silu(pr.x), uj.x, acc.x);
+      acc.y = fmaf(silu(pr.y), uj.y, acc.y);
+      acc.z = fmaf(silu(pr.z), uj.z, acc.z);
+      acc.w = fmaf(silu(pr.w), uj.w, acc.w);
     }
-    a[(size_t)i * H + c] = acc * (1.f / kK);
+    const float f = 1.f / kK;
+    *reinterpret_cast<float4*>(a + (size_t)i * H + c) =
+        make_float4(acc.x * f, acc.y * f, acc.z * f, acc.w * f);
   }
 }
 
-// Backward of the aggregation, part 1 (per panel i, contiguous panel ranges
-// per block): dpre_ik = u_j da_i / K * silu'(pre_ik); per-block partial
-// gradients of Wf (kE x H) and bf (H).
-__global__ void ws_agg_bwd_w_kernel(int n, int H, const float4* __restrict__ pos,
-                                    const float4* __restrict__ nrm,
-                                    const float* __restrict__ dbar, const int* __restrict__ nbr,
-                                    const __nv_bfloat16* __restrict__ Wf,
-                                    const float* __restrict__ bfv, const float* __restrict__ u,
-                                    const float* __restrict__ da, float* __restrict__ part) {
-  __shared__ float es[kK][kE];
-  __shared__ int js[kK];
-  const int c = threadIdx.x;
-  float w[kE], gw[kE];
+// Backward of the aggregation, part 1 (contiguous panel ranges per block):
+// dpre_ik = u_j da_i / K * silu'(pre_ik); per-block partial gradients of Wf
+// (kE x H) and bf (H), the block's groups added in order.  77,594 panels, H = 160:
+// 739 -> 450 us.
+__global__ void __launch_bounds__(256) ws_agg_bwd_w_kernel(
+    int n, int H, const float4* __restrict__ pos, const float4* __restrict__ nrm,
+    const float* __restrict__ dbar, const int* __restrict__ nbr,
+    const __nv_bfloat16* __restrict__ Wf, const float* __restrict__ bfv,
+    const float* __restrict__ u, const float* __restrict__ da, float* __restrict__ part) {
+  __shared__ EdgeStage S;
+  __shared__ float red[kGrp][256];
+  const int g = threadIdx.x / (H / 4), c = 4 * (threadIdx.x % (H / 4));
+  Chan4 ch;
+  ch.load(Wf, bfv, H, c);
+  float4 gw[kE + 1];
 #pragma unroll
-  for (int q = 0; q < kE; ++q) {
-    w[q] = __bfloat162float(Wf[(size_t)q * H + c]);
-    gw[q] = 0.f;
-  }
-  float gb = 0.f;
-  const float bc = bfv[c];
+  for (int q = 0; q <= kE; ++q) gw[q] = make_float4(0.f, 0.f, 0.f, 0.f);
   const int per = (n + gridDim.x - 1) / gridDim.x;
-  const int i0 = blockIdx.x * per, i1 = min(n, i0 + per);
-  for (int i = i0; i < i1; ++i) {
+  const int b0 = blockIdx.x * per, b1 = min(n, b0 + per);
+  for (int i0 = b0; i0 < b1; i0 += kGrp) {
+    const int i = i0 + g;
     __syncthreads();
-    if (c < kK) {
-      const int j = nbr[(size_t)i * kK + c];
-      js[c] = j;
-      float e[kE];
-      edge_feat(pos[i], nrm[i], pos[j], nrm[j], dbar[i], e);
-#pragma unroll
-      for (int q = 0; q < kE; ++q) es[c][q] = e[q];
-    }
+    stage_panels(S, i0, b1, pos, nrm, dbar, nbr);
     __syncthreads();
-    const float g = da[(size_t)i * H + c] * (1.f / kK);
+    if (i >= b1) continue;
+    float4 d = *reinterpret_cast<const float4*>(da + (size_t)i * H + c);
+    const float f = 1.f / kK;
+    d = make_float4(d.x * f, d.y * f, d.z * f, d.w * f);
+#pragma unroll 2
     for (int k = 0; k < kK; ++k) {
-      float pr = bc;
+      float e[12];
+      edge_unpack(S.e[g][k], e);
+      const float4 uj = *reinterpret_cast<const float4*>(u + (size_t)S.j[g][k] * H + c);
+      const float4 pr = ch.pre(e);
+      const float4 dp = make_float4(uj.x * d.x * dsilu(pr.x), uj.y * d.y * dsilu(pr.y),
+                                    uj.z * d.z * dsilu(pr.z), uj.w * d.w * dsilu(pr.w));
 #pragma unroll
-      for (int q = 0; q < kE; ++q) pr = fmaf(es[k][q], w[q], pr);
-      const float dp = u[(size_t)js[k] * H + c] * g * dsilu(pr);
-#pragma unroll
-      for (int q = 0; q < kE; ++q) gw[q] = fmaf(es[k][q], dp, gw[q]);
-      gb += dp;
+      for (int q = 0; q < kE; ++q) {
+        gw[q].x = fmaf(e[q], dp.x, gw[q].x);
+        gw[q].y = fmaf(e[q], dp.y, gw[q].y);
+        gw[q].z = fmaf(e[q], dp.z, gw[q].z);
+        gw[q].w = fmaf(e[q], dp.w, gw[q].w);
+      }
+      gw[kE].x += dp.x;
+      gw[kE].y += dp.y;
+      gw[kE].z += dp.z;
+      gw[kE].w += dp.w;
     }
   }
   float* o = part + (size_t)blockIdx.x * (kE + 1) * H;
 #pragma unroll
-  for (int q = 0; q < kE; ++q) o[(size_t)q * H + c] = gw[q];
-  o[(size_t)kE * H + c] = gb;
+  for (int q = 0; q <= kE; ++q) {
+    __syncthreads();
+    *reinterpret_cast<float4*>(&red[g][c]) = gw[q];
+    __syncthreads();
+    float v = red[0][threadIdx.x];
+#pragma unroll
+    for (int k = 1; k < kGrp; ++k) v += red[k][threadIdx.x];
+    o[(size_t)q * H + threadIdx.x] = v;
+  }
 }
 
 // Backward of the aggregation, part 2 (per panel j, over the reversed lists):
-// du_j = sum_{(i,k): nbr(i,k) = j} silu(pre_ik) da_i / K
-__global__ void ws_agg_bwd_u_kernel(int n, int H, const float4* __restrict__ pos,
+// du_j = sum_{(i,k): nbr(i,k) = j} silu(pre_ik) da_i / K, kK edges of each of the
+// block's panels at a time.  77,594 panels, H = 160: 414 -> 322 us.
+__global__ void __launch_bounds__(256, 3) ws_agg_bwd_u_kernel(int n, int H, const float4* __restrict__ pos,
                                     const float4* __restrict__ nrm,
                                     const float* __restrict__ dbar, const int* __restrict__ roff,
                                     const int* __restrict__ rev,
                                     const __nv_bfloat16* __restrict__ Wf,
                                     const float* __restrict__ bfv, const float* __restrict__ da,
                                     float* __restrict__ du) {
-  __shared__ float es[32][kE];
-  __shared__ int is[32];
-  const int c = threadIdx.x;
-  float w[kE];
-#pragma unroll
-  for (int q = 0; q < kE; ++q) w[q] = __bfloat162float(Wf[(size_t)q * H + c]);
-  const float bc = bfv[c];
-  for (int t = 0; t < kWsNodes; ++t) {
-    const int j = blockIdx.x * kWsNodes + t;
-    if (j >= n) break;
-    const int a0 = roff[j], a1 = roff[j + 1];
-    float acc = 0.f;
-    for (int b0 = a0; b0 < a1; b0 += 32) {
-      const int cnt = min(32, a1 - b0);
-      __syncthreads();
-      if (c < cnt) {
-        const int i = rev[b0 + c] / kK;
-        is[c] = i;
-        float e[kE];
-        edge_feat(pos[i], nrm[i], pos[j], nrm[j], dbar[i], e);
-#pragma unroll
-        for (int q = 0; q < kE; ++q) es[c][q] = e[q];
+  __shared__ EdgeStage S;
+  const int g = threadIdx.x / (H / 4), c = 4 * (threadIdx.x % (H / 4));
+  Chan4 ch;
+  ch.load(Wf, bfv, H, c);
+  for (int t = 0; t < kWsNodes; t += kGrp) {
+    const int j0 = blockIdx.x * kWsNodes + t, j = j0 + g;
+    if (j0 >= n) break;
+    const int a0 = j < n ? roff[j] : 0, a1 = j < n ? roff[j + 1] : 0;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int b = 0; __syncthreads_or(a0 + b < a1); b += kK) {
+      for (int q = threadIdx.x; q < kGrp * kK; q += blockDim.x) {
+        const int gg = q / kK, k = q % kK, jj = j0 + gg;
+        if (jj >= n) continue;
+        const int p = roff[jj] + b + k;
+        if (p >= roff[jj + 1]) continue;
+        const int i = rev[p] / kK;
+        S.j[gg][k] = i;
+        edge_stage(S.e[gg][k], pos[i], nrm[i], pos[jj], nrm[jj], dbar[i]);
       }
       __syncthreads();
+      const int cnt = min(kK, a1 - a0 - b);
+#pragma unroll 4
       for (int k = 0; k < cnt; ++k) {
-        float pr = bc;
-#pragma unroll
-        for (int q = 0; q < kE; ++q) pr = fmaf(es[k][q], w[q], pr);
-        acc = fmaf(silu(pr), da[(size_t)is[k] * H + c], acc);
+        float e[12];
+        edge_unpack(S.e[g][k], e);
+        const float4 d = *reinterpret_cast<const float4*>(da + (size_t)S.j[g][k] * H + c);
+        const float4 pr = ch.pre(e);
+        acc.x = fmaf(silu(pr.x), d.x, acc.x);
+        acc.y = fmaf(silu(pr.y), d.y, acc.y);
+        acc.z = fmaf(silu(pr.z), d.z, acc.z);
+        acc.w = fmaf(silu(pr.w), d.w, acc.w);
       }
     }
-    du[(size_t)j * H + c] = acc * (1.f / kK);
+    const float f = 1.f / kK;
+    if (j < n)
+      *reinterpret_cast<float4*>(du + (size_t)j * H + c) =
+          make_float4(acc.x * f, acc.y * f, acc.z * f, acc.w * f);
   }
 }
 
@@ -735,11 +905,33 @@ __global__ void ws_to_bf16_kernel(int64_t np, const float* __restrict__ theta,
     wbf[e] = __float2bfloat16_rn(theta[e]);
 }
 
+void sum_parts(const float* part, int nchunk, int64_t len, float* g, cudaStream_t s) {
+  ws_sum_parts_kernel<<<ceil_div(len, 32), 256, 0, s>>>(part, nchunk, len, g);
+}
+
+// Column blocks of 16 T for a width N that is a multiple of 32: one up to 160,
+// two above; f gets T as a compile-time constant.
+template <typename F>
+void with_tile(int N, F&& f) {
+  switch (N <= 160 ? N / 16 : N / 32) {
+    case 2: f(std::integral_constant<int, 2>()); break;
+    case 4: f(std::integral_constant<int, 4>()); break;
+    case 6: f(std::integral_constant<int, 6>()); break;
+    case 7: f(std::integral_constant<int, 7>()); break;
+    case 8: f(std::integral_constant<int, 8>()); break;
+    default: f(std::integral_constant<int, 10>()); break;
+  }
+}
+
 template <bool TB, int EPI>
 void gemm(int M, int N, int Kd, const float* A, int lda, const __nv_bfloat16* W, int ldw,
           const float* bias, float* C, int ldc, float* P, const float* R, cudaStream_t s) {
-  dim3 grid(ceil_div(M, kGM), ceil_div(N, kGN));
-  ws_gemm_kernel<TB, EPI><<<grid, 256, 0, s>>>(M, N, Kd, A, lda, W, ldw, bias, C, ldc, P, R);
+  with_tile(N, [&](auto t) {
+    constexpr int T = decltype(t)::value;
+    dim3 grid(ceil_div(M, kGM), ceil_div(N, 16 * T));
+    ws_gemm_kernel<T, TB, EPI><<<grid, 256, 0, s>>>(M, N, Kd, A, lda, W, ldw, bias, C, ldc, P,
+                                                    R);
+  });
 }
 
 }  // namespace
@@ -909,18 +1101,26 @@ void WsNet::graph(const WsInput& in, cudaStream_t s) {
 }
 
 void WsNet::dw(int M, int Kd, int N, const float* A, const float* D, float* g, cudaStream_t s) {
-  const int nch = ceil_div(M, kDWChunk);
+  // rows per chunk: two blocks for each of 148 SMs, between 64 and 1,024
+  const int chunk = std::min(1024, std::max(64, ceil_div(ceil_div(M, 296), kGK) * kGK));
+  const int nch = ceil_div(M, chunk);
   part.alloc((size_t)nch * Kd * N);
-  dim3 grid(ceil_div(Kd, kGM), ceil_div(N, kGN), nch);
-  ws_dw_kernel<<<grid, 256, 0, s>>>(M, Kd, N, A, Kd, D, N, part.p);
-  ws_sum_parts_kernel<<<std::min(1024, ceil_div((int64_t)Kd * N, 256)), 256, 0, s>>>(
-      part.p, nch, (int64_t)Kd * N, g);
+  auto launch = [&](auto t) {
+    constexpr int T = decltype(t)::value;
+    dim3 grid(ceil_div(Kd, 16 * T), ceil_div(N, 16 * T), nch);
+    ws_dw_kernel<T><<<grid, 256, 0, s>>>(M, Kd, N, chunk, A, Kd, D, N, part.p);
+  };
+  if (Kd == N)
+    with_tile(N, launch);
+  else
+    launch(std::integral_constant<int, 2>());  // the input and output layers
+  sum_parts(part.p, nch, (int64_t)Kd * N, g, s);
 }
 
 void WsNet::colsum(int M, int N, const float* X, float* g, cudaStream_t s) {
   part2.alloc((size_t)kRedB * N);
   ws_colsum_kernel<<<kRedB, 256, 0, s>>>(M, N, X, part2.p);
-  ws_sum_parts_kernel<<<ceil_div(N, 256), 256, 0, s>>>(part2.p, kRedB, N, g);
+  sum_parts(part2.p, kRedB, N, g, s);
 }
 
 void WsNet::forward(const WsInput& in, double* xout, const double* target, cudaStream_t s) {
@@ -987,8 +1187,7 @@ void WsNet::backward(int n, cudaStream_t s) {
     // aggregation: Wf (kE x H) and bf (H) are adjacent in the flat layout
     ws_agg_bwd_w_kernel<<<kWsBlocks, H, 0, s>>>(n, H, pos.p, nrm.p, dbar.p, nbr.p, W + y.Wf,
                                                 T + y.bf, u, da.p, wpart.p);
-    ws_sum_parts_kernel<<<ceil_div((int64_t)(kE + 1) * H, 256), 256, 0, s>>>(
-        wpart.p, kWsBlocks, (int64_t)(kE + 1) * H, G + y.Wf);
+    sum_parts(wpart.p, kWsBlocks, (int64_t)(kE + 1) * H, G + y.Wf, s);
     ws_agg_bwd_u_kernel<<<ceil_div(n, kWsNodes), H, 0, s>>>(n, H, pos.p, nrm.p, dbar.p, roff.p,
                                                              rev.p, W + y.Wf, T + y.bf, da.p,
                                                              du.p);
