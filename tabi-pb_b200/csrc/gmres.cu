@@ -31,33 +31,70 @@ struct Coefs {
 
 __global__ void __launch_bounds__(kRedThreads) lincomb_kernel(const double* __restrict__ V,
                                                               int64_t ld, int n, int nv,
-                                                              Coefs cf, double* __restrict__ out,
-                                                              double* __restrict__ part) {
-  double acc = 0.0;
+                                                              Coefs cf, double* __restrict__ out) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     double v = 0.0;
     for (int j = 0; j < nv; ++j) v = fma(cf.c[j], V[(int64_t)j * ld + i], v);
     out[i] = v;
+  }
+}
+
+// DRLCAL and ISDGMR in one pass over the Krylov vectors: out = sum_j cf[j] V_j with
+// the coefficients that dorth_kernel left on the device, its squared norm to
+// *norm2 (block partials, added in order by the last block to finish), and
+// the new vector V_{nv} times 1/snormw for the next step (unused if there is
+// none).  Nothing is done when re-orthogonalisation is due (cf[nv + 1] != 0):
+// the host then takes the steps one by one.
+__global__ void __launch_bounds__(kRedThreads) residual_kernel(double* V, int64_t ld, int n,
+                                                               int nv,
+                                                               const double* __restrict__ cf,
+                                                               double* __restrict__ out,
+                                                               double* part, double* norm2,
+                                                               unsigned* done) {
+  if (cf[nv + 1] != 0.0) return;
+  __shared__ double c[64];
+  if ((int)threadIdx.x < nv) c[threadIdx.x] = cf[threadIdx.x];
+  __syncthreads();
+  const double scale = cf[nv];
+  double acc = 0.0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    double v = 0.0, last = 0.0;
+#pragma unroll 4
+    for (int j = 0; j < nv; ++j) {
+      last = V[(int64_t)j * ld + i];
+      v = fma(c[j], last, v);
+    }
+    out[i] = v;
+    V[(int64_t)(nv - 1) * ld + i] = scale * last;
     acc = fma(v, v, acc);
   }
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   __shared__ double s[kRedThreads / 32];
+  __shared__ bool is_last;
   if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = acc;
   __syncthreads();
-  if (threadIdx.x == 0 && part) {
+  if (threadIdx.x == 0) {
     double t = 0.0;
     for (int k = 0; k < kRedThreads / 32; ++k) t += s[k];
     part[blockIdx.x] = t;
+    __threadfence();
+    is_last = atomicAdd(done, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!is_last) return;
+  __threadfence();
+  __shared__ double sp[kRedBlocks];
+  for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x)
+    sp[k] = *(volatile double*)(part + k);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+    for (int k = 0; k < (int)gridDim.x; ++k) t += sp[k];
+    *norm2 = t;
+    *done = 0;
   }
 }
 
-// y += sign * (*coef) * x
-__global__ void axpy_dcoef_kernel(int n, const double* __restrict__ coef, double sign,
-                                  const double* __restrict__ x, double* __restrict__ y) {
-  double a = sign * (*coef);
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    y[i] = fma(a, x[i], y[i]);
-}
 __global__ void axpy_kernel(int n, double a, const double* __restrict__ x,
                             double* __restrict__ y) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
@@ -106,11 +143,62 @@ __device__ __forceinline__ void block_partial(double acc, double* part, double* 
 // thread owns the same elements in every pass, so an axpy and the next dot
 // need no barrier; the partial sums are double-buffered and every block adds
 // them in the same order, so all blocks see the same h_i.
+// At the end one thread forms the coefficients of DRLCAL's residual from the
+// new column (DHEQR's rotations of it, those of the earlier columns given): the
+// residual's launch then needs no host round trip.  cf receives the ll + 1
+// coefficients, 1/snormw, and whether re-orthogonalisation is due
+// (:1397-1414).
+struct Rotations {
+  double q[120];  // cosine and sine of columns 1..ll-1
+  double r0nrm, prod;
+};
+
+__device__ void residual_coefs(const Rotations& R, int i0, int ll, const double* h, double vn2,
+                               double wn2, double* cf) {
+  const double vnrm = sqrt(vn2), snormw = sqrt(wn2);
+  // h(i0..ll) rotated
+  double t1 = 0.0;
+  for (int k = 1; k <= ll; ++k) {
+    const double hk = k >= i0 ? h[k - 1] : 0.0;
+    if (k == 1)
+      t1 = hk;
+    else
+      t1 = R.q[2 * (k - 2) + 1] * t1 + R.q[2 * (k - 2)] * hk;
+  }
+  const double t2 = snormw;
+  double c, sn;
+  if (t2 == 0.0) {
+    c = 1.0;
+    sn = 0.0;
+  } else if (fabs(t2) >= fabs(t1)) {
+    const double t = t1 / t2;
+    sn = -1.0 / sqrt(1.0 + t * t);
+    c = -sn * t;
+  } else {
+    const double t = t2 / t1;
+    c = 1.0 / sqrt(1.0 + t * t);
+    sn = -c * t;
+  }
+  const double scale = R.r0nrm * (R.prod * sn);
+  // cf_j = c_j s_{j+1} .. s_ll (c_0 = 1): suffix products of the sines
+  double suffix = scale;
+  cf[ll] = c / snormw * scale;
+  suffix *= sn;
+  for (int j = ll - 1; j >= 0; --j) {
+    cf[j] = (j == 0 ? 1.0 : R.q[2 * (j - 1)]) * suffix;
+    if (j > 0) suffix *= R.q[2 * (j - 1) + 1];
+  }
+  cf[ll + 1] = 1.0 / snormw;
+  cf[ll + 2] = vnrm + 0.001 * snormw != vnrm ? 0.0 : 1.0;
+}
+
 __global__ void __launch_bounds__(kOrthThreads) dorth_kernel(const double* __restrict__ V,
                                                             int64_t ld, int n, int i0, int ll,
                                                             int maxlp1, double* __restrict__ vn,
                                                             double* __restrict__ part,
-                                                            double* __restrict__ out) {
+                                                            double* __restrict__ out,
+                                                            Rotations rot,
+                                                            double* __restrict__ cf) {
   namespace cg = cooperative_groups;
   cg::grid_group grid = cg::this_grid();
   __shared__ double sm[kOrthThreads / 32];
@@ -118,14 +206,12 @@ __global__ void __launch_bounds__(kOrthThreads) dorth_kernel(const double* __res
   const int stride = gridDim.x * blockDim.x;
   const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
   int buf = 0;
-  double acc = 0.0;
+  double acc = 0.0, vn2 = 0.0;
   for (int k = t0; k < n; k += stride) acc = fma(vn[k], vn[k], acc);
   block_partial(acc, part + buf * np, sm);
   grid.sync();
-  {
-    double s = block_sum_parts(part + buf * np, np, sm);
-    if (blockIdx.x == 0 && threadIdx.x == 0) out[maxlp1] = s;
-  }
+  vn2 = block_sum_parts(part + buf * np, np, sm);
+  if (blockIdx.x == 0 && threadIdx.x == 0) out[maxlp1] = vn2;
   for (int i = i0; i <= ll; ++i) {
     const double* vi = V + (int64_t)(i - 1) * ld;
     buf ^= 1;
@@ -144,7 +230,10 @@ __global__ void __launch_bounds__(kOrthThreads) dorth_kernel(const double* __res
   grid.sync();
   {
     double s = block_sum_parts(part + buf * np, np, sm);
-    if (blockIdx.x == 0 && threadIdx.x == 0) out[maxlp1 + 1] = s;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      out[maxlp1 + 1] = s;
+      residual_coefs(rot, i0, ll, out, vn2, s, cf);
+    }
   }
 }
 
@@ -189,7 +278,7 @@ void op_msolve(Handle& H, const double* r, double* z, cudaStream_t s) {
 
 void gmres_dev(Handle& H, const double* b, double* x, int* iter_out, double* err_out,
                int* ierr_out, double* hist, int* nhist, cudaStream_t s, double tol_in,
-               const double* minv_b, double minv_b_nrm) {
+               const double* minv_b, double minv_b_nrm, bool x_known_zero) {
   const int n = 2 * H.n;
   int maxl = H.prm.maxl;
   if (maxl == 0) maxl = 10;
@@ -207,7 +296,9 @@ void gmres_dev(Handle& H, const double* b, double* x, int* iter_out, double* err
   H.d_dl.alloc(n);
   H.d_gz.alloc(n);
   H.d_r.alloc(n);
-  H.d_coef.alloc(4 * (size_t)maxlp1 + kRedBlocks + 8);
+  // the new column of the Hessenberg matrix with the norms (maxlp1 + 3), the
+  // residual's coefficients (maxlp1 + 3), block partials, a counter
+  H.d_coef.alloc(4 * (size_t)maxlp1 + kRedBlocks + 16);
   H.d_red.alloc(kRedBlocks + 8);
   // cooperative DORTH: every block must be resident
   int orth_blocks = 0;
@@ -227,20 +318,24 @@ void gmres_dev(Handle& H, const double* b, double* x, int* iter_out, double* err
   double* z = H.d_gz.p;
   double* r = H.d_r.p;
   double* d_h = H.d_coef.p;                       // HES column slots
-  double* d_part = H.d_coef.p + 4 * maxlp1;       // partial sums
+  double* d_cf = H.d_coef.p + 2 * maxlp1 + 4;     // the residual's coefficients
+  double* d_part = H.d_coef.p + 4 * maxlp1 + 8;   // partial sums
+  unsigned* d_done = reinterpret_cast<unsigned*>(d_part + kRedBlocks + 1);
+  TABI_CUDA(cudaMemsetAsync(d_done, 0, sizeof(unsigned), s));
   std::vector<double> hes((size_t)maxlp1 * maxl), q(2 * maxl), r0ls(maxlp1 + 1);
   auto HES = [&](int i, int j) -> double& { return hes[(size_t)(j - 1) * ldh + (i - 1)]; };
   auto Vc = [&](int j) { return V + (size_t)(j - 1) * n; };
   const int vb = kVecBlocks, vt = 256;
-  auto lincomb_norm = [&](int nv, const Coefs& cf, double* out, bool want_norm) -> double {
-    int nb = std::min(kRedBlocks, ceil_div(n, kRedThreads));
-    { TABI_K(K_VEC, s); lincomb_kernel<<<nb, kRedThreads, 0, s>>>(V, n, n, nv, cf, out, want_norm ? d_part : nullptr); }
-    if (!want_norm) return 0.0;
-    { TABI_K(K_VEC, s); reduce_final_kernel<<<1, 256, 0, s>>>(d_part, nb, d_part + kRedBlocks); }
-    TABI_CUDA(cudaMemcpyAsync(H.h_pinned, d_part + kRedBlocks, sizeof(double),
-                              cudaMemcpyDeviceToHost, s));
-    TABI_CUDA(cudaStreamSynchronize(s));
-    return std::sqrt(H.h_pinned[0]);
+  const int nb = std::max(1, std::min(kRedBlocks, ceil_div(n, kRedThreads)));
+  auto lincomb = [&](int nv, const Coefs& cf, double* out) {
+    TABI_K(K_VEC, s);
+    lincomb_kernel<<<nb, kRedThreads, 0, s>>>(V, n, n, nv, cf, out);
+  };
+  // the residual and its norm, and the new vector scaled, after dorth_kernel
+  auto residual = [&](int nv) {
+    TABI_K(K_VEC, s);
+    residual_kernel<<<nb, kRedThreads, 0, s>>>(V, n, n, nv, d_cf, dl, d_part, d_h + maxlp1 + 2,
+                                               d_done);
   };
 
   int iter = 0, ierr = 0, nh = 0;
@@ -262,7 +357,7 @@ void gmres_dev(Handle& H, const double* b, double* x, int* iter_out, double* err
   // r0 = b - A x; MATVECmain (main.f90:478-479) returns y = x for sum|x| <
   // 1e-10, so an x of exact zeros gives r0 = b bit for bit and M^-1 r0 is the
   // M^-1 b already in r: DPIGMR's first preconditioner apply is skipped
-  const double ax = asum_dev(H, x, n, s);
+  const double ax = x_known_zero ? 0.0 : asum_dev(H, x, n, s);
   const bool x_zero = ax == 0.0;
   if (!x_zero) {
     if (ax < 1e-10)
@@ -285,7 +380,8 @@ void gmres_dev(Handle& H, const double* b, double* x, int* iter_out, double* err
       op_msolve(H, wk, r, s);
     }
     TABI_CUDA(cudaMemcpyAsync(Vc(1), r, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
-    double r0nrm = nrm2_dev(H, Vc(1), n, s);
+    // from x = 0 the first residual is M^-1 b itself
+    double r0nrm = nrsts == 0 && x_zero ? bnrm : nrm2_dev(H, Vc(1), n, s);
     TABI_REQUIRE(nrsts > 0 || std::isfinite(r0nrm), TABI_ERR_ARG,
                  "the initial residual is not finite (x0 holds NaN or Inf)");
     err = r0nrm / bnrm;  // ISDGMR with LGMR = 0
@@ -310,18 +406,27 @@ void gmres_dev(Handle& H, const double* b, double* x, int* iter_out, double* err
           double* vnp = vn;
           double* pp = d_orth_part;
           double* op = d_h;
+          Rotations rot{};
+          std::copy(q.begin(), q.begin() + 2 * (ll - 1), rot.q);
+          rot.r0nrm = r0nrm;
+          rot.prod = prod;
+          double* cfp = d_cf;
           void* args[] = {(void*)&Vp, (void*)&ldv, (void*)&nn, (void*)&ii0, (void*)&lll,
-                          (void*)&mlp1, (void*)&vnp, (void*)&pp, (void*)&op};
+                          (void*)&mlp1, (void*)&vnp, (void*)&pp, (void*)&op, (void*)&rot,
+                          (void*)&cfp};
           TABI_CUDA(cudaLaunchCooperativeKernel((const void*)dorth_kernel, dim3(orth_blocks),
                                                 dim3(kOrthThreads), args, 0, s));
         }
-        TABI_CUDA(cudaMemcpyAsync(H.h_pinned, d_h, sizeof(double) * (maxlp1 + 2),
+        residual(ll + 1);
+        TABI_CUDA(cudaMemcpyAsync(H.h_pinned, d_h, sizeof(double) * (maxlp1 + 3),
                                   cudaMemcpyDeviceToHost, s));
         TABI_CUDA(cudaStreamSynchronize(s));
         for (int i = i0; i <= ll; ++i) HES(i, ll) = H.h_pinned[i - 1];
         double vnrm = std::sqrt(H.h_pinned[maxlp1]);
         snormw = std::sqrt(H.h_pinned[maxlp1 + 1]);
-        if (!(vnrm + 0.001 * snormw != vnrm)) {
+        double rl2 = H.h_pinned[maxlp1 + 2];
+        const bool reorth = !(vnrm + 0.001 * snormw != vnrm);
+        if (reorth) {
           // conditional re-orthogonalisation (dgmres_dep.f:1397-1414)
           double sumdsq = 0.0;
           for (int i = i0; i <= ll; ++i) {
@@ -356,22 +461,32 @@ void gmres_dev(Handle& H, const double* b, double* x, int* iter_out, double* err
         }
         prod = prod * q[2 * ll - 1];
         rho = std::fabs(prod * r0nrm);
-        // ---- ISDGMR with DRLCAL: dl = r0nrm*prod * (recurrence of V columns)
-        Coefs cf{};
-        cf.c[0] = 1.0;
-        for (int i = 1; i <= ll - 1; ++i) {
-          double sn = q[2 * i - 1], c = q[2 * i - 2];
-          for (int j = 0; j < i; ++j) cf.c[j] *= sn;
-          cf.c[i] += c;
+        // ---- ISDGMR with DRLCAL: dl = r0nrm*prod * (recurrence of V columns),
+        // formed by residual_kernel unless re-orthogonalisation changed the column
+        if (reorth) {
+          double cf[64] = {};
+          cf[0] = 1.0;
+          for (int i = 1; i <= ll - 1; ++i) {
+            double sn = q[2 * i - 1], c = q[2 * i - 2];
+            for (int j = 0; j < i; ++j) cf[j] *= sn;
+            cf[i] += c;
+          }
+          {
+            double sn = q[2 * ll - 1], c = q[2 * ll - 2] / snormw;
+            for (int j = 0; j < ll; ++j) cf[j] *= sn;
+            cf[ll] += c;
+          }
+          for (int j = 0; j <= ll; ++j) cf[j] *= r0nrm * prod;
+          cf[ll + 1] = 1.0 / snormw;
+          cf[ll + 2] = 0.0;
+          TABI_CUDA(cudaMemcpyAsync(d_cf, cf, sizeof(double) * (ll + 3), cudaMemcpyHostToDevice, s));
+          residual(ll + 1);
+          TABI_CUDA(cudaMemcpyAsync(H.h_pinned, d_h + maxlp1 + 2, sizeof(double),
+                                    cudaMemcpyDeviceToHost, s));
+          TABI_CUDA(cudaStreamSynchronize(s));
+          rl2 = H.h_pinned[0];
         }
-        {
-          double sn = q[2 * ll - 1], c = q[2 * ll - 2] / snormw;
-          for (int j = 0; j < ll; ++j) cf.c[j] *= sn;
-          cf.c[ll] += c;
-        }
-        for (int j = 0; j <= ll; ++j) cf.c[j] *= r0nrm * prod;
-        double rl = lincomb_norm(ll + 1, cf, dl, true);
-        err = rl / bnrm;
+        err = std::sqrt(rl2) / bnrm;
         if (hist) hist[nh] = err;
         nh++;
         if (err <= tol) {
@@ -379,7 +494,6 @@ void gmres_dev(Handle& H, const double* b, double* x, int* iter_out, double* err
           break;
         }
         if (ll == maxl) break;
-        { TABI_K(K_VEC, s); scal_kernel<<<vb, vt, 0, s>>>(n, 1.0 / snormw, vn); }
       }
       if (!go200 && !go120) {
         if (rho < r0nrm) {
@@ -411,7 +525,7 @@ void gmres_dev(Handle& H, const double* b, double* x, int* iter_out, double* err
         }
         Coefs cf{};
         for (int i = 0; i < l; ++i) cf.c[i] = r0ls[i];
-        lincomb_norm(l, cf, z, false);
+        lincomb(l, cf, z);
         zero_z = false;
       }
     }
@@ -448,13 +562,14 @@ void gmres_dev(Handle& H, const double* b, double* x, int* iter_out, double* err
 // |M^-1 b| (at most (nrmax+1)*maxl of them, the same cap as the FP64 path,
 // which also bounds the inner iterations in total).
 void solve_dev(Handle& H, const double* b, double* x, int* iter_out, double* err_out,
-               int* ierr_out, double* hist, int* nhist, cudaStream_t s) {
+               int* ierr_out, double* hist, int* nhist, cudaStream_t s, bool x_known_zero) {
   TABI_REQUIRE(!H.tree.ranged || H.xchg, TABI_ERR_STATE,
                "a target range is set: the handle computes one shard of the operator, and "
                "the solve across the shards needs an exchange (tabi_set_exchange)");
   if (H.prm.precision != TABI_PREC_MIXED) {
     H.mv_prec = TABI_PREC_FP64;
-    gmres_dev(H, b, x, iter_out, err_out, ierr_out, hist, nhist, s);
+    gmres_dev(H, b, x, iter_out, err_out, ierr_out, hist, nhist, s, -1.0, nullptr, 0.0,
+              x_known_zero);
     return;
   }
   const int n = 2 * H.n;
@@ -483,7 +598,7 @@ void solve_dev(Handle& H, const double* b, double* x, int* iter_out, double* err
     // FP64 residual and its ITOL = 2 measure; from an x of exact zeros the
     // residual is b and M^-1 b is already in t
     H.mv_prec = TABI_PREC_FP64;
-    if (outer == 0 && asum_dev(H, x, n, s) == 0.0) {
+    if (outer == 0 && (x_known_zero || asum_dev(H, x, n, s) == 0.0)) {
       TABI_CUDA(cudaMemcpyAsync(r, b, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
     } else {
       op_matvec(H, x, r, s, true);
@@ -507,7 +622,7 @@ void solve_dev(Handle& H, const double* b, double* x, int* iter_out, double* err
     TABI_CUDA(cudaMemsetAsync(d, 0, sizeof(double) * n, s));
     int it = 0, ie = 0, nhi = 0;
     double ei = 0.0;
-    gmres_dev(H, r, d, &it, &ei, &ie, inner_hist.data(), &nhi, s, tol / err, t, tnrm);
+    gmres_dev(H, r, d, &it, &ei, &ie, inner_hist.data(), &nhi, s, tol / err, t, tnrm, true);
     for (int k = 0; k < nhi && nh < cap; ++k) {
       if (hist) hist[nh] = inner_hist[k] * err;
       ++nh;

@@ -27,8 +27,10 @@ namespace {
 
 constexpr int kAsmCols = 8;
 
+// CHECK false: kappa times the distance is inside the exponential's table.
 // The four kernels of one pair times -A_j (d = r_j - r_i, m = A_j v_j; the near
 // field's forms, see matvec.cu), 1/(4 pi) included in A_j.
+template <bool CHECK>
 __device__ __forceinline__ void asm_pair(double dx, double dy, double dz, double vx, double vy,
                                          double vz, double mx, double my, double mz, double A,
                                          double kappa, double eps, double inv_eps,
@@ -37,7 +39,7 @@ __device__ __forceinline__ void asm_pair(double dx, double dy, double dz, double
   const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
   const double i = fast_rsqrt(r2), i2 = i * i, i3 = i * i2;
   const double kr = kappa * (r2 * i);
-  const double e = exp_neg(kr, tab);
+  const double e = exp_neg<CHECK>(kr, tab);
   const double t = fma(kr, e, e);
   const double md = fma(mx, dx, fma(my, dy, mz * dz));
   const double vd = fma(vx, dx, fma(vy, dy, vz * dz));
@@ -53,6 +55,7 @@ __device__ __forceinline__ void asm_pair(double dx, double dy, double dz, double
 // rows of one column at a time, so that leaves of any size keep the block's
 // warps busy (with a thread per row the mean leaf of 160 left 96 of 256
 // idle).
+template <bool CHECK>
 __global__ void __launch_bounds__(256) assemble_kernel(
     const int2* __restrict__ tiles, const int2* __restrict__ leaf_rng,
     const int64_t* __restrict__ blk_off, const double* __restrict__ px,
@@ -78,7 +81,7 @@ __global__ void __launch_bounds__(256) assemble_kernel(
     if (i != j) {
       const int t = ib + i, s = ib + j;
       const double Aj = area[s] * kOneOver4Pi;
-      asm_pair(px[s] - px[t], py[s] - py[t], pz[s] - pz[t], nx[t], ny[t], nz[t], Aj * nx[s],
+      asm_pair<CHECK>(px[s] - px[t], py[s] - py[t], pz[s] - pz[t], nx[t], ny[t], nz[t], Aj * nx[s],
                Aj * ny[s], Aj * nz[s], Aj, kappa, eps, inv_eps, tab, K1, K2, K3, K4);
     }
     c1[i] = K1;
@@ -1869,6 +1872,19 @@ __global__ void diag_kernel(const double* r, double* z, int n, double s1, double
   else if (i < 2 * n) z[i] = r[i] / s2;
 }
 
+// the leaf blocks' kernel values for the given (leaf, column) tiles
+void launch_assemble(Handle& H, const int2* tiles, int ntiles, cudaStream_t s) {
+  Tree& T = H.tree;
+  double rad = 0.0;
+  for (int c : T.leaves) rad = std::max(rad, T.rad[c]);
+  TABI_K(K_ASSEMBLE, s);
+  // no two faces of a leaf are further apart than its diameter
+  (H.prm.kappa * 2.0 * rad < 0.99 * kExpTabEnd ? assemble_kernel<false> : assemble_kernel<true>)<<<
+      ntiles, 256, 0, s>>>(tiles, T.d_leaf_rng.p, T.d_blk_off.p, H.d_x.p, H.d_y.p, H.d_z.p,
+                           H.d_nx.p, H.d_ny.p, H.d_nz.p, H.d_area.p, H.prm.kappa,
+                           H.prm.eps1 / H.prm.eps0, T.d_lu.p);
+}
+
 }  // namespace
 
 void build_precond(Handle& H, cudaStream_t s) {
@@ -1904,10 +1920,7 @@ void build_precond(Handle& H, cudaStream_t s) {
   H.pc_h_rng.upload(T.d_leaf_rng, s);
   tiles.upload(d_tiles, s);
   double eps = H.prm.eps1 / H.prm.eps0;
-  { TABI_K(K_ASSEMBLE, s); assemble_kernel<<<(int)tiles.len, 256, 0, s>>>(d_tiles.p, T.d_leaf_rng.p, T.d_blk_off.p,
-                                                    H.d_x.p, H.d_y.p, H.d_z.p, H.d_nx.p,
-                                                    H.d_ny.p, H.d_nz.p, H.d_area.p,
-                                                    H.prm.kappa, eps, T.d_lu.p); }
+  launch_assemble(H, d_tiles.p, (int)tiles.len, s);
   TABI_CUDA(cudaMemsetAsync(d_info.p, 0, sizeof(int) * nl, s));
   // apply lists (they depend on the leaf sizes only, so they are built while
   // the assembly runs): blocks of order > 512 get 512 threads (one wave on the GPU),
@@ -2135,11 +2148,7 @@ void finish_precond(Handle& H, cudaStream_t s) {
       H.pc_tiles2.alloc(ptiles.size());
       TABI_CUDA(cudaMemcpyAsync(H.pc_tiles2.p, ptiles.data(), sizeof(int2) * ptiles.size(),
                                 cudaMemcpyHostToDevice, s));
-      TABI_K(K_ASSEMBLE, s);
-      assemble_kernel<<<(int)ptiles.size(), 256, 0, s>>>(H.pc_tiles2.p, T.d_leaf_rng.p,
-                                                         T.d_blk_off.p, H.d_x.p, H.d_y.p,
-                                                         H.d_z.p, H.d_nx.p, H.d_ny.p, H.d_nz.p,
-                                                         H.d_area.p, H.prm.kappa, eps, T.d_lu.p);
+      launch_assemble(H, H.pc_tiles2.p, (int)ptiles.size(), s);
     }
   } else {
     for (int l = 0; l < nl; ++l) pv_leaves.push_back(l);

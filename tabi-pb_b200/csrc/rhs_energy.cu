@@ -152,12 +152,42 @@ constexpr int kET = 256;
 
 // potential_molecule (main.f90:614-657) for kEA atoms per block, bound by the
 // FP64 pipe: 34 instructions per (face, atom) with the kernels formed as sums
-// over the weighted source (as in the near field) and the table exponential
+// over the weighted source (as in the near field) and the table exponential.
+// CHECK false: kappa times any distance is inside the table (root_mid and
+// root_rad, the tree's root, bound them), and the eight pairs of a face are one
+// block of straight-line code that the scheduler can interleave.
+template <bool CHECK>
+__device__ __forceinline__ void energy_sum(
+    const double* __restrict__ px, const double* __restrict__ py, const double* __restrict__ pz,
+    const double* __restrict__ nx, const double* __restrict__ ny, const double* __restrict__ nz,
+    const double* __restrict__ area, const double* __restrict__ x, int n, double kappa, double eps,
+    const double (&ax)[kEA], const double (&ay)[kEA], const double (&az)[kEA],
+    const double* tab, double (&acc)[kEA]) {
+  for (int j = blockIdx.y * blockDim.x + threadIdx.x; j < n; j += gridDim.y * blockDim.x) {
+    const double rx = px[j], ry = py[j], rz = pz[j];
+    const double A = area[j], w1 = A * x[j], w = A * x[n + j];
+    const double mx = w1 * nx[j], my = w1 * ny[j], mz = w1 * nz[j];
+#pragma unroll
+    for (int k = 0; k < kEA; ++k) {
+      const double dx = rx - ax[k], dy = ry - ay[k], dz = rz - az[k];
+      const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+      const double i = fast_rsqrt(r2);
+      const double kr = kappa * (r2 * i);
+      const double e = exp_neg<CHECK>(kr, tab);
+      const double t = fma(kr, e, e);
+      const double md = fma(mx, dx, fma(my, dy, mz * dz));
+      // (G1 - eps G2) w1 + (G0 - Gk) w without 1/(4 pi)
+      acc[k] = fma(i, fma(i * i * md, fma(-eps, t, 1.0), fma(-e, w, w)), acc[k]);
+    }
+  }
+}
+
 __global__ void __launch_bounds__(kET) energy_kernel(
     const double* __restrict__ px, const double* __restrict__ py, const double* __restrict__ pz,
     const double* __restrict__ nx, const double* __restrict__ ny, const double* __restrict__ nz,
     const double* __restrict__ area, const double* __restrict__ x, int n,
     const double* __restrict__ atoms4, int nchr, double kappa, double eps,
+    const double* __restrict__ root_mid, const double* __restrict__ root_rad,
     double* __restrict__ ptl) {
   __shared__ double tab[kExpTab];
   exp_table_fill(tab);
@@ -172,23 +202,17 @@ __global__ void __launch_bounds__(kET) energy_kernel(
     az[k] = atoms4[4 * (size_t)a + 2];
     acc[k] = 0.0;
   }
-  for (int j = blockIdx.y * blockDim.x + threadIdx.x; j < n; j += gridDim.y * blockDim.x) {
-    const double rx = px[j], ry = py[j], rz = pz[j];
-    const double A = area[j], w1 = A * x[j], w = A * x[n + j];
-    const double mx = w1 * nx[j], my = w1 * ny[j], mz = w1 * nz[j];
+  double far_end = 0.0;  // no face is further from any of the block's atoms
+  if (root_mid)
 #pragma unroll
     for (int k = 0; k < kEA; ++k) {
-      const double dx = rx - ax[k], dy = ry - ay[k], dz = rz - az[k];
-      const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
-      const double i = fast_rsqrt(r2);
-      const double kr = kappa * (r2 * i);
-      const double e = exp_neg(kr, tab);
-      const double t = fma(kr, e, e);
-      const double md = fma(mx, dx, fma(my, dy, mz * dz));
-      // (G1 - eps G2) w1 + (G0 - Gk) w without 1/(4 pi)
-      acc[k] = fma(i, fma(i * i * md, fma(-eps, t, 1.0), fma(-e, w, w)), acc[k]);
+      const double dx = ax[k] - root_mid[0], dy = ay[k] - root_mid[1], dz = az[k] - root_mid[2];
+      far_end = fmax(far_end, sqrt(dx * dx + dy * dy + dz * dz) + root_rad[0]);
     }
-  }
+  if (root_mid && kappa * far_end < 0.99 * kExpTabEnd)
+    energy_sum<false>(px, py, pz, nx, ny, nz, area, x, n, kappa, eps, ax, ay, az, tab, acc);
+  else
+    energy_sum<true>(px, py, pz, nx, ny, nz, area, x, n, kappa, eps, ax, ay, az, tab, acc);
   __shared__ double s[kEA][kET / 32];
   int w = threadIdx.x >> 5, l = threadIdx.x & 31;
 #pragma unroll
@@ -215,8 +239,7 @@ __global__ void coulomb_kernel(const double* __restrict__ atoms4, int nchr, doub
   for (int l = k + 1 + threadIdx.x; l < nchr; l += blockDim.x) {
     double dx = xk - atoms4[4 * (size_t)l], dy = yk - atoms4[4 * (size_t)l + 1],
            dz = zk - atoms4[4 * (size_t)l + 2];
-    double dist = sqrt(dx * dx + dy * dy + dz * dz);
-    acc += 1.0 / eps0 / dist * qk * atoms4[4 * (size_t)l + 3];
+    acc = fma(rsqrt(fma(dx, dx, fma(dy, dy, dz * dz))), atoms4[4 * (size_t)l + 3], acc);
   }
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   __shared__ double s[8];
@@ -225,7 +248,7 @@ __global__ void coulomb_kernel(const double* __restrict__ atoms4, int nchr, doub
   if (threadIdx.x == 0) {
     double t = 0.0;
     for (int q = 0; q < (int)(blockDim.x >> 5); ++q) t += s[q];
-    out[k] = t;
+    out[k] = t * qk / eps0;
   }
 }
 
@@ -410,7 +433,8 @@ void energy_dev(Handle& H, int nchr, const double* /*chrpos*/, const double* /*a
   double eps = H.prm.eps1 / H.prm.eps0;
   { TABI_K(K_ENERGY, s); energy_kernel<<<dim3(gx, gy), kET, 0, s>>>(H.d_x.p, H.d_y.p, H.d_z.p, H.d_nx.p, H.d_ny.p,
                                              H.d_nz.p, H.d_area.p, x, n, H.d_atoms.p, nchr,
-                                             H.prm.kappa, eps, H.d_ptl.p); }
+                                             H.prm.kappa, eps, H.has_tree ? H.tree.d_mid.p : nullptr,
+                                             H.has_tree ? H.tree.d_rad.p : nullptr, H.d_ptl.p); }
   double* d_cou = H.d_ptl.p + (size_t)gy * nchr;
   { TABI_K(K_ENERGY, s); coulomb_kernel<<<nchr, 256, 0, s>>>(H.d_atoms.p, nchr, H.prm.eps0, d_cou); }
   std::vector<double> ptl((size_t)gy * nchr), cou(nchr), q(4 * (size_t)nchr);

@@ -213,9 +213,19 @@ void lists_and_precond(Handle& H, cudaStream_t s, const std::function<void(const
   }
 }
 
-void do_build(Handle& H, cudaStream_t s) {
+// orderarr (may be null): the permutation, copied while the factorisation runs
+void do_build(Handle& H, cudaStream_t s, int* orderarr) {
   build_tree(H, s);
-  lists_and_precond(H, s, [](const char*) {});
+  std::vector<int> perm;
+  lists_and_precond(H, s, [&](const char* step) {
+    if (!orderarr || std::strcmp(step, "lists") != 0) return;
+    perm.resize(H.n);
+    TABI_CUDA(cudaMemcpyAsync(perm.data(), H.d_perm.p, sizeof(int) * H.n, cudaMemcpyDeviceToHost,
+                              H.side));
+    TABI_CUDA(cudaStreamSynchronize(H.side));
+  });
+  if (orderarr)
+    for (int i = 0; i < H.n; ++i) orderarr[i] = perm[i] + 1;
 }
 
 template <typename T>
@@ -305,7 +315,7 @@ void run_molecule(Handle& H, WsNet* ws, const MolDev& m, double* x_dev, double* 
   }
   int iter = 0, ierr = 0;
   double err = 0.0, se = 0.0, ce = 0.0;
-  solve_dev(H, b.p, x, &iter, &err, &ierr, nullptr, nullptr, s);
+  solve_dev(H, b.p, x, &iter, &err, &ierr, nullptr, nullptr, s, ws == nullptr);
   mark("gmres");
   energy_dev(H, nchr, nullptr, nullptr, x, &se, &ce, s);
   mark("energy");
@@ -520,9 +530,7 @@ int tabi_build_tree(tabi_h h, int* orderarr, int* nleaf) {
     TABI_REQUIRE(H.has_surface, TABI_ERR_STATE, "no surface loaded");
     TABI_REQUIRE(!H.has_tree, TABI_ERR_STATE, "tree already built for this surface");
     set_device(H);
-    do_build(H, H.stream);
-    if (orderarr)
-      for (int i = 0; i < H.n; ++i) orderarr[i] = H.h_perm[i] + 1;
+    do_build(H, H.stream, orderarr);
     if (nleaf) *nleaf = H.tree.nleaf;
   });
 }

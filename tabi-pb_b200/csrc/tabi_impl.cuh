@@ -394,7 +394,6 @@ struct Handle {
   // order after)
   DBuf<double> d_x, d_y, d_z, d_nx, d_ny, d_nz, d_area;
   DBuf<int> d_perm;  // tree slot -> original index
-  std::vector<int> h_perm;
   Tree tree;
   // matvec scratch
   DBuf<double> d_mraw;    // moment partials
@@ -509,14 +508,16 @@ void msolve_dev(Handle& H, const double* r, double* z, cudaStream_t s);
 void output_potential_dev(Handle& H, int nspt, const double* sptpos, int nface, const int* nvert,
                           const double* x, double* x_orig, double* vert_ptl, cudaStream_t s);
 // gmres (gmres.cu)
-// minv_b (may be null): M^-1 b already formed (device, 2n) and its norm
+// minv_b (may be null): M^-1 b already formed (device, 2n) and its norm;
+// x_known_zero: the caller has just zeroed x
 void gmres_dev(Handle& H, const double* b, double* x, int* iter, double* err, int* ierr,
                double* hist, int* nhist, cudaStream_t s, double tol = -1.0,
-               const double* minv_b = nullptr, double minv_b_nrm = 0.0);
+               const double* minv_b = nullptr, double minv_b_nrm = 0.0,
+               bool x_known_zero = false);
 // the solve the handle's precision asks for: gmres_dev (FP64) or FP64 GMRES-IR
 // around FP32-operator GMRES (mixed)
 void solve_dev(Handle& H, const double* b, double* x, int* iter, double* err, int* ierr,
-               double* hist, int* nhist, cudaStream_t s);
+               double* hist, int* nhist, cudaStream_t s, bool x_known_zero = false);
 double dot_dev(Handle& H, const double* a, const double* b, int n, cudaStream_t s);
 double nrm2_dev(Handle& H, const double* a, int n, cudaStream_t s);
 

@@ -30,7 +30,9 @@ namespace tabi {
 
 namespace {
 
-constexpr int kChunk = 4096;  // faces per tree-build chunk
+// faces per tree-build chunk: short enough that a molecule's few chunks spread
+// over the SMs (93k faces in chunks of 4,096 ran on 23 of them; scatter 26 -> 9 us)
+constexpr int kChunk = 1024;
 constexpr int kBT = 256;      // tree-build block size
 
 __device__ __forceinline__ unsigned long long ord_enc(double v) {
@@ -460,25 +462,28 @@ void build_tree(Handle& H, cudaStream_t s) {
     hsplit.resize(lv1);
     TABI_CUDA(cudaMemcpyAsync(hsplit.data() + lv0, split.p + lv0, sizeof(int) * (lv1 - lv0),
                               cudaMemcpyDeviceToHost, s));
-    TABI_CUDA(cudaStreamSynchronize(s));
+    // the nodes to split are known by their sizes: their faces are coded right
+    // away, and one round trip brings the split dimensions and the counts
     std::vector<int> splitting;
-    for (int c = lv0; c < lv1; ++c) {
+    for (int c = lv0; c < lv1; ++c)
+      if (T.num[c] > L) splitting.push_back(c);
+    make_chunks(splitting);
+    const int nch = (int)chunks.size();
+    std::vector<int> hist(8 * (size_t)nch), base(8 * (size_t)nch);
+    if (nch > 0) {
+      upload_chunks();
+      H.d_hist.alloc(8 * (size_t)nch);
+      H.d_base.alloc(8 * (size_t)nch);
+      { TABI_K(K_TREE, s); code_kernel<<<nch, kBT, 0, s>>>(H.d_chunks.p, H.d_x.p, H.d_y.p, H.d_z.p, mid.p, split.p,
+                                      H.d_code.p, H.d_hist.p); }
+      TABI_CUDA(cudaMemcpyAsync(hist.data(), H.d_hist.p, sizeof(int) * hist.size(),
+                                cudaMemcpyDeviceToHost, s));
+    }
+    TABI_CUDA(cudaStreamSynchronize(s));
+    for (int c = lv0; c < lv1; ++c)
       if (hsplit[c] & 8)
         throw Error(TABI_ERR_ARG, "more than maxparnode coincident face centroids");
-      if (T.num[c] > L) splitting.push_back(c);
-    }
     if (splitting.empty()) break;
-    make_chunks(splitting);
-    upload_chunks();
-    int nch = (int)chunks.size();
-    H.d_hist.alloc(8 * (size_t)nch);
-    H.d_base.alloc(8 * (size_t)nch);
-    { TABI_K(K_TREE, s); code_kernel<<<nch, kBT, 0, s>>>(H.d_chunks.p, H.d_x.p, H.d_y.p, H.d_z.p, mid.p, split.p,
-                                    H.d_code.p, H.d_hist.p); }
-    std::vector<int> hist(8 * (size_t)nch), base(8 * (size_t)nch);
-    TABI_CUDA(cudaMemcpyAsync(hist.data(), H.d_hist.p, sizeof(int) * hist.size(),
-                              cudaMemcpyDeviceToHost, s));
-    TABI_CUDA(cudaStreamSynchronize(s));
     // child ranges: per node, code-major then chunk order
     int nxt0 = (int)T.ibeg.size();
     size_t ci = 0;
@@ -584,13 +589,10 @@ void build_tree(Handle& H, cudaStream_t s) {
   { TABI_K(K_TREE, s); gather4_kernel<<<ceil_div(n, 256), 256, 0, s>>>(H.d_perm.p, n, H.d_nx.p, H.d_ny.p, H.d_nz.p,
                                                   H.d_area.p, H.d_tx.p, H.d_ty.p, H.d_tz.p,
                                                   tarea.p); }
-  TABI_CUDA(cudaMemcpyAsync(H.d_nx.p, H.d_tx.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
-  TABI_CUDA(cudaMemcpyAsync(H.d_ny.p, H.d_ty.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
-  TABI_CUDA(cudaMemcpyAsync(H.d_nz.p, H.d_tz.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
-  TABI_CUDA(cudaMemcpyAsync(H.d_area.p, tarea.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
-  H.h_perm.resize(n);
-  TABI_CUDA(cudaMemcpyAsync(H.h_perm.data(), H.d_perm.p, sizeof(int) * n,
-                            cudaMemcpyDeviceToHost, s));
+  H.d_nx.swap(H.d_tx);
+  H.d_ny.swap(H.d_ty);
+  H.d_nz.swap(H.d_tz);
+  H.d_area.swap(tarea);
   TABI_CUDA(cudaStreamSynchronize(s));
 }
 
