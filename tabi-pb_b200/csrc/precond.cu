@@ -1778,16 +1778,20 @@ __global__ void __launch_bounds__(kNPT, 2) lu_np_border_kernel(
 // C = A[r0:r0+128, c0:c0+64] -= A[r0:, k0:k0+kd] A[k0:k0+kd, c0:] with
 // kd = min(kdepth, m - k0), rows and columns clipped at m.  FP64 tensor cores, a
 // 32 x 32 tile per warp: -C is loaded into the accumulators, the products are added
-// in order of k, and the negative of the sum is stored.  32-deep slices of L
-// (k-major) and U (by column) arrive by cp.async, double-buffered (zero-filled
+// in order of k, and the negative of the sum is stored.  16-deep slices of L
+// (k-major) and U (by column) arrive by cp.async in a ring of four (zero-filled
 // outside the tile: m, r0, c0, k0 and the depth are even, so a 16-byte chunk is
-// wholly inside or outside).  The form with 8 x 4 outputs per thread on DFMA
+// wholly inside or outside), with one barrier per slice: three slices are in
+// flight while one is multiplied.  Two 32-deep slices and two barriers each took
+// 579 us instead of 562 at depth 128 and 400 instead of 372 at depth 64 (31 leaves
+// of order ~1400).  The form with 8 x 4 outputs per thread on DFMA
 // was bound by its 12 shared-load words per 32 multiply-adds: 45-50 % of the
 // FP64 pipe.
-constexpr int kG2M = 128, kG2N = 64, kG2K = 32;
+constexpr int kG2M = 128, kG2N = 64, kG2K = 16;
 constexpr int kG2LP = kG2M + 4;  // L slice: pitch of a depth's 128 rows
-constexpr int kG2UP = kG2K + 4;  // U slice: pitch of a column's 32 depths
-constexpr size_t kGemm2Smem = sizeof(double) * 2 * (kG2K * kG2LP + kG2N * kG2UP);
+constexpr int kG2UP = kG2K + 4;  // U slice: pitch of a column's depths
+constexpr int kG2S = 4;           // slices in the ring
+constexpr size_t kGemm2Smem = sizeof(double) * kG2S * (kG2K * kG2LP + kG2N * kG2UP);
 
 __global__ void __launch_bounds__(256, 2) lu_gemm2_kernel(const int4* __restrict__ items, int k0,
                                                           int kdepth,
@@ -1797,8 +1801,8 @@ __global__ void __launch_bounds__(256, 2) lu_gemm2_kernel(const int4* __restrict
   extern __shared__ __align__(16) double gsm2[];
   chain_wait();  // the previous launch of the chain has finished
   chain_signal();
-  double* sL = gsm2;                      // [2][kG2K][kG2LP]  L slice, k-major
-  double* sU = gsm2 + 2 * kG2K * kG2LP;   // [2][kG2N][kG2UP] U slice, by column
+  double* sL = gsm2;                      // [kG2S][kG2K][kG2LP]  L slices, k-major
+  double* sU = gsm2 + kG2S * kG2K * kG2LP;  // [kG2S][kG2N][kG2UP]  U slices, by column
   const int4 it = items[blockIdx.x];
   const int leaf = it.x, r0 = it.y, c0 = it.z;
   const int m = 2 * leaf_rng[leaf].y;
@@ -1826,8 +1830,11 @@ __global__ void __launch_bounds__(256, 2) lu_gemm2_kernel(const int4* __restrict
     }
     asm volatile("cp.async.commit_group;\n" ::);
   };
-  load_slice(0, 0);
-  if (kG2K < kd) load_slice(kG2K, 1);
+#pragma unroll
+  for (int p = 0; p < kG2S - 1; ++p) {
+    if (p * kG2K < kd) load_slice(p * kG2K, p);
+    else asm volatile("cp.async.commit_group;\n" ::);
+  }
   // this warp's tile, and the lane's row and column in it
   const int wr = 32 * (warp & 3), wc = 32 * (warp >> 2);
   const int rl = r0 + wr + (lane >> 2), cl = c0 + wc + 2 * (lane & 3);
@@ -1844,21 +1851,14 @@ __global__ void __launch_bounds__(256, 2) lu_gemm2_kernel(const int4* __restrict
         acc[i][q][b] = (c < m && r < m) ? -cc[r] : 0.0;
       }
     }
-  for (int kc = 0, buf = 0; kc < kd; kc += kG2K, buf ^= 1) {
-    if (kc + kG2K < kd) {
-      asm volatile("cp.async.wait_group 1;\n" ::);
-    } else {
-      asm volatile("cp.async.wait_group 0;\n" ::);
-    }
+  for (int kc = 0, buf = 0; kc < kd; kc += kG2K, buf = (buf + 1) & (kG2S - 1)) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(kG2S - 2));
     __syncthreads();
-    // all 32 k of the slice: zero-filled past the depth
-    if (r0 + wr < m && c0 + wc < m)  // a warp past the edge leaves the pipe to the others
+    if (kc + (kG2S - 1) * kG2K < kd) load_slice(kc + (kG2S - 1) * kG2K, (buf + kG2S - 1) & (kG2S - 1));
+    else asm volatile("cp.async.commit_group;\n" ::);
+    if (r0 + wr < m && c0 + wc < m)
       dmma_tile<4, 4, kG2LP, kG2UP, kG2K>(acc, sL + buf * kG2K * kG2LP + wr,
                                           sU + buf * kG2N * kG2UP + wc * kG2UP);
-    if (kc + 2 * kG2K < kd) {  // buffer buf takes the slice two on
-      __syncthreads();
-      load_slice(kc + 2 * kG2K, buf);
-    }
   }
 #pragma unroll
   for (int q = 0; q < 4; ++q)
