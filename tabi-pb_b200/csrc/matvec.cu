@@ -287,7 +287,9 @@ __global__ void __launch_bounds__(kFarThreads) far_harm_kernel(
 // more warps stop paying for the spills: far field at orders 3, 4, 5, 6 and 8
 // 232 -> 212, 575 -> 389, 967 -> 723, 1,239 -> 1,131 and 2,092 -> 1,493 us;
 // order 7 is fastest without one (863, 919 at 168 registers).
-constexpr int far_blocks(int p) { return p == 3 ? 12 : p == 4 || p == 5 ? 8 : p == 6 || p == 8 ? 6 : 1; }
+constexpr int far_blocks(int p) {
+  return p == 3 ? 12 : p == 4 || p == 5 ? 8 : p == 6 || p == 8 ? 6 : 1;
+}
 
 template <int P>
 __global__ void __launch_bounds__(64, far_blocks(P)) far_kernel(const WorkItem* __restrict__ work,

@@ -1081,153 +1081,217 @@ __global__ void lu_diaginv_kernel(const int2* __restrict__ blocks,  // (leaf, k0
   for (int i = 0; i < kDB; ++i) Ui[(size_t)lane * kDB + i] = x[i];
 }
 
-// Forward/back substitution with the factored block (DGETRS 'N') in 32-row
-// steps: gather through the pivot permutation, then per step every warp
-// applies the diagonal block's precomputed inverse to the step's 32 running
-// values (a 32 x 32 GEMV, redundant per warp, so no warp waits for another)
-// and updates its rows below (above) with a 32-wide GEMV.  The finalised
-// values go to a second array, so one barrier per step suffices: running
-// values r (xs in the forward sweep, fin in the backward one) and results are
-// never the same words within a step.  No L2 prefetch of the coming steps'
-// panels: with all large blocks prefetching at once, one step ahead measured
-// 203 us per apply of the bench molecule, two 225 us, four 263 us, and none
-// 188 us; the prefetches compete for DRAM and L2 with the loads the steps
-// wait for.  Large blocks run with 512 threads; leaf_list selects the
-// launch's leaves.  Shared memory: 2 m + NT doubles.
-template <int NT>
-__global__ void __launch_bounds__(NT, (NT <= 256 ? 4 : 1)) solve_kernel(
+// Forward/back substitution with the factored block (DGETRS 'N'), one CTA per
+// leaf: gather through the pivot permutation, then L and U in 32-row steps.
+// Step t needs sum_u T(t,u) y_u over the earlier steps' 32 x 32 tiles T and
+// the precomputed inverse of its diagonal block, y_t = Dinv (r_t - sum).
+//
+// The tiles of both sweeps form one sequence, known from the start, in the
+// order they are needed, so eight warps copy them into a ring of RING tiles by
+// cp.async well ahead of their use and the loads wait for nothing but the ring;
+// a thread copies the 16-byte chunks (two rows of two columns) that it
+// multiplies itself, so a tile costs no barrier.  Per step, T(t,t-1) y_{t-1}
+// is the only product that waits for the step before; then, while the ninth
+// warp forms y_t, the others already sum step t+1's tiles with u < t.  Two
+// barriers per step.
+//
+// Bound by the chain of steps (two barriers, the sums across warps and a 32-deep
+// dot product each, 0.6 us) and, for blocks of order ~1,000, by one SM's rate of
+// taking tiles.  The form before this one updated all rows below (above) with
+// each y, so every step's panel loads were issued after its barrier and waited
+// for memory.  Per apply: 2,544 unknowns in blocks of ~320 41 -> 30 us;
+// 121,352 unknowns (590 MB of factors) 171 -> 156 us; 186,260 unknowns (800 MB)
+// 176 -> 168 us with L2 flushed, in blocks of 200 79 -> 53 us, of 60 92 -> 70 us;
+// 807,640 unknowns (1,970 MB) 395 -> 361 us.
+//
+// Blocks of order > 512: two groups of eight warps, each with a ring of nine
+// tiles (one group: 210 us where two take 182), which shared memory holds up to
+// order 6,912.  The others: one group and five tiles, so that three CTAs share
+// an SM (two CTAs with six tiles: 383 instead of 375 us for 807,640 unknowns in
+// blocks of ~300).  Taking two or three tiles per wait keeps fewer in flight: 607
+// and 643 instead of 573 us at order 2,464 (623 before), 170 and 174 instead of
+// 166 us for 800 MB.  Above order ~5,000 the chain's one SM is slower than the
+// form before, whose 512 threads kept 131 KB in flight (order 5,818: 2.97
+// against 2.81 ms, beside a factorisation of 131 GFLOP).
+constexpr int kTile = kDB * kDB, kDRing = 3, kRingBig = 9, kRingSmall = 5;
+constexpr int kRingHuge = 6, kSolveHuge = 6912;  // blocks above this order
+constexpr int kSolveSmall = 512;     // largest order of the lists' small class
+constexpr int kMaxSolveLeaf = 5760;  // faces
+
+// threads and shared memory of solve_kernel<G, RING> for a block of the given order
+constexpr int solve_threads(int G) { return 256 * G + 32; }
+constexpr size_t solve_bytes(int G, int RING, int order) {
+  return sizeof(double) * ((size_t)(order + kDB - 1) / kDB * kDB + (8 * G + 1) * kDB +
+                           kDRing * kTile + G * RING * kTile);
+}
+
+template <int G, int RING>
+__global__ void __launch_bounds__(solve_threads(G), (G == 1 ? 3 : 1)) solve_kernel(
     const int2* __restrict__ leaf_rng, const int64_t* __restrict__ blk_off,
     const int64_t* __restrict__ dinv_off, const int* __restrict__ leaf_list,
     const double* __restrict__ lu, const double* __restrict__ dinv,
     const int* __restrict__ perm, int N, const double* __restrict__ r,
     double* __restrict__ z) {
-  extern __shared__ double sm[];
-  int leaf = leaf_list[blockIdx.x];
-  int2 lr = leaf_rng[leaf];
+  extern __shared__ __align__(16) double sm[];
+  const int leaf = leaf_list[blockIdx.x];
+  const int2 lr = leaf_rng[leaf];
   const int n = lr.y, m = 2 * n, ib = lr.x;
-  double* xs = sm;             // forward sweep: running; backward: results
-  double* fin = sm + m;        // forward sweep: results; backward: running
-  double* ys = sm + 2 * m;     // per warp: the step's 32 diagonal results
-  const double* A = lu + blk_off[leaf];
-  const double* Di = dinv + dinv_off[leaf];
-  const int* pm = perm + 2 * ib;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int i = tid; i < m; i += NT) {
-    int src = pm[i];
-    xs[i] = (src < n) ? r[ib + src] : r[N + ib + src - n];
-  }
-  // the inverse diagonal block of sweep step t (L blocks 0..nblk-1, then U
-  // blocks nblk-1..0), staged into shared memory one step ahead by cp.async
   const int nblk = (m + kDB - 1) / kDB;
-  double* dbuf = ys + 32 * (NT / 32);  // [2][kDB * kDB]
-  auto stage = [&](int t, int buf) {
-    if (t >= 2 * nblk) return;
-    const int b = t < nblk ? t : 2 * nblk - 1 - t;
-    const double* src = Di + (size_t)b * 2 * kDB * kDB + (t < nblk ? 0 : kDB * kDB);
-    for (int e = 2 * tid; e < kDB * kDB; e += 2 * NT) {
-      const unsigned d = (unsigned)__cvta_generic_to_shared(dbuf + buf * kDB * kDB + e);
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src + e));
-    }
-    asm volatile("cp.async.commit_group;\n" ::);
+  double* vec = sm;                       // r, then y, then x (zero past m)
+  double* part = vec + kDB * nblk;        // [8 G][32] the warps' sums
+  double* sv = part + 8 * G * kDB;            // [32] the step's right-hand side
+  double* dbuf = sv + kDB;                // [kDRing] inverse diagonal blocks
+  double* ring = dbuf + kDRing * kTile;   // [G][RING] tiles, by column
+  const double* A = lu + blk_off[leaf];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int* pm = perm + 2 * ib;
+  auto copy16 = [](double* dst, const double* src, bool valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(
+                     (unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(valid ? 16 : 0)
+                 : "memory");
   };
-  // step t: y = Dinv * run[k0 .. k0+nb), res[k0 ..] = y, run[i] -= A[i, k0 ..
-  // k0+nb) y for the rows [i0, i1); the next step's block is copied while the
-  // rows are updated.  Four partial sums per dot product keep the dependent
-  // FMA chains 8 deep.
-  // y = Dinv * run[k0 .. k0+nb) for lane `lane`, four partial sums
-  auto diag = [&](int t, int k0, int nb, const double* run) {
-    const double* Dblk = dbuf + (t & 1) * kDB * kDB;
-    double v0 = 0.0, v1 = 0.0, v2 = 0.0, v3 = 0.0;
-    if (nb == kDB) {  // run + k0 is 16-byte aligned: paired loads
-      const double2* r2 = reinterpret_cast<const double2*>(run + k0);
+  auto commit = [] { asm volatile("cp.async.commit_group;\n" ::: "memory"); };
+  // block of sweep `back`'s step t
+  auto block = [&](int back, int t) { return back ? nblk - 1 - t : t; };
+  if (warp == 8 * G) {
+    // the chain: inverse diagonal blocks kDRing - 1 steps ahead
+    const double* Di = dinv + dinv_off[leaf];
+    auto stage = [&](int q) {  // step q of both sweeps
+      if (q < 2 * nblk) {
+        const int back = q >= nblk, b = block(back, back ? q - nblk : q);
+        const double* src = Di + (size_t)b * 2 * kTile + (back ? kTile : 0);
+        double* dst = dbuf + (q % kDRing) * kTile;
 #pragma unroll
-      for (int q = 0; q < kDB; q += 4) {
-        const double2 ra = r2[q / 2], rb = r2[q / 2 + 1];
-        v0 = fma(Dblk[q * kDB + lane], ra.x, v0);
-        v1 = fma(Dblk[(q + 1) * kDB + lane], ra.y, v1);
-        v2 = fma(Dblk[(q + 2) * kDB + lane], rb.x, v2);
-        v3 = fma(Dblk[(q + 3) * kDB + lane], rb.y, v3);
+        for (int e = 2 * lane; e < kTile; e += 64) copy16(dst + e, src + e, true);
       }
-    } else {
-      for (int q = 0; q < nb; ++q) v0 = fma(Dblk[q * kDB + lane], run[k0 + q], v0);
-    }
-    return (v0 + v1) + (v2 + v3);
-  };
-  // run[i] -= A[i, k0 .. k0+nb) y for row i, tq preloaded when `have`
-  auto row = [&](int k0, int nb, int i, const double* y, double (&tq)[kDB], bool have,
-                 double* run) {
-    const double* a = A + (size_t)k0 * m + i;
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-    if (nb == kDB) {
-      if (!have) {
+      commit();
+    };
+    for (int q = 0; q < kDRing - 1; ++q) stage(q);
+    __syncthreads();  // vec
+    for (int q = 0; q < 2 * nblk; ++q) {
+      const int back = q >= nblk, b = block(back, back ? q - nblk : q);
+      stage(q + kDRing - 1);
+      asm volatile("cp.async.wait_group %0;\n" ::"n"(kDRing - 1) : "memory");
+      __syncthreads();  // the warps' sums
+      double p[4] = {};
 #pragma unroll
-        for (int q = 0; q < kDB; ++q) tq[q] = a[(size_t)q * m];
-      }
-      const double2* y2 = reinterpret_cast<const double2*>(y);
-#pragma unroll
-      for (int q = 0; q < kDB; q += 4) {
-        const double2 ya = y2[q / 2], yb = y2[q / 2 + 1];
-        s0 = fma(tq[q], ya.x, s0);
-        s1 = fma(tq[q + 1], ya.y, s1);
-        s2 = fma(tq[q + 2], yb.x, s2);
-        s3 = fma(tq[q + 3], yb.y, s3);
-      }
-    } else {
-      for (int q = 0; q < nb; ++q) s0 = fma(a[(size_t)q * m], y[q], s0);
-    }
-    run[i] -= (s0 + s1) + (s2 + s3);
-  };
-  auto step = [&](int t, int k0, int nb, double* run, double* res, int i0, int i1) {
-    double tq[kDB];
-    if constexpr (NT >= 512) {
-      // warp 0 forms y and shares it through shared memory (one more barrier,
-      // against 16 warps each reading the 8 KB block); the first row's panel
-      // values are loaded meanwhile
-      const int ifirst = i0 + tid;
-      const bool pre = ifirst < i1 && nb == kDB;
-      if (pre) {
-        const double* a = A + (size_t)k0 * m + ifirst;
-#pragma unroll
-        for (int q = 0; q < kDB; ++q) tq[q] = a[(size_t)q * m];
-      }
-      if (warp == 0) {
-        const double v = diag(t, k0, nb, run);
-        ys[lane] = v;
-        if (lane < nb) res[k0 + lane] = v;
-      }
-      stage(t + 1, (t + 1) & 1);
-      __syncthreads();
-      for (int i = ifirst; i < i1; i += NT) row(k0, nb, i, ys, tq, pre && i == ifirst, run);
-    } else {
-      // every warp forms y itself (no barrier before the rows)
-      double* yw = ys + 32 * warp;
-      const double v = diag(t, k0, nb, run);
-      yw[lane] = v;
-      if (warp == 0 && lane < nb) res[k0 + lane] = v;
+      for (int w = 0; w < 8 * G; ++w) p[w & 3] += part[w * kDB + lane];
+      sv[lane] = vec[kDB * b + lane] - ((p[0] + p[1]) + (p[2] + p[3]));
       __syncwarp();
-      stage(t + 1, (t + 1) & 1);
-      for (int i = i0 + tid; i < i1; i += NT) row(k0, nb, i, yw, tq, false, run);
+      const double* D = dbuf + (q % kDRing) * kTile + lane;
+      const double2* s2 = reinterpret_cast<const double2*>(sv);
+      double v0 = 0.0, v1 = 0.0, v2 = 0.0, v3 = 0.0;
+#pragma unroll
+      for (int k = 0; k < kDB; k += 4) {
+        const double2 a = s2[k / 2], c = s2[k / 2 + 1];
+        v0 = fma(D[k * kDB], a.x, v0);
+        v1 = fma(D[(k + 1) * kDB], a.y, v1);
+        v2 = fma(D[(k + 2) * kDB], c.x, v2);
+        v3 = fma(D[(k + 3) * kDB], c.y, v3);
+      }
+      vec[kDB * b + lane] = (v0 + v1) + (v2 + v3);
+      __syncthreads();  // y_t
     }
-    asm volatile("cp.async.wait_group 0;\n" ::);
-    __syncthreads();
-  };
-  stage(0, 0);
-  asm volatile("cp.async.wait_group 0;\n" ::);
-  __syncthreads();
-  // L y = P r: running values in xs, y in fin
-  for (int k0 = 0, t = 0; k0 < m; k0 += kDB, ++t) {
-    const int nb = min(kDB, m - k0);
-    step(t, k0, nb, xs, fin, k0 + nb, m);
+  } else {
+    // group g takes the tiles of the source steps u = g modulo G; this thread's
+    // rows and columns of a tile:
+    const int g = warp >> 3, rp = 2 * (tid & 15), cp = 2 * ((tid >> 4) & 15);
+    double* const mine = ring + g * RING * kTile + cp * kDB + rp;
+    double* const last = mine + (RING - 1) * kTile;
+    // the tile to copy next: sweep, step, tiles left in the step, offset in A, column
+    int ps = g + 1 < nblk ? 0 : 2, pt = g + 1, left = 1, off = 0, pj = 0;
+    bool rows = false;
+    const unsigned first = (unsigned)__cvta_generic_to_shared(mine);
+    unsigned dst = first;
+    auto strip = [&] {  // first tile of step pt
+      const int i = kDB * block(ps, pt) + rp;
+      pj = kDB * block(ps, g) + cp;
+      rows = i < m;
+      off = pj * m + i;
+      left = (pt - g + G - 1) / G;
+    };
+    if (ps < 2) strip();
+    auto issue = [&] {
+      if (ps < 2) {
+        const bool ok = rows && pj < m;  // m, the row and the column are even
+        const double* src = A + (ok ? off : 0);
+        const int size = ok ? 16 : 0;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n"
+                     "cp.async.cg.shared.global [%0 + %4], [%3], 16, %2;\n" ::"r"(dst),
+                     "l"(src), "r"(size), "l"(src + (ok ? m : 0)), "n"(kDB * sizeof(double))
+                     : "memory");
+        const int d = ps ? -G * kDB : G * kDB;
+        off += d * m;
+        pj += d;
+        if (--left == 0) {
+          if (++pt == nblk) {
+            pt = g + 1;
+            ++ps;
+          }
+          if (ps < 2) strip();
+        }
+      }
+      dst = dst == first + (RING - 1) * kTile * (unsigned)sizeof(double)
+                ? first
+                : dst + kTile * (unsigned)sizeof(double);
+      commit();
+    };
+#pragma unroll 1
+    for (int q = 0; q < RING - 1; ++q) issue();
+    for (int i = tid; i < kDB * nblk; i += 256 * G) {
+      double v = 0.0;
+      if (i < m) {
+        const int k = pm[i];
+        v = (k < n) ? r[ib + k] : r[N + ib + k - n];
+      }
+      vec[i] = v;
+    }
+    double a00 = 0.0, a10 = 0.0, a01 = 0.0, a11 = 0.0;  // rows rp, rp + 1 by columns cp, cp + 1
+    const double* t = mine;
+    auto mul = [&](const double* v) {  // the ring's next tile times y
+      const double2 x = *reinterpret_cast<const double2*>(t);
+      const double2 y = *reinterpret_cast<const double2*>(t + kDB);
+      const double2 w = *reinterpret_cast<const double2*>(v);
+      a00 = fma(x.x, w.x, a00);
+      a10 = fma(x.y, w.x, a10);
+      a01 = fma(y.x, w.y, a01);
+      a11 = fma(y.y, w.y, a11);
+      t = t == last ? mine : t + kTile;
+    };
+    __syncthreads();  // vec
+    for (int back = 0; back < 2; ++back) {
+      const int d = back ? -G * kDB : G * kDB;  // from a source step of the group to its next
+      const double* v0 = vec + kDB * block(back, g) + cp;
+      for (int q = 0; q < nblk; ++q) {
+        const bool prev = q > 0 && (q - 1) % G == g;
+        if (prev) {
+          asm volatile("cp.async.wait_group %0;\n" ::"n"(RING - 2) : "memory");
+          mul(vec + kDB * block(back, q - 1) + cp);
+        }
+        double s0 = a00 + a01, s1 = a10 + a11;
+        s0 += __shfl_xor_sync(0xffffffffu, s0, 16);
+        s1 += __shfl_xor_sync(0xffffffffu, s1, 16);
+        if (lane < 16) *reinterpret_cast<double2*>(part + warp * kDB + rp) = make_double2(s0, s1);
+        a00 = a10 = a01 = a11 = 0.0;
+        __syncthreads();  // the warps' sums
+        if (prev) issue();
+        if (q + 1 < nblk) {
+          const double* v = v0;
+#pragma unroll 1
+          for (int u = g; u < q; u += G, v += d) {
+            asm volatile("cp.async.wait_group %0;\n" ::"n"(RING - 2) : "memory");
+            mul(v);
+            issue();  // into the slot of the tile before this one
+          }
+        }
+        __syncthreads();  // y_t
+      }
+    }
   }
-  // U x = y: running values in fin, x in xs
-  for (int b = nblk - 1, t = nblk; b >= 0; --b, ++t) {
-    const int k0 = b * kDB;
-    const int nb = min(kDB, m - k0);
-    step(t, k0, nb, fin, xs, 0, k0);
-  }
-  for (int i = tid; i < n; i += NT) {
-    z[ib + i] = xs[i];
-    z[N + ib + i] = xs[n + i];
+  for (int i = tid; i < n; i += solve_threads(G)) {
+    z[ib + i] = vec[i];
+    z[N + ib + i] = vec[n + i];
   }
 }
 
@@ -1944,8 +2008,8 @@ void build_precond(Handle& H, cudaStream_t s) {
   launch_assemble(H, d_tiles.p, (int)tiles.len, s);
   TABI_CUDA(cudaMemsetAsync(d_info.p, 0, sizeof(int) * nl, s));
   // apply lists (they depend on the leaf sizes only, so they are built while
-  // the assembly runs): blocks of order > 512 get 512 threads (one wave on the GPU),
-  // the others 256 threads on the side stream; largest first in each
+  // the assembly runs): blocks of order > 512 get two groups of warps, the others
+  // one group, on the side stream (see solve_kernel); largest first in each
   {
     std::vector<int> big, small;
     for (int l = 0; l < nl; ++l) (2 * rng[l].y > 512 ? big : small).push_back(l);
@@ -2425,14 +2489,7 @@ void msolve_dev(Handle& H, const double* r, double* z, cudaStream_t s) {
     return;
   }
   TABI_PHASE(K_PHASE_APPLY, s);
-  // two arrays of the block order m = 2 * leaf size, 32 doubles per warp and
-  // two staged 32 x 32 inverse diagonal blocks
-  size_t smem = sizeof(double) * (4 * (size_t)T.max_leaf + 512 + 2 * kDB * kDB);
-  TABI_REQUIRE(smem <= 200 * 1024, TABI_ERR_LIMIT, "leaf too large for the block solve");
-  if (smem > 48 * 1024) {
-    raise_smem_limit((const void*)solve_kernel<256>, smem);
-    raise_smem_limit((const void*)solve_kernel<512>, smem);
-  }
+  TABI_REQUIRE(T.max_leaf <= kMaxSolveLeaf, TABI_ERR_LIMIT, "leaf too large for the block solve");
   // a shard applies the leaves of its target range only
   const int nbig = T.ranged ? T.r_solve_big : T.n_solve_big;
   const int nsmall = T.ranged ? T.r_solve_small : T.n_solve_small;
@@ -2443,18 +2500,22 @@ void msolve_dev(Handle& H, const double* r, double* z, cudaStream_t s) {
     TABI_CUDA(cudaEventRecord(H.ev_fork, s));
     TABI_CUDA(cudaStreamWaitEvent(s2, H.ev_fork, 0));
   }
-  if (nbig > 0) {
-    TABI_K(K_SOLVE, s);
-    solve_kernel<512><<<nbig, 512, smem, s>>>(T.d_leaf_rng.p, T.d_blk_off.p, T.d_dinv_off.p,
-                                              list, T.d_lu.p, T.d_dinv.p, T.d_lu_perm.p, n, r,
-                                              z);
-  }
-  if (nsmall > 0) {
-    TABI_K(K_SOLVE, s2);
-    solve_kernel<256><<<nsmall, 256, smem, s2>>>(T.d_leaf_rng.p, T.d_blk_off.p, T.d_dinv_off.p,
-                                                 list + nbig, T.d_lu.p, T.d_dinv.p,
-                                                 T.d_lu_perm.p, n, r, z);
-  }
+  auto launch = [&](auto* kernel, int G, size_t smem, int count, const int* leaves,
+                    cudaStream_t st) {
+    if (count == 0) return;
+    raise_smem_limit((const void*)kernel, smem);
+    TABI_K(K_SOLVE, st);
+    kernel<<<count, solve_threads(G), smem, st>>>(T.d_leaf_rng.p, T.d_blk_off.p, T.d_dinv_off.p,
+                                                  leaves, T.d_lu.p, T.d_dinv.p, T.d_lu_perm.p, n,
+                                                  r, z);
+  };
+  const int order = 2 * T.max_leaf;
+  if (order <= kSolveHuge)
+    launch(solve_kernel<2, kRingBig>, 2, solve_bytes(2, kRingBig, order), nbig, list, s);
+  else  // the vector (92 KB for the largest leaf) leaves room for fewer tiles
+    launch(solve_kernel<2, kRingHuge>, 2, solve_bytes(2, kRingHuge, order), nbig, list, s);
+  launch(solve_kernel<1, kRingSmall>, 1,
+         solve_bytes(1, kRingSmall, std::min(order, kSolveSmall)), nsmall, list + nbig, s2);
   if (fork) {
     TABI_CUDA(cudaEventRecord(H.ev_join, s2));
     TABI_CUDA(cudaStreamWaitEvent(s, H.ev_join, 0));

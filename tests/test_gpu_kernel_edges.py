@@ -67,6 +67,38 @@ def test_leaf_block(gpu_lib, faces, kappa):
     assert np.linalg.norm(z - zo) <= 1e-10 * np.linalg.norm(zo)
 
 
+def test_huge_leaf_block(gpu_lib):
+    """One block of order 7,000 (above the apply's 6,912): B z = r, with B as
+    LEAFMATVECpara assembles it."""
+    kappa, eps = 0.1257, EPS1 / EPS0
+    case = born_case(4, radius=6.0)
+    case["nvert"] = np.ascontiguousarray(case["nvert"][:3500])
+    s, g = _handle(case, kappa=kappa, iprcd=1, maxparnode=4000)
+    with s:
+        n, o = s.nface, s.orderarr - 1
+        assert n == 3500 and s.leaves()[1].size == 1
+        r = np.random.default_rng(9).normal(size=2 * n)
+        z = s.msolve(r)
+        xyz, nrm, ar = (np.asarray(v).reshape(len(s.orderarr), -1)[o] for v in g[:3])
+    for i in range(0, n, 500):
+        d = xyz[None] - xyz[i:i + 500, None]
+        rs = np.sqrt((d ** 2).sum(-1))
+        own = rs == 0
+        rs[own] = 1.0
+        g0, e = 1 / (4 * np.pi * rs), np.exp(-kappa * rs)
+        v, v0 = nrm[None], nrm[i:i + 500, None]
+        c, c0, vv = (v * d).sum(-1) / rs, (v0 * d).sum(-1) / rs, (v * v0).sum(-1)
+        t1, t2 = g0 / rs, (1 + kappa * rs) * e
+        g3 = (vv - 3 * c0 * c) / rs * t1
+        k1, k2 = c * t1 * (1 - eps * t2), g0 * (1 - e)
+        k3, k4 = g3 * (t2 - 1) - kappa ** 2 * c0 * c * e * g0, c0 * t1 * (1 - t2 / eps)
+        a = np.where(own, 0.0, ar.ravel()[None])
+        y1 = .5 * (1 + eps) * z[i:i + 500] - (k1 * a) @ z[:n] - (k3 * a) @ z[n:]
+        y2 = .5 * (1 + 1 / eps) * z[n + i:n + i + 500] - (k2 * a) @ z[:n] - (k4 * a) @ z[n:]
+        assert np.abs(y1 - r[i:i + 500]).max() <= 1e-10
+        assert np.abs(y2 - r[n + i:n + i + 500]).max() <= 1e-10
+
+
 @pytest.mark.parametrize("order", range(1, 9))
 def test_mixed_orders(gpu_lib, order):
     import tabipb
