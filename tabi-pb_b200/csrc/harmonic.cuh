@@ -32,8 +32,8 @@
 // contraction and a short recurrence, about 310 FP64 instructions at p = 3 and
 // 870 at p = 6; the Cartesian form took about 1,640 and 5,300 (two passes of a
 // 3-index recurrence and 16 moment sets each).  Bound by the FP64 pipe.  Measured
-// per operator apply: order 3, 3.29 M interactions, 0.375 -> 0.12 ms; order 6,
-// 10.4 M, 4.59 -> 0.86 ms.
+// per operator apply: order 3, 3.29 M interactions, 0.375 -> 0.097 ms; order 6,
+// 10.4 M, 4.59 -> 0.79 ms.
 #pragma once
 
 #include "fast_math.cuh"

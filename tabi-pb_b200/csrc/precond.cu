@@ -1303,17 +1303,17 @@ __global__ void __launch_bounds__(solve_threads(G), (G == 1 ? 3 : 1)) solve_kern
 // blocks of a well-resolved surface are strongly diagonal (the 2n x 2n blocks
 // of the benchmark molecule have condition numbers near 100 and no row
 // interchange at all), so the factorisation runs first without pivot
-// searches, right-looking in outer blocks of 256 columns, three launches each
+// searches, right-looking in outer blocks of 128 columns, three launches each
 // over all leaves of a group:
-//   lu_np_block_kernel   the 256 x 256 diagonal block of every leaf, one CTA
-//                        each, in four 64-column steps, with the inverses of
+//   lu_np_block_kernel   the 128 x 128 diagonal block of every leaf, one CTA
+//                        each, in two 64-column steps, with the inverses of
 //                        the 64 x 64 diagonal blocks' L and U (and their
 //                        32 x 32 diagonal blocks for the applies);
 //   lu_np_border_kernel  the block's L21 = A21 U11^{-1} by 64-row chunks and
 //                        U12 = L11^{-1} A12 by 64-column chunks: each chunk's
-//                        four 64-deep steps depend on no other chunk, so one
+//                        two 64-deep steps depend on no other chunk, so one
 //                        CTA takes them all from shared memory;
-//   lu_gemm2_kernel      A22 -= L21 U12, 256 deep.
+//   lu_gemm2_kernel      A22 -= L21 U12, 128 deep.
 // Every multiplier l is checked: |l| <= 1 - 2^-20 for all of them certifies
 // that partial pivoting (on these values or on the reference's, which differ
 // by rounding only) keeps the diagonal row at every column, so the factors
@@ -1621,7 +1621,7 @@ __device__ bool lu_diag64(double* D, int m, int d, double* li, double* ui, doubl
 }
 
 // Per leaf (leaves[blockIdx.x]) with m > K0: the diagonal block A[K0:K0+D,
-// K0:K0+D], D = min(256, m - K0), factored in place; scr and dinv receive the
+// K0:K0+D], D = min(kOB2, m - K0), factored in place; scr and dinv receive the
 // inverses of its 64 x 64 diagonal blocks (see lu_diag64).  Step j: the
 // diagonal block, L_ij = A_ij U_jj^{-1} (multipliers checked), and per block
 // column k U_jk = L_jj^{-1} A_jk and A_ik -= L_ij U_jk, all as 64 x 64 x 64
@@ -2021,7 +2021,7 @@ void build_precond(Handle& H, cudaStream_t s) {
     H.pc_h_solve_list.assign(big.data(), big.size());
     H.pc_h_solve_list.upload(T.d_solve_list, s);
   }
-  // ---- unpivoted factorisation of every leaf, certified (see lu_np_diag_kernel)
+  // ---- unpivoted factorisation of every leaf, certified (see lu_np_block_kernel)
   H.pc_lu_phase.emplace(H.prof, K_PHASE_LU, s);
   const bool try_np = (H.prm.flags & TABI_FLAG_PIVOTED_LU) == 0;
   if (try_np) {
