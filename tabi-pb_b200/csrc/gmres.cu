@@ -147,14 +147,16 @@ __device__ __forceinline__ void block_partial(double acc, double* part, double* 
 // new column (DHEQR's rotations of it, those of the earlier columns given): the
 // residual's launch then needs no host round trip.  cf receives the ll + 1
 // coefficients, 1/snormw, and whether re-orthogonalisation is due
-// (:1397-1414).
+// (:1397-1414).  The answer is given once, here, with each operation rounded as
+// DORTH's are (a fused multiply-add answers otherwise at the rounding tie); the
+// host reads it back (reorth) instead of asking again.
 struct Rotations {
   double q[120];  // cosine and sine of columns 1..ll-1
   double r0nrm, prod;
 };
 
 __device__ void residual_coefs(const Rotations& R, int i0, int ll, const double* h, double vn2,
-                               double wn2, double* cf) {
+                               double wn2, double* cf, double* reorth) {
   const double vnrm = sqrt(vn2), snormw = sqrt(wn2);
   // h(i0..ll) rotated
   double t1 = 0.0;
@@ -189,7 +191,7 @@ __device__ void residual_coefs(const Rotations& R, int i0, int ll, const double*
     if (j > 0) suffix *= R.q[2 * (j - 1) + 1];
   }
   cf[ll + 1] = 1.0 / snormw;
-  cf[ll + 2] = vnrm + 0.001 * snormw != vnrm ? 0.0 : 1.0;
+  *reorth = cf[ll + 2] = __dadd_rn(vnrm, __dmul_rn(0.001, snormw)) != vnrm ? 0.0 : 1.0;
 }
 
 __global__ void __launch_bounds__(kOrthThreads) dorth_kernel(const double* __restrict__ V,
@@ -232,7 +234,7 @@ __global__ void __launch_bounds__(kOrthThreads) dorth_kernel(const double* __res
     double s = block_sum_parts(part + buf * np, np, sm);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       out[maxlp1 + 1] = s;
-      residual_coefs(rot, i0, ll, out, vn2, s, cf);
+      residual_coefs(rot, i0, ll, out, vn2, s, cf, out + maxlp1 + 3);
     }
   }
 }
@@ -296,8 +298,9 @@ void gmres_dev(Handle& H, const double* b, double* x, int* iter_out, double* err
   H.d_dl.alloc(n);
   H.d_gz.alloc(n);
   H.d_r.alloc(n);
-  // the new column of the Hessenberg matrix with the norms (maxlp1 + 3), the
-  // residual's coefficients (maxlp1 + 3), block partials, a counter
+  // the new column of the Hessenberg matrix with the norms and the answer on
+  // re-orthogonalisation (maxlp1 + 4), the residual's coefficients (maxlp1 + 3),
+  // block partials, a counter
   H.d_coef.alloc(4 * (size_t)maxlp1 + kRedBlocks + 16);
   H.d_red.alloc(kRedBlocks + 8);
   // cooperative DORTH: every block must be resident
@@ -418,14 +421,13 @@ void gmres_dev(Handle& H, const double* b, double* x, int* iter_out, double* err
                                                 dim3(kOrthThreads), args, 0, s));
         }
         residual(ll + 1);
-        TABI_CUDA(cudaMemcpyAsync(H.h_pinned, d_h, sizeof(double) * (maxlp1 + 3),
+        TABI_CUDA(cudaMemcpyAsync(H.h_pinned, d_h, sizeof(double) * (maxlp1 + 4),
                                   cudaMemcpyDeviceToHost, s));
         TABI_CUDA(cudaStreamSynchronize(s));
         for (int i = i0; i <= ll; ++i) HES(i, ll) = H.h_pinned[i - 1];
-        double vnrm = std::sqrt(H.h_pinned[maxlp1]);
         snormw = std::sqrt(H.h_pinned[maxlp1 + 1]);
         double rl2 = H.h_pinned[maxlp1 + 2];
-        const bool reorth = !(vnrm + 0.001 * snormw != vnrm);
+        const bool reorth = H.h_pinned[maxlp1 + 3] != 0.0;
         if (reorth) {
           // conditional re-orthogonalisation (dgmres_dep.f:1397-1414)
           double sumdsq = 0.0;

@@ -1,0 +1,59 @@
+"""Values at the edges of the solver's arithmetic: the rounding tie that decides
+on a second orthogonalisation."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from conftest import BULK, EPS0, EPS1, born_case
+
+pytestmark = pytest.mark.gpu
+
+
+def _kappa():
+    import tabipb
+
+    return tabipb.kappa(BULK, EPS1)
+
+
+def test_second_orthogonalisation_at_the_tie(gpu_lib):
+    """The second step's vector in a Krylov space made by the exchange hook, with
+    0.001 * |w| a double on the rounding tie of |v| + 0.001 |w| == |v|, while the
+    unrounded product lies above it: the test is DORTH's, each operation rounded,
+    and all of the step follows one answer."""
+    import tabipb
+
+    s0 = float.fromhex("0x1.f4p-44")  # 0.001 * s0 rounds to 2^-53
+    assert 0.001 * s0 == 2.0 ** -53 and np.sqrt(s0 * s0) == s0
+    rt = C.CDLL("libcudart.so.12")
+    rt.cudaStreamSynchronize.argtypes = [C.c_void_p]
+    rt.cudaMemcpy.argtypes = [C.c_void_p, C.c_void_p, C.c_size_t, C.c_int]
+    case = born_case(1)
+    calls = []
+    with tabipb.TabiSolver(order=3, maxparnode=40, theta=0.8, eps0=EPS0, eps1=EPS1,
+                           kappa=_kappa(), iprcd=0, tol=0.0, maxl=2, nrmax=-1) as s:
+        s.form_matrix(case["sptpos"], case["sptnrm"], case["nvert"], case["chrpos"],
+                      case["atmchr"])
+        s.build_tree()
+        n = s.nface
+        # M^-1 b, then A V1, M^-1 A V1, A V2, M^-1 A V2
+        heads = [[1.0], [0.0], [1.0, s0], [0.0], [0.3, 0.5, 0.4]]
+
+        def exchange(v, n2, t0, t1, stream):
+            w = np.zeros(n2)
+            w[:len(heads[len(calls)])] = heads[len(calls)]
+            calls.append(n2)
+            assert rt.cudaStreamSynchronize(stream) == 0
+            assert rt.cudaMemcpy(v, w.ctypes.data, w.nbytes, 1) == 0
+
+        s.set_target_range(0, int(s.leaves()[1][0]))
+        s.set_exchange(exchange)
+        res = s.dgmres(np.ones(2 * n))
+        s.set_exchange(None)
+    assert len(calls) == len(heads) and s.exchange_error is None
+    # |e1 - H y| over the two columns of H
+    h1, h2 = np.array([1.0, s0, 0.0]), np.array([0.3, 0.5, 0.4])
+    nrm = np.cross(h1, h2)
+    want = [s0, abs(nrm[0]) / np.linalg.norm(nrm)]
+    np.testing.assert_allclose(res["err_hist"], want, rtol=1e-9)
+    assert res["iter"] == 2 and res["ierr"] == 1
