@@ -1405,10 +1405,12 @@ __device__ __forceinline__ void tile_each(double (&acc)[MT][NT][2], F&& f) {
       for (int b = 0; b < 2; ++b) f(r + 8 * i, c + 8 * q + b, acc[i][q][b]);
 }
 
-// 1/x to about an ulp for normal, finite x: one third-order Householder step
-// y (1 + e + e^2), e = 1 - x y, from the hardware's approximation (relative
-// error 2^-20); a chain of four operations after it, half the latency of a
-// division.
+// 1/x to about an ulp for x from the smallest normal to kRcpMax: one third-order
+// Householder step y (1 + e + e^2), e = 1 - x y, from the hardware's approximation
+// (relative error 2^-20); a chain of four operations after it, half the latency
+// of a division.  Above 2^1022 the reciprocal is subnormal and the approximation
+// gives 0.
+constexpr double kRcpMax = 0x1p1021;
 __device__ __forceinline__ double fast_rcp(double x) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
@@ -1421,8 +1423,8 @@ __device__ __forceinline__ double fast_rcp(double x) {
 // place without interchanges (DGETRF2's scaling: multipliers times the pivot's
 // reciprocal); rcp receives the reciprocals of the pivots (0 from d on).  True
 // in threads whose entry fails the certificate; a pivot that is zero, subnormal
-// (where DGETRF2 divides instead) or not finite fails it too, and the leaf goes
-// to the pivoted kernels, which follow DGETRF2 there.  Step t reads row and
+// (where DGETRF2 divides instead), above kRcpMax or not finite fails it too, and
+// the leaf goes to the pivoted kernels, which follow DGETRF2 there.  Step t reads row and
 // column t and writes only entries right of and below them, so one barrier a
 // step is enough.  One warp with eight entries a lane took 475 cycles a step
 // (its own 110 instructions), one entry a thread takes a third of that.
@@ -1450,7 +1452,7 @@ __device__ __forceinline__ bool lu_diag16(double* A, int d, double* rcp) {
     bad = !(fabs(a) <= kNoPivBound);
   } else if (r == c) {
     if (r < d)
-      bad = !(fabs(a) >= 2.2250738585072014e-308 && fabs(a) <= 1.7976931348623157e308);
+      bad = !(fabs(a) >= 2.2250738585072014e-308 && fabs(a) <= kRcpMax);
     else
       rcp[r] = 0.0;
   }

@@ -1,5 +1,5 @@
-"""Values at the edges of the solver's arithmetic: the rounding tie that decides
-on a second orthogonalisation."""
+"""Values at the edges of the solver's arithmetic: pivots whose reciprocal is
+subnormal, and the rounding tie that decides on a second orthogonalisation."""
 import ctypes as C
 
 import numpy as np
@@ -14,6 +14,43 @@ def _kappa():
     import tabipb
 
     return tabipb.kappa(BULK, EPS1)
+
+
+def test_pivots_above_the_reciprocal(gpu_lib):
+    """A dielectric ratio of 1e308: the diagonal of the blocks' first half is
+    5e307, whose reciprocal is subnormal.  B z = r with B as LEAFMATVECpara
+    assembles it; the subnormal reciprocals (1e-308, to 5e-324) leave 1e-13."""
+    import tabipb
+
+    kappa, eps = 0.1257, 1e308
+    case = born_case(1, radius=3.0)
+    with tabipb.TabiSolver(order=3, maxparnode=100, theta=0.8, eps0=1.0, eps1=eps, kappa=kappa,
+                           iprcd=1) as s:
+        xyz, nrm, ar, _ = s.form_matrix(case["sptpos"], case["sptnrm"], case["nvert"],
+                                        case["chrpos"], case["atmchr"])
+        s.build_tree()
+        n, o = s.nface, s.orderarr - 1
+        assert s.leaves()[1].size == 1
+        r = np.random.default_rng(1).normal(size=2 * n)
+        r[:n] *= 1e300
+        z = s.msolve(r)
+    xyz, nrm, ar = xyz[o], nrm[o], ar[o]
+    d = xyz[None] - xyz[:, None]
+    rs = np.sqrt((d ** 2).sum(-1))
+    own = rs == 0
+    rs[own] = 1.0
+    g0, e = 1 / (4 * np.pi * rs), np.exp(-kappa * rs)
+    c, c0 = (nrm[None] * d).sum(-1) / rs, (nrm[:, None] * d).sum(-1) / rs
+    t1, t2 = g0 / rs, (1 + kappa * rs) * e
+    g3 = (nrm @ nrm.T - 3 * c0 * c) / rs * t1
+    a = np.where(own, 0.0, ar[None])
+    k1, k2 = c * t1 * (1 - eps * t2) * a, g0 * (1 - e) * a
+    k3 = (g3 * (t2 - 1) - kappa ** 2 * c0 * c * e * g0) * a
+    k4 = c0 * t1 * (1 - t2 / eps) * a
+    y1 = .5 * (1 + eps) * z[:n] - k1 @ z[:n] - k3 @ z[n:]
+    y2 = .5 * (1 + 1 / eps) * z[n:] - k2 @ z[:n] - k4 @ z[n:]
+    assert np.abs(y1 - r[:n]).max() <= 1e-10 * 1e300
+    assert np.abs(y2 - r[n:]).max() <= 1e-10
 
 
 def test_second_orthogonalisation_at_the_tie(gpu_lib):
