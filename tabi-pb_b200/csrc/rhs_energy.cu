@@ -55,6 +55,39 @@ __device__ __forceinline__ void rhs_pair(double4 a, const double* r0, const doub
   b2 = fma(t * (inv * inv), vd, b2);
 }
 
+// b1 and b2 of a face whose rhs_pair sums are not finite, by the library's root
+// and the factors in the reference's order: fast_rsqrt(0) is NaN where 1/rs is
+// Inf (an atom on the face's centroid), and the sums without 1/(4 pi) overflow
+// first.
+__device__ __noinline__ double2 rhs_edge(const double* __restrict__ atoms4, int nchr, double rx,
+                                         double ry, double rz, double vx, double vy, double vz) {
+  double b1 = 0.0, b2 = 0.0;
+  for (int k = 0; k < nchr; ++k) {
+    const double* a = atoms4 + 4 * (size_t)k;
+    const double dx = a[0] - rx, dy = a[1] - ry, dz = a[2] - rz;
+    const double inv = rsqrt(fma(dx, dx, fma(dy, dy, dz * dz)));
+    const double cosr = fma(vx, dx, fma(vy, dy, vz * dz)) * inv;
+    b1 = fma(a[3], kOneOver4Pi * inv, b1);
+    b2 = fma(a[3], cosr * inv * inv * kOneOver4Pi, b2);
+  }
+  return make_double2(b1, b2);
+}
+
+// face i's entries of the right-hand side from its rhs_pair sums
+__device__ __forceinline__ void rhs_store(double* __restrict__ b, int i, int nface, double b1,
+                                          double b2, const double* __restrict__ atoms4, int nchr,
+                                          const double* r0, const double* v0, double eps0) {
+  b1 *= kOneOver4Pi;
+  b2 *= kOneOver4Pi;
+  if (!(isfinite(b1) && isfinite(b2))) {
+    const double2 e = rhs_edge(atoms4, nchr, r0[0], r0[1], r0[2], v0[0], v0[1], v0[2]);
+    b1 = e.x;
+    b2 = e.y;
+  }
+  b[i] = b1 / eps0;
+  b[nface + i] = b2 / eps0;
+}
+
 // atoms4: (x, y, z, q) per atom
 __global__ void __launch_bounds__(kFaceThreads) form_matrix_kernel(
     const double* __restrict__ sptpos, const double* __restrict__ sptnrm,
@@ -101,10 +134,7 @@ __global__ void __launch_bounds__(kFaceThreads) form_matrix_kernel(
 #pragma unroll 4
       for (int q = 0; q < cnt; ++q) rhs_pair(sa[q], r0, v0, b1, b2);
   }
-  if (own) {
-    b[i] = b1 * kOneOver4Pi / eps0;
-    b[nface + i] = b2 * kOneOver4Pi / eps0;
-  }
+  if (own) rhs_store(b, i, nface, b1, b2, atoms4, nchr, r0, v0, eps0);
 }
 
 // RHS only, surface already loaded (SoA)
@@ -141,10 +171,7 @@ __global__ void __launch_bounds__(kFaceThreads) rhs_kernel(const double* __restr
 #pragma unroll 4
       for (int q = 0; q < cnt; ++q) rhs_pair(sa[q], r0, v0, b1, b2);
   }
-  if (own) {
-    b[i] = b1 * kOneOver4Pi / eps0;
-    b[nface + i] = b2 * kOneOver4Pi / eps0;
-  }
+  if (own) rhs_store(b, i, nface, b1, b2, atoms4, nchr, r0, v0, eps0);
 }
 
 constexpr int kEA = 8;  // atoms per energy block

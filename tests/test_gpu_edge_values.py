@@ -1,5 +1,6 @@
 """Values at the edges of the solver's arithmetic: pivots whose reciprocal is
-subnormal, and the rounding tie that decides on a second orthogonalisation."""
+subnormal, atoms on a face's centroid, and the rounding tie that decides on a
+second orthogonalisation."""
 import ctypes as C
 
 import numpy as np
@@ -51,6 +52,32 @@ def test_pivots_above_the_reciprocal(gpu_lib):
     y2 = .5 * (1 + 1 / eps) * z[n:] - k2 @ z[:n] - k4 @ z[n:]
     assert np.abs(y1 - r[:n]).max() <= 1e-10 * 1e300
     assert np.abs(y2 - r[n:]).max() <= 1e-10
+
+
+@pytest.mark.parametrize("charge", [1.5, -1.5])
+def test_atom_on_a_centroid(gpu_lib, charge):
+    """1/|d| is infinite for the face whose centroid is the atom's place, and
+    that face alone: its potential half is +-Inf, its field half (0 * Inf) NaN,
+    from tabi_form_matrix and tabi_rhs alike."""
+    import tabipb
+
+    case = born_case(2, radius=3.0)
+    # more atoms than one staged tile, the one on the centroid in the second
+    chrpos = np.random.default_rng(0).normal(size=(700, 3)) * 0.3
+    q = np.full(700, 0.01)
+    args = case["sptpos"], case["sptnrm"], case["nvert"]
+    with tabipb.TabiSolver(order=3, maxparnode=100, theta=0.8, eps0=EPS0, eps1=EPS1,
+                           kappa=_kappa()) as s:
+        xyz, _, _, b0 = s.form_matrix(*args, chrpos, q)
+        n, k = s.nface, 77
+        chrpos[600], q[600] = xyz[k], charge
+        b = s.form_matrix(*args, chrpos, q)[3]
+        rhs = s.rhs(chrpos, q)
+    assert np.isfinite(b0).all()
+    for v in (b, rhs):
+        assert v[k] == np.copysign(np.inf, charge) and np.isnan(v[n + k])
+        rest = np.delete(v, [k, n + k])
+        assert np.isfinite(rest).all()
 
 
 def test_second_orthogonalisation_at_the_tie(gpu_lib):
