@@ -1,6 +1,6 @@
 """Values at the edges of the solver's arithmetic: pivots whose reciprocal is
-subnormal, atoms on a face's centroid, and the rounding tie that decides on a
-second orthogonalisation."""
+subnormal, atoms on a face's centroid, gates far below zero, and the rounding tie
+that decides on a second orthogonalisation."""
 import ctypes as C
 
 import numpy as np
@@ -78,6 +78,42 @@ def test_atom_on_a_centroid(gpu_lib, charge):
         assert v[k] == np.copysign(np.inf, charge) and np.isnan(v[n + k])
         rest = np.delete(v, [k, n + k])
         assert np.isfinite(rest).all()
+
+
+@pytest.mark.parametrize("x", [-87.0, -87.5, -88.0, -88.6, -88.8, -95.0])
+def test_gate_far_below_zero(gpu_lib, x):
+    """silu(x) for x around -ln(FLT_MAX), where the sigmoid is subnormal: the
+    input layer's output, with zero message-passing layers, times 1e36.  The
+    exponential's argument is rounded to 2^-24 of 88 (5e-6 of its value), the
+    subnormal quotient to 2^-149 (4e-7 of 3e-39); e^88.73 and above overflows
+    and gives 0."""
+    import torch
+    import warmstart_ref as W
+
+    from tabipb.warmstart import WarmStart
+
+    hidden = 32
+    theta = {n: np.zeros(s, np.float32) for n, s in W.param_shapes(hidden, 1, 8)}
+    theta["b0"][:] = x
+    theta["Wo"][:, 0] = 1e36
+    ws = WarmStart(hidden=hidden, layers=1, seed=0)
+    ws.set_params(np.concatenate([theta[n].ravel() for n, _ in W.param_shapes(hidden, 1, 8)]))
+    import oracle as O
+
+    c = born_case(1, radius=3.0)
+    xyz, tq, ar, b = O.form_matrix(c["sptpos"], c["sptnrm"], c["nvert"], c["chrpos"] + 0.4,
+                                   c["atmchr"], 1.0)
+    n = len(ar)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a, dtype=np.float64).ravel()).cuda()
+    s = dict(n=n, xyz=t(xyz), tq=t(tq), area=t(ar), b=t(b), z=t(0 * b), x=t(b))
+    out = torch.empty_like(s["b"])
+    ws.predict_dev(s, out)
+    out = out.cpu().numpy()[:n] / np.sqrt(np.mean(b[:n] ** 2))
+    wo = float(W.bf16_round(np.float32([1e36]))[0])
+    want = hidden * wo * x / (1.0 + np.exp(-float(np.float32(x))))
+    if x < -88.73:
+        want = 0.0
+    assert np.abs(out - want).max() <= 1e-4 * abs(want)
 
 
 def test_second_orthogonalisation_at_the_tie(gpu_lib):
