@@ -852,7 +852,7 @@ __global__ void __launch_bounds__(kUT, 2) lu_gemm_kernel(const int4* __restrict_
                                                          const int2* __restrict__ leaf_rng,
                                                          const int64_t* __restrict__ blk_off,
                                                          double* __restrict__ lu) {
-  extern __shared__ double gsm[];
+  extern __shared__ __align__(16) double gsm[];
   double* sLb = gsm;                      // [2][kBP][kGT]: L slice, k-major
   double* sUb = gsm + 2 * kBP * kGT;      // [2][kGT][kUPitch]: U slice, by column
   const int4 it = items[blockIdx.x];

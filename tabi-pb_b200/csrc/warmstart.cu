@@ -704,7 +704,7 @@ __global__ void __launch_bounds__(256) ws_agg_bwd_w_kernel(
     const __nv_bfloat16* __restrict__ Wf, const float* __restrict__ bfv,
     const float* __restrict__ u, const float* __restrict__ da, float* __restrict__ part) {
   __shared__ EdgeStage S;
-  __shared__ float red[kGrp][256];
+  __shared__ __align__(16) float red[kGrp][256];
   const int g = threadIdx.x / (H / 4), c = 4 * (threadIdx.x % (H / 4));
   Chan4 ch;
   ch.load(Wf, bfv, H, c);
