@@ -93,6 +93,17 @@ int tabi_create(tabi_h* h, const tabi_params* p);
 int tabi_destroy(tabi_h h);
 const char* tabi_last_error(tabi_h h);
 
+/* Gives back to the driver what the library keeps of destroyed handles and
+ * networks for the next one: device memory (at most 4 GiB per device),
+ * page-locked memory (256 MiB) and the streams and events of 16 handles, all
+ * for the current device.  Live objects keep theirs.  Without this call they are
+ * kept until the process ends, or until an allocation of the library's own
+ * fails; another allocator in the process does not see them as free.
+ * cudaDeviceReset, once every handle and network of the device is destroyed,
+ * leaves nothing behind either: the next tabi_create starts anew.  No
+ * counterpart in the reference. */
+int tabi_release_cache(void);
+
 /* main.f90:546-610 form_matrix.  sptpos/sptnrm: 3 x nspt vertices and
  * vertex normals (MSMS .vert), nvert: 3 x nface 1-based (MSMS .face, already
  * filtered by readin.f90:264-333 surface_area), chrpos: 3 x nchr, atmchr:

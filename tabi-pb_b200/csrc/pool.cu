@@ -7,16 +7,40 @@
 // streams and their events -- of 17.5 ms for a 1,031-atom protein of 24k faces,
 // 7.5 in creating and destroying the handle and 2 in the allocations of its
 // first tree.  Blocks that an object gives back stay here for the next one, up
-// to a bound per device; beyond it, and when an allocation fails, they go back
-// to the driver.
+// to a bound per context; beyond it, when an allocation fails, and when the
+// program asks (tabi_release_cache), they go back to the driver.
+//
+// Everything is kept by the CUDA context that owns it and is only handed out or
+// freed while that context is current: the id of a context is unique for the
+// life of the process, so nothing of a context that cudaDeviceReset destroyed is
+// met again.
+#include <cuda.h>
+
 #include "tabi_impl.cuh"
 
 namespace tabi {
 
+unsigned long long context_id(bool create) {
+  using Query = CUresult (*)(CUcontext, unsigned long long*);
+  static const Query query = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess)
+      f = nullptr;
+    return reinterpret_cast<Query>(f);
+  }();
+  unsigned long long id = 0;
+  if (!query) return 0;
+  if (query(nullptr, &id) == CUDA_SUCCESS) return id;
+  // no context yet, or one that a reset destroyed: the runtime's next call makes one
+  if (!create || cudaFree(nullptr) != cudaSuccess) return 0;
+  return query(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+}
+
 namespace {
 
-// device blocks kept per device, page-locked blocks kept in all, resource
-// bundles kept per device
+// per context: device blocks and page-locked blocks kept, resource bundles kept
 constexpr size_t kMaxDevice = size_t(4) << 30, kMaxPinned = size_t(256) << 20;
 constexpr size_t kMaxRes = 16;
 
@@ -27,11 +51,14 @@ struct Shelf {
   size_t total = 0;
 };
 
+struct Store {
+  Shelf dev, pinned;
+  std::vector<HandleRes> res;
+};
+
 struct Pool {
   std::mutex mu;
-  std::map<int, Shelf> dev;  // by device
-  Shelf pinned;
-  std::map<int, std::vector<HandleRes>> res;
+  std::map<unsigned long long, Store> ctx;  // by context id
 };
 
 // never destroyed: blocks that live to the end of the process go with it
@@ -50,11 +77,13 @@ void trim(Shelf& sh, bool pinned) {
 
 MemPool::Block MemPool::get(size_t bytes, bool pinned) {
   Block b;
-  if (!pinned) TABI_CUDA(cudaGetDevice(&b.device));
-  {
+  b.pinned = pinned;
+  b.ctx = context_id(true);
+  if (b.ctx) {
     Pool& P = pool();
     std::lock_guard<std::mutex> lk(P.mu);
-    Shelf& sh = pinned ? P.pinned : P.dev[b.device];
+    Store& st = P.ctx[b.ctx];
+    Shelf& sh = pinned ? st.pinned : st.dev;
     auto it = sh.blocks.lower_bound(bytes);
     // at most twice the request, so that a small object does not hold a large
     // one's block
@@ -76,10 +105,11 @@ MemPool::Block MemPool::get(size_t bytes, bool pinned) {
   cudaError_t e = alloc();
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
-    {
+    if (b.ctx) {
       Pool& P = pool();
       std::lock_guard<std::mutex> lk(P.mu);
-      trim(pinned ? P.pinned : P.dev[b.device], pinned);
+      Store& st = P.ctx[b.ctx];
+      trim(pinned ? st.pinned : st.dev, pinned);
     }
     e = alloc();
     if (e == cudaErrorMemoryAllocation) {
@@ -94,23 +124,36 @@ MemPool::Block MemPool::get(size_t bytes, bool pinned) {
 
 void MemPool::put(Block b) {
   if (!b.p) return;
-  const bool pinned = b.device < 0;
-  bool keep = true;
-  if (!pinned && tl_idle == 0) keep = cudaDeviceSynchronize() == cudaSuccess;
-  int cur = 0;
-  if (!pinned && (cudaGetDevice(&cur) != cudaSuccess || cur != b.device))
-    keep = false;  // another device is current: its work is not known to be done
+  // under another context the owner's work is not known to be done
+  bool keep = b.ctx != 0 && b.ctx == context_id(false);
+  if (keep && !b.pinned && tl_idle == 0) keep = cudaDeviceSynchronize() == cudaSuccess;
   if (keep) {
     Pool& P = pool();
     std::lock_guard<std::mutex> lk(P.mu);
-    Shelf& sh = pinned ? P.pinned : P.dev[b.device];
-    if (sh.total + b.bytes <= (pinned ? kMaxPinned : kMaxDevice)) {
+    Store& st = P.ctx[b.ctx];
+    Shelf& sh = b.pinned ? st.pinned : st.dev;
+    if (sh.total + b.bytes <= (b.pinned ? kMaxPinned : kMaxDevice)) {
       sh.blocks.emplace(b.bytes, b.p);
       sh.total += b.bytes;
       return;
     }
   }
-  pinned ? cudaFreeHost(b.p) : cudaFree(b.p);
+  b.pinned ? cudaFreeHost(b.p) : cudaFree(b.p);
+}
+
+void MemPool::release() {
+  Store st;
+  {
+    Pool& P = pool();
+    std::lock_guard<std::mutex> lk(P.mu);
+    auto it = P.ctx.find(context_id(false));
+    if (it == P.ctx.end()) return;
+    std::swap(st, it->second);
+    P.ctx.erase(it);
+  }
+  trim(st.dev, false);
+  trim(st.pinned, true);
+  for (HandleRes& r : st.res) r.destroy();
 }
 
 MemPool::Idle::Idle() {
@@ -121,11 +164,12 @@ MemPool::Idle::~Idle() {
   if (ok) --tl_idle;
 }
 
-HandleRes HandleRes::get(int device) {
-  {
+HandleRes HandleRes::get() {
+  const unsigned long long id = context_id(true);
+  if (id) {
     Pool& P = pool();
     std::lock_guard<std::mutex> lk(P.mu);
-    std::vector<HandleRes>& v = P.res[device];
+    std::vector<HandleRes>& v = P.ctx[id].res;
     if (!v.empty()) {
       HandleRes r = v.back();
       v.pop_back();
@@ -133,6 +177,7 @@ HandleRes HandleRes::get(int device) {
     }
   }
   HandleRes r;
+  r.ctx = id;
   try {
     int prio_lo = 0, prio_hi = 0;
     TABI_CUDA(cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi));
@@ -152,11 +197,11 @@ HandleRes HandleRes::get(int device) {
   return r;
 }
 
-void HandleRes::put(int device, bool idle) {
-  if (idle && stream && h_pinned) {
+void HandleRes::put(bool idle) {
+  if (idle && stream && h_pinned && ctx != 0 && ctx == context_id(false)) {
     Pool& P = pool();
     std::lock_guard<std::mutex> lk(P.mu);
-    std::vector<HandleRes>& v = P.res[device];
+    std::vector<HandleRes>& v = P.ctx[ctx].res;
     if (v.size() < kMaxRes) {
       v.push_back(*this);
       return;

@@ -388,7 +388,7 @@ int tabi_create(tabi_h* h, const tabi_params* p) {
     nh->H.mv_prec = p->precision;
     TABI_CUDA(cudaGetDevice(&nh->H.device));
     Handle& H = nh->H;
-    H.res = HandleRes::get(H.device);
+    H.res = HandleRes::get();
     H.stream = H.res.stream;
     H.side = H.res.side;
     H.lu_hi = H.res.lu_hi;
@@ -414,10 +414,13 @@ int tabi_destroy(tabi_h h) {
   cudaSetDevice(h->H.device);
   MemPool::Idle idle;  // all work on the handle's buffers, on any stream, is done
   HandleRes res = h->H.res;
-  const int device = h->H.device;
   delete h;
-  res.put(device, idle.ok);
+  res.put(idle.ok);
   return TABI_OK;
+}
+
+int tabi_release_cache(void) {
+  return guarded(nullptr, [] { MemPool::release(); });
 }
 
 const char* tabi_last_error(tabi_h h) { return h ? h->H.err.c_str() : g_err.c_str(); }

@@ -43,6 +43,10 @@ struct Error : std::runtime_error {
     if (!(cond)) throw ::tabi::Error((code), (msg));    \
   } while (0)
 
+// Id of the current CUDA context, never used again in the process; 0 if there is
+// none (create: one is made then) or it cannot be told.
+unsigned long long context_id(bool create);
+
 // Cache of device and page-locked memory blocks (pool.cu), shared by all
 // handles and threads.  A block goes back when the GPU is done with it: put
 // waits for the device, as cudaFree does, unless the thread holds an Idle,
@@ -51,10 +55,12 @@ struct MemPool {
   struct Block {
     void* p = nullptr;
     size_t bytes = 0;
-    int device = -1;  // -1: page-locked
+    bool pinned = false;
+    unsigned long long ctx = 0;  // the context it belongs to
   };
   static Block get(size_t bytes, bool pinned);
   static void put(Block b);
+  static void release();  // the current context's idle blocks and bundles to the driver
   struct Idle {
     bool ok;
     Idle();
@@ -65,15 +71,16 @@ struct MemPool {
 };
 
 // Streams, events and a small page-locked scratch of one handle, kept for the
-// next handle of the device.
+// next handle of the context.
 struct HandleRes {
   cudaStream_t stream = nullptr, side = nullptr, lu_hi = nullptr, aux = nullptr,
                lu_small = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_la = nullptr, ev_rest = nullptr,
               ev_lu_join = nullptr;
   double* h_pinned = nullptr;
-  static HandleRes get(int device);
-  void put(int device, bool idle);  // idle: the device has finished the streams' work
+  unsigned long long ctx = 0;  // the context they belong to
+  static HandleRes get();
+  void put(bool idle);  // idle: the device has finished the streams' work
   void destroy();
 };
 
@@ -529,12 +536,11 @@ inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 // own molecule's need: one thread could lower it under another's launch.
 inline void raise_smem_limit(const void* func, size_t bytes) {
   static std::mutex mu;
-  static std::map<std::pair<const void*, int>, size_t> high;
-  int dev = 0;
-  TABI_CUDA(cudaGetDevice(&dev));
+  static std::map<std::pair<const void*, unsigned long long>, size_t> high;
+  const unsigned long long ctx = context_id(true);
   std::lock_guard<std::mutex> lk(mu);
-  size_t& h = high[{func, dev}];
-  if (bytes <= h) return;
+  size_t& h = high[{func, ctx}];
+  if (ctx != 0 && bytes <= h) return;
   TABI_CUDA(cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
   h = bytes;
 }

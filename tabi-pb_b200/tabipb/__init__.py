@@ -5,4 +5,4 @@ package binds its C ABI (include/tabi_gpu.h) and provides the input formats.
 """
 from ._lib import FLAG_PIVOTED_LU, PREC_FP64, PREC_MIXED, TabiError, load  # noqa: F401
 from .solver import (TabiSolver, default_params, kappa, probe_fp32_peak, probe_fp64_peak,  # noqa: F401
-                     solve_molecule)
+                     release_cache, solve_molecule)

@@ -36,6 +36,7 @@ SYMBOLS = [
     "tabi_output_potential", "tabi_output_potential_dev", "tabi_set_target_range",
     "tabi_direct_targets", "tabi_pivoted_leaves", "tabi_probe_fp32_peak",
     "tabi_face_filter_dev", "tabi_set_exchange",
+    "tabi_release_cache",
 ]
 
 # tabi_exchange_fn: int (*)(void* user, double* v_dev, int n2, int t0, int t1, void* stream)
@@ -140,6 +141,7 @@ def load(path: str = LIB_PATH):
     L.tabi_pivoted_leaves.argtypes = [_vp, _ip]
     L.tabi_output_potential.argtypes = [_vp, C.c_int, _dp, C.c_int, _ip, _dp, _dp, _dp]
     L.tabi_output_potential_dev.argtypes = [_vp, C.c_int, _vp, C.c_int, _vp, _vp, _vp, _vp, _vp]
+    L.tabi_release_cache.argtypes = []
     L.tabi_batch_run_dev.argtypes = [C.POINTER(Params), C.c_int, C.POINTER(MolDev), _vp, C.c_int,
                                      _dp]
     for s in SYMBOLS:

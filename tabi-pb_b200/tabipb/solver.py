@@ -316,6 +316,14 @@ class TabiSolver:
                     near_pairs=int(st[5]), far=int(st[6]), nleaf=int(st[7]))
 
 
+def release_cache():
+    """Gives the memory, streams and events that closed solvers left for the next
+    one back to the driver (tabi_release_cache)."""
+    rc = _lib.load().tabi_release_cache()
+    if rc != 0:
+        raise TabiError(rc, _lib.load().tabi_last_error(None).decode())
+
+
 def probe_fp64_peak(ms=200.0) -> float:
     f = C.c_double()
     rc = _lib.load().tabi_probe_fp64_peak(ms, C.byref(f))
