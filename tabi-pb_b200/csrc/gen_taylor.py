@@ -326,6 +326,7 @@ def main():
     L.append("template <int P, typename T>")
     L.append("__device__ __forceinline__ void far_eval(T dx, T dy, T dz, T kappa, const float4* __restrict__ Mw,")
     L.append("                                         T n0, T n1, T n2, T eps, T inv_eps, T& o1, T& o2) {")
+    L.append('  static_assert(sizeof(T) == sizeof(float), "the moments are FP32");')
     for p in range(1, maxp + 1):
         kw = "if" if p == 1 else "else if"
         L.append(f"  {kw} constexpr (P == {p}) far_eval_p{p}<T>(dx, dy, dz, kappa, Mw, n0, n1, n2, eps, inv_eps, o1, o2);")
