@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(128) harm_final_kernel(const int2* __restrict_
 
 // ---- far field
 // FP64 (harmonic.cuh): one block per (cluster, up to 64 NT of its targets), NT =
-// far_pair(P) targets per thread, which share every coefficient's shared load.
+// far_nt targets per thread, which share every coefficient's shared load.
 
 template <int P, int NT>
 __global__ void __launch_bounds__(kFarThreads) far_harm_kernel(
@@ -292,7 +292,7 @@ constexpr int far_blocks(int p) {
 }
 
 template <int P>
-__global__ void __launch_bounds__(64, far_blocks(P)) far_kernel(const WorkItem* __restrict__ work,
+__global__ void __launch_bounds__(kFarThreads, far_blocks(P)) far_kernel(const WorkItem* __restrict__ work,
                                                  const int2* __restrict__ ent,
                                                  const float* __restrict__ mw,
                                                  const double* __restrict__ nd_mid,
@@ -310,16 +310,16 @@ __global__ void __launch_bounds__(64, far_blocks(P)) far_kernel(const WorkItem* 
   for (int q = threadIdx.x; q < 4 * NT; q += blockDim.x) smw[q] = src[q];
   __syncthreads();
   for (int k = threadIdx.x; k < wi.count; k += blockDim.x) {
-  int2 e = ent[wi.start + k];
-  int t = e.x;
-  // COMP_TCOEFF :707-709: dx = target - mid
-  float dx = (float)(px[t] - nd_mid[3 * wi.node]);
-  float dy = (float)(py[t] - nd_mid[3 * wi.node + 1]);
-  float dz = (float)(pz[t] - nd_mid[3 * wi.node + 2]);
-  float o1, o2;
-  far_eval<P, float>(dx, dy, dz, kappa, smw, (float)nx[t], (float)ny[t], (float)nz[t], eps,
-                     1.f / eps, o1, o2);
-  res[e.y] = make_double2((double)o1 * kOneOver4Pi, (double)o2 * kOneOver4Pi);
+    const int2 e = ent[wi.start + k];
+    const int t = e.x;
+    // COMP_TCOEFF :707-709: dx = target - mid
+    const float dx = (float)(px[t] - nd_mid[3 * wi.node]);
+    const float dy = (float)(py[t] - nd_mid[3 * wi.node + 1]);
+    const float dz = (float)(pz[t] - nd_mid[3 * wi.node + 2]);
+    float o1, o2;
+    far_eval<P, float>(dx, dy, dz, kappa, smw, (float)nx[t], (float)ny[t], (float)nz[t], eps,
+                       1.f / eps, o1, o2);
+    res[e.y] = make_double2((double)o1 * kOneOver4Pi, (double)o2 * kOneOver4Pi);
   }
 }
 
@@ -593,13 +593,14 @@ void launch_far(Handle& H, bool f32, cudaStream_t s) {
   const double eps = H.prm.eps1 / H.prm.eps0;
   TABI_K(K_FAR, s);
   if (f32)
-    far_kernel<P><<<nw, 64, 0, s>>>(
+    far_kernel<P><<<nw, kFarThreads, 0, s>>>(
         fw, fe, H.d_mwf.p, T.d_mid.p, H.d_x.p, H.d_y.p, H.d_z.p,
         H.d_nx.p, H.d_ny.p, H.d_nz.p, (float)H.prm.kappa, (float)eps, H.d_res.p);
   else
-    far_harm_kernel<P, far_pair(P)><<<nw, kFarThreads, 0, s>>>(
-        fw, fe, H.d_mw.p, T.d_mid.p, H.d_x.p, H.d_y.p, H.d_z.p,
-        H.d_nx.p, H.d_ny.p, H.d_nz.p, H.prm.kappa, 1.0 / eps, H.d_res.p);
+    (T.far_nt > 1 ? far_harm_kernel<P, far_pair(P)> : far_harm_kernel<P, 1>)<<<
+        nw, kFarThreads, 0, s>>>(fw, fe, H.d_mw.p, T.d_mid.p, H.d_x.p, H.d_y.p, H.d_z.p,
+                                 H.d_nx.p, H.d_ny.p, H.d_nz.p, H.prm.kappa, 1.0 / eps,
+                                 H.d_res.p);
 }
 
 // FP32 copies of the faces relative to their leaf centres (once per tree)

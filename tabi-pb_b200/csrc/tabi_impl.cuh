@@ -252,6 +252,7 @@ struct Tree {
   PinVec<WorkItem> far_work, near_work;  // page-locked: uploaded per tree
   DBuf<WorkItem> d_far_work, d_near_work;
   int near_split = 1;  // threads per target of the FP64 near field (near_work's chunks)
+  int far_nt = 1;      // targets per thread of the FP64 far field (far_work's chunks)
   int nmslot = 0;
   std::vector<int> mslot_node;  // node id per moment slot
   DBuf<int> d_mslot_node;

@@ -663,7 +663,13 @@ void build_lists(Handle& H, cudaStream_t s) {
       far_cnt.p, near_cnt.p, T.d_far_ent.p, T.d_near_ent.p, H.d_err.p); }
   // work items and moment slots
   const int kMomChunk = 256;
-  const int far_chunk = kFarThreads * far_pair(H.prm.order);
+  // A mixed-precision handle's FP32 far field takes the same items and their targets
+  // in turn: pairs make its blocks too few until the list is long (operator apply
+  // at 474 faces, orders 6 and 8: 55 and 74 us with 64 targets per item, 65 and 105
+  // with 128; 60,244 faces, order 6, 3.7 M interactions: 894 and 916; from 25 M
+  // on the FP64 one's gain decides: the solve of 403,820 faces 123.0 and 122.0 ms).
+  T.far_nt = H.prm.precision == TABI_PREC_MIXED && tf < (8 << 20) ? 1 : far_pair(H.prm.order);
+  const int far_chunk = kFarThreads * T.far_nt;
   // threads per target of the FP64 near field, as few as give every SM 8 blocks
   // of 128 threads: below that the SMs idle (1,272 targets: 49 us with one, 20
   // with 16), above it more threads only stage the same leaf more often.  The

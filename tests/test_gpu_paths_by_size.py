@@ -1,0 +1,61 @@
+"""Kernels that a call takes by its size, on both sides of each line, against the
+CPU oracle or the other form."""
+import numpy as np
+import pytest
+
+from conftest import BULK, EPS0, EPS1, born_case, molecule_case
+
+pytestmark = pytest.mark.gpu
+
+
+def _solver(case, **kw):
+    import tabipb
+
+    kw = dict(dict(order=3, maxparnode=500, theta=0.8, eps0=EPS0, eps1=EPS1,
+                   kappa=tabipb.kappa(BULK, EPS1), iprcd=0), **kw)
+    s = tabipb.TabiSolver(**kw)
+    g = s.form_matrix(case["sptpos"], case["sptnrm"], case["nvert"], case["chrpos"],
+                      case["atmchr"])
+    s.build_tree()
+    return s, g
+
+
+# far lists below and above 8 M interactions: a mixed handle's items of 64 and of
+# 128 targets.  The FP32 sums hold some 1e-6 of cancelling terms (the bar of the
+# mixed operator's own tests); the handle's FP64 operator is the FP64 handle's, up
+# to the order of each target's sums.
+@pytest.mark.parametrize("order", [6, 7, 8])
+@pytest.mark.parametrize("level,leaf", [(3, 20), (6, 30)])
+def test_mixed_far_items(gpu_lib, order, level, leaf):
+    import tabipb
+
+    case = born_case(level, radius=6.0)
+    kw = dict(order=order, maxparnode=leaf, theta=0.4 if level > 3 else 0.8, tol=1e-9)
+    with _solver(case, **kw)[0] as s:
+        n = s.nface
+        far = s.counts()[1]
+        x = np.random.default_rng(order).normal(size=2 * n)
+        y = s.matvec(x)
+    with _solver(case, precision=tabipb.PREC_MIXED, **kw)[0] as s:
+        assert s.counts()[1] == far
+        y32 = s.matvec(x)
+    assert (far >= 8 << 20) == (level > 3)
+    assert np.linalg.norm(y32 - y) <= 2e-5 * np.linalg.norm(y)
+
+
+@pytest.mark.parametrize("order", [6, 8])
+def test_mixed_far_field_in_double(gpu_lib, order):
+    """The FP64 residual of a small mixed solve takes one target per thread, the
+    FP64 handle's operator two: the mixed solution satisfies the latter."""
+    import tabipb
+
+    case = molecule_case(60, 6.0, 2.0, seed=2)
+    kw = dict(order=order, maxparnode=100, theta=0.7, iprcd=1, tol=1e-9)
+    with _solver(case, precision=tabipb.PREC_MIXED, **kw)[0] as s:
+        b = np.random.default_rng(order).normal(size=2 * s.nface)
+        r = s.dgmres(b)
+    assert r["ierr"] == 0
+    with _solver(case, **kw)[0] as s:
+        d = s.msolve(b - s.matvec(r["x"]))
+        m = s.msolve(b)
+    assert np.linalg.norm(d) <= 1.01e-9 * np.linalg.norm(m)
