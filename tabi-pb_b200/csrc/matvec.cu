@@ -23,6 +23,7 @@
 // All results are written to per-(target, interaction) slots fixed by the
 // traversal, so the sums are deterministic.
 #include <algorithm>
+#include <type_traits>
 
 #include "bie_kernels.cuh"
 #include "fast_math.cuh"
@@ -37,47 +38,55 @@ namespace {
 
 // ---- moments
 // Cartesian moments of the mixed-precision far field, summed in FP64.  A group
-// of G threads takes a chunk of up to 256 sources of a cluster, a thread one
-// term of the 4 raw sets: the powers of 64 sources at a time and the 4 charges
-// lie in shared memory, and 7 shared words serve 4 sums (a thread per (set,
-// term) read 4 words for each of its own).  Every sum runs over its chunk's
-// sources in order.
-template <int P>
+// of G threads takes a chunk of up to 256 sources of a cluster, a thread S of the 4
+// raw sets of a term: the powers of 64 sources at a time and the 4 charges lie in
+// shared memory, and with S = 4 seven shared words serve 4 sums, with S = 1 four
+// words each sum.  Every sum runs over its chunk's sources in order, so S changes
+// no bit.  S = 1 up to order 5 while there are few (source, term) pairs (kMomFew),
+// where the length of a thread's loop counts and not its loads: order 3, leaves of
+// up to 400, S = 1 and 4: 1,098 faces 5.9 and 9.5 us, 11,184 faces 8.8 and 17.0,
+// 28,550 faces 22.0 and 19.8; order 5, 7,328 faces 10.4 and 11.8, 11,184 faces 13.6
+// and 12.1; order 6, 7,328 faces 17.7 and 14.3.
+template <int P, int S>
 struct MomShape {
-  static constexpr int NT = tabi_nterms(P), W = 3 * (P + 1) + 4, TILE = 64;
-  static constexpr int G = (NT + 31) / 32 * 32, CPB = G >= 128 ? 1 : 128 / G;
-  static constexpr int PITCH = (W + 1) / 2 * 2;  // 16-byte aligned rows
+  static constexpr int NT = tabi_nterms(P), W = 3 * (P + 1) + 4, TILE = S == 1 ? 128 : 64;
+  static constexpr int G = (NT * (4 / S) + 31) / 32 * 32;
+  static constexpr int CPB = S == 1 || G >= 128 ? 1 : 128 / G;
+  static constexpr int PITCH = S == 1 ? W : (W + 1) / 2 * 2;  // S = 4: 16-byte aligned rows
 };
+constexpr int64_t kMomFew = 400000;
 
-template <int P>
-__global__ void __launch_bounds__(MomShape<P>::G* MomShape<P>::CPB) mom_partial_kernel(
+template <int P, int S>
+__global__ void __launch_bounds__(MomShape<P, S>::G* MomShape<P, S>::CPB) mom_partial_kernel(
     const int4* __restrict__ chunks, int nchunk, const int* __restrict__ mslot_node,
     const double* __restrict__ nd_mid, const double* __restrict__ px,
     const double* __restrict__ py, const double* __restrict__ pz, const double* __restrict__ nx,
     const double* __restrict__ ny, const double* __restrict__ nz,
     const double* __restrict__ area, const double* __restrict__ x, int n,
     double* __restrict__ mraw) {
-  using M = MomShape<P>;
+  using M = MomShape<P, S>;
   constexpr int NT = M::NT, TILE = M::TILE, G = M::G;
   __shared__ __align__(16) double stage[M::CPB][TILE][M::PITCH];
-  const int g = threadIdx.x / G, term = threadIdx.x % G;
+  const int g = threadIdx.x / G, t = threadIdx.x % G;
+  const int set0 = t / NT, term = t - set0 * NT;  // S = 4: set0 is 0 for every term
+  const bool own = t < NT * (4 / S);
   const int c = blockIdx.x * M::CPB + g;
   const int4 ch = c < nchunk ? chunks[c] : make_int4(0, 0, 0, 0);
   const int node = mslot_node[ch.x];
   const double mx = nd_mid[3 * node], my = nd_mid[3 * node + 1], mz = nd_mid[3 * node + 2];
   double(*st)[M::PITCH] = stage[g];
   int k1 = 0, k2 = 0, k3 = 0;
-  if (term < NT) {
+  if (own) {
     const signed char(*tt)[3] = tabi_terms<P>();
     k1 = 4 + tt[term][0];
     k2 = 4 + P + 1 + tt[term][1];
     k3 = 4 + 2 * (P + 1) + tt[term][2];
   }
-  double acc[4] = {};
+  double acc[S] = {};
   for (int base = 0; base < 256; base += TILE) {
     const int cnt = min(TILE, ch.z - base);
     if (__syncthreads_and(cnt <= 0)) break;
-    for (int q = term; q < cnt; q += G) {
+    for (int q = t; q < cnt; q += G) {
       const int i = ch.y + base + q;
       // COMP_MS :876-889: dx = x - mid, powers by repeated multiplication
       const double dx = px[i] - mx, dy = py[i] - my, dz = pz[i] - mz;
@@ -99,21 +108,25 @@ __global__ void __launch_bounds__(MomShape<P>::G* MomShape<P>::CPB) mom_partial_
       st[q][3] = (nz[i] * A) * x1;
     }
     __syncthreads();
-    if (term < NT)
+    if (own)
 #pragma unroll 4
       for (int q = 0; q < cnt; ++q) {
-        const double2 s0 = *reinterpret_cast<const double2*>(&st[q][0]);
-        const double2 s1 = *reinterpret_cast<const double2*>(&st[q][2]);
         const double txyz = st[q][k1] * st[q][k2] * st[q][k3];
-        acc[0] = fma(s0.x, txyz, acc[0]);
-        acc[1] = fma(s0.y, txyz, acc[1]);
-        acc[2] = fma(s1.x, txyz, acc[2]);
-        acc[3] = fma(s1.y, txyz, acc[3]);
+        if constexpr (S == 1) {
+          acc[0] = fma(st[q][set0], txyz, acc[0]);
+        } else {
+          const double2 s0 = *reinterpret_cast<const double2*>(&st[q][0]);
+          const double2 s1 = *reinterpret_cast<const double2*>(&st[q][2]);
+          acc[0] = fma(s0.x, txyz, acc[0]);
+          acc[1] = fma(s0.y, txyz, acc[1]);
+          acc[2] = fma(s1.x, txyz, acc[2]);
+          acc[3] = fma(s1.y, txyz, acc[3]);
+        }
       }
   }
-  if (c < nchunk && term < NT)
+  if (c < nchunk && own)
 #pragma unroll
-    for (int set = 0; set < 4; ++set) mraw[((size_t)ch.w * 4 + set) * NT + term] = acc[set];
+    for (int k = 0; k < S; ++k) mraw[((size_t)ch.w * 4 + set0 + k) * NT + term] = acc[k];
 }
 
 // the 16 weighted sets (kk and der_cof, main.f90:358-399) in the order the far
@@ -559,13 +572,19 @@ void launch_moments(Handle& H, const double* x, bool f32, cudaStream_t s) {
   if (T.nmslot == 0) return;
   const int nch = T.mslot_chunk0.back() + T.mslot_nchunk.back();
   if (f32) {
-    using M = MomShape<P>;
-    {
+    auto partial = [&](auto sets) {
+      constexpr int S = decltype(sets)::value;
+      using M = MomShape<P, S>;
       TABI_K(K_MOMENTS, s);
-      mom_partial_kernel<P><<<ceil_div(nch, M::CPB), M::G * M::CPB, 0, s>>>(
+      mom_partial_kernel<P, S><<<ceil_div(nch, M::CPB), M::G * M::CPB, 0, s>>>(
           T.d_mchunks.p, nch, T.d_mslot_node.p, T.d_mid.p, H.d_x.p, H.d_y.p, H.d_z.p, H.d_nx.p,
           H.d_ny.p, H.d_nz.p, H.d_area.p, x, H.n, H.d_mraw.p);
+    };
+    const bool few = (int64_t)H.n * tabi_nterms(P) <= kMomFew;
+    if constexpr (P <= 5) {
+      if (few) partial(std::integral_constant<int, 1>());
     }
+    if (P > 5 || !few) partial(std::integral_constant<int, 4>());
     TABI_K(K_MOMENTS, s);
     mom_final_kernel<P><<<T.nmslot, 256, 0, s>>>(T.d_mslot_chunks.p, H.d_mraw.p, H.d_mwf.p);
     return;

@@ -43,6 +43,23 @@ def test_mixed_far_items(gpu_lib, order, level, leaf):
     assert np.linalg.norm(y32 - y) <= 2e-5 * np.linalg.norm(y)
 
 
+# orders whose Cartesian moments take one or four raw sets per thread: faces times
+# terms below and above 400,000
+@pytest.mark.parametrize("order", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("level", [2, 4, 5, 6])
+def test_mixed_moments(gpu_lib, order, level):
+    import tabipb
+
+    case = born_case(level, radius=6.0)
+    kw = dict(order=order, maxparnode=20 if level < 5 else 150, theta=0.7)
+    y = []
+    for prec in (tabipb.PREC_FP64, tabipb.PREC_MIXED):
+        with _solver(case, precision=prec, **kw)[0] as s:
+            x = np.random.default_rng(order).normal(size=2 * s.nface)
+            y.append(s.matvec(x))
+    assert np.linalg.norm(y[1] - y[0]) <= 2e-5 * np.linalg.norm(y[0])
+
+
 @pytest.mark.parametrize("order", [6, 8])
 def test_mixed_far_field_in_double(gpu_lib, order):
     """The FP64 residual of a small mixed solve takes one target per thread, the
