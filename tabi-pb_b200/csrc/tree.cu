@@ -672,11 +672,17 @@ void build_lists(Handle& H, cudaStream_t s) {
   const int far_chunk = kFarThreads * T.far_nt;
   // threads per target of the FP64 near field, as few as give every SM 8 blocks
   // of 128 threads: below that the SMs idle (1,272 targets: 49 us with one, 20
-  // with 16), above it more threads only stage the same leaf more often.  The
-  // FP32 one keeps a thread per target, and with it its summation order.
+  // with 16), above it more threads only stage the same leaf more often.  Once
+  // every SM has a block, a thread keeps 8 faces of the mean leaf: with less, the
+  // blocks only take the SMs from the far field beside them (operator apply,
+  // order 2, 1,098 faces in leaves of 20: 55 us with 8 threads, 43 with 2, 46
+  // before the split).  The FP32 one keeps a thread per target, and with it its
+  // summation order.
   T.near_split = 1;
   if (H.prm.precision == TABI_PREC_FP64)
-    while (T.near_split < 16 && tn * T.near_split < 148LL * 8 * 128) T.near_split *= 2;
+    while (T.near_split < 16 && tn * T.near_split < 148LL * 8 * 128 &&
+           (pairs >= 16 * T.near_split * tn || tn * T.near_split < 148LL * 128))
+      T.near_split *= 2;
   const int near_chunk = 128 / T.near_split;
   T.far_work.clear();
   T.near_work.clear();

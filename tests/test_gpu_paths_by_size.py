@@ -76,3 +76,55 @@ def test_mixed_far_field_in_double(gpu_lib, order):
         d = s.msolve(b - s.matvec(r["x"]))
         m = s.msolve(b)
     assert np.linalg.norm(d) <= 1.01e-9 * np.linalg.norm(m)
+
+
+def _near_lists(nodes, xyz, theta):
+    """(entries, entries times their leaf's faces, far interactions) of the lists."""
+    num, nchild, geo = nodes["numpar"], nodes["nchild"], nodes["geo"]
+    at, out = [0], [0, 0, 0]
+
+    def walk(t):  # the nodes come in the order of this walk
+        c = at[0]
+        at[0] += 1
+        far = np.zeros(len(t), bool)
+        if num[c] > 40 and len(t):
+            far = geo[c, 3] < np.sqrt(((geo[c, :3] - xyz[t]) ** 2).sum(1)) * theta
+        out[2] += int(far.sum())
+        t = t[~far]
+        if nchild[c] == 0:
+            out[0] += len(t)
+            out[1] += len(t) * int(num[c])
+        for _ in range(nchild[c]):
+            walk(t)
+
+    walk(np.arange(len(xyz)))
+    return out
+
+
+# threads per target of the FP64 near field (tree.cu, near_split), 1e-12 as in
+# test_gpu_matvec_paths.py: sums of the same terms in another order
+@pytest.mark.parametrize("level,leaf,theta,split", [
+    (3, 20, 0.8, 1), (5, 30, 0.8, 1), (3, 60, 0.7, 2), (5, 150, 0.8, 2), (4, 600, 0.8, 4),
+    (1, 7, 0.8, 8), (0, 20, 0.8, 16), (4, 1300, 0.8, 16)])
+def test_threads_per_near_target(gpu_lib, level, leaf, theta, split):
+    import oracle as O
+
+    case = born_case(level, radius=6.0)
+    s, g = _solver(case, maxparnode=leaf, theta=theta)
+    with s:
+        n, o = s.nface, s.orderarr - 1
+        tn, pairs, far = _near_lists(s.tree_nodes(), g[0][o], theta)
+        assert (pairs - n, far) == s.counts()
+        k = 1
+        while k < 16 and tn * k < 148 * 8 * 128 and (pairs >= 16 * k * tn or tn * k < 148 * 128):
+            k *= 2
+        assert k == split
+        x = np.random.default_rng(level).normal(size=2 * n)
+        y = s.unpermute(s.matvec(np.concatenate([x[:n][o], x[n:][o]])))
+    T = O.Tree(*g, 3, leaf, theta)
+    oo = T.orderarr - 1
+    yo = T.matvec(O.kappa(BULK, EPS1), EPS1 / EPS0, np.concatenate([x[:n][oo], x[n:][oo]]),
+                  nthreads=4)
+    ref = np.empty_like(yo)
+    ref[oo], ref[n + oo] = yo[:n], yo[n:]
+    assert np.linalg.norm(y - ref) <= 1e-12 * np.linalg.norm(ref)
