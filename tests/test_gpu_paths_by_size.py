@@ -128,3 +128,45 @@ def test_threads_per_near_target(gpu_lib, level, leaf, theta, split):
     ref = np.empty_like(yo)
     ref[oo], ref[n + oo] = yo[:n], yo[n:]
     assert np.linalg.norm(y - ref) <= 1e-12 * np.linalg.norm(ref)
+
+
+# one leaf around the near field's 256-face tile: a last tile of 255, 1, 44 and 1
+# faces, and the target's own face in it
+@pytest.mark.parametrize("faces", [255, 256, 257, 300, 513])
+def test_near_tiles(gpu_lib, faces):
+    import oracle as O
+
+    case = born_case(3, radius=6.0)
+    case["nvert"] = np.ascontiguousarray(case["nvert"][:faces])
+    s, g = _solver(case, maxparnode=600)
+    with s:
+        n, o = s.nface, s.orderarr - 1
+        assert n == faces and s.leaves()[1].size == 1
+        x = np.random.default_rng(faces).normal(size=2 * n)
+        y = s.unpermute(s.matvec(np.concatenate([x[:n][o], x[n:][o]])))
+    yo = O.matvec_direct(*g[:3], O.kappa(BULK, EPS1), EPS1 / EPS0, x)
+    assert np.linalg.norm(y - yo) <= 1e-12 * np.linalg.norm(yo)
+
+
+# blocks around the unpivoted factorisation's 16, 32, 64 and 128 columns: certified,
+# so the edges tested are its own and not the pivoted kernels'
+@pytest.mark.parametrize("faces", [2, 7, 8, 9, 15, 16, 17, 31, 32, 33, 63, 64, 65, 97, 129, 193,
+                                   320])
+def test_edges_are_certified(gpu_lib, faces):
+    import oracle as O
+
+    kappa = O.kappa(BULK, EPS1)
+    case = born_case(2, radius=3.0)
+    case["nvert"] = np.ascontiguousarray(case["nvert"][:faces])
+    s, g = _solver(case, iprcd=1, kappa=kappa)
+    with s:
+        n, o = s.nface, s.orderarr - 1
+        assert n == faces and s.pivoted_leaves() == 0
+        r = np.random.default_rng(faces).normal(size=2 * n)
+        z = s.unpermute(s.msolve(np.concatenate([r[:n][o], r[n:][o]])))
+    T = O.Tree(*g, 3, 500, 0.8)
+    oo = T.orderarr - 1
+    zt = T.msolve(kappa, EPS1 / EPS0, np.concatenate([r[:n][oo], r[n:][oo]]))
+    zo = np.empty_like(zt)
+    zo[oo], zo[n + oo] = zt[:n], zt[n:]
+    assert np.linalg.norm(z - zo) <= 1e-10 * np.linalg.norm(zo)
