@@ -357,8 +357,8 @@ __global__ void ws_node_kernel(int n, const float4* __restrict__ pos, const floa
 //   3: P = acc + bias, C = silu(P)
 //   4: P = P_in + acc, C = R + silu(P)  (second half of z = h Wb1 + a Wb2 + bb,
 //      P_in = h Wb1 + bb; R the residual input h)
-// A block takes 64 rows and 16 T columns -- all of them up to a width of 160 --
-// in 16-deep k steps, 4 x T outputs per thread (one 16-byte and T/2 8-byte shared
+// A block takes 64 rows and 16 T columns -- all of them up to a width of 160, where
+// there are rows enough -- in 16-deep k steps, 4 x T outputs per thread (one 16-byte and T/2 8-byte shared
 // loads for 4 T multiply-adds), the next step's operands in registers
 // meanwhile; three blocks per SM where the epilogue reads two more matrices,
 // else two with the accumulators' registers unspilled.  Each output is one
@@ -927,7 +927,11 @@ void with_tile(int N, F&& f) {
 template <bool TB, int EPI>
 void gemm(int M, int N, int Kd, const float* A, int lda, const __nv_bfloat16* W, int ldw,
           const float* bias, float* C, int ldc, float* P, const float* R, cudaStream_t s) {
-  with_tile(N, [&](auto t) {
+  // the widest column blocks whose grid gives every SM one: all columns from 148
+  // blocks of rows on, 64 from 37, else 32 (a prediction at H = 160: 1,112 panels 637,
+  // 528 and 511 us, 5,436 panels 696, 636 and 639; 597 and 689 with 64 x 64 tiles)
+  const int rows = ceil_div(M, kGM);
+  with_tile(rows >= 148 ? N : rows >= 37 ? std::min(N, 64) : 32, [&](auto t) {
     constexpr int T = decltype(t)::value;
     dim3 grid(ceil_div(M, kGM), ceil_div(N, 16 * T));
     ws_gemm_kernel<T, TB, EPI><<<grid, 256, 0, s>>>(M, N, Kd, A, lda, W, ldw, bias, C, ldc, P,
