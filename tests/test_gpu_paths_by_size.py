@@ -170,3 +170,42 @@ def test_edges_are_certified(gpu_lib, faces):
     zo = np.empty_like(zt)
     zo[oo], zo[n + oo] = zt[:n], zt[n:]
     assert np.linalg.norm(z - zo) <= 1e-10 * np.linalg.norm(zo)
+
+
+# the network's products in column blocks of 64 (80 blocks of 64 panels) and of all or
+# half the columns (320); blocks of 32 are test_gpu_kernel_edges.py's.  Bars as there.
+@pytest.mark.parametrize("level,hidden", [(4, 32), (4, 96), (4, 160), (4, 256), (5, 32), (5, 96),
+                                          (5, 160), (5, 224)])
+def test_network_products(gpu_lib, level, hidden):
+    import torch
+    import warmstart_ref as W
+
+    import oracle as O
+    from tabipb.warmstart import WarmStart
+
+    c = born_case(level, radius=3.0)
+    xyz, tq, ar, b = O.form_matrix(c["sptpos"], c["sptnrm"], c["nvert"], c["chrpos"] + 0.4,
+                                   c["atmchr"], 1.0)
+    rng = np.random.default_rng(hidden)
+    x = b * 0.3 + rng.standard_normal(b.size) * np.std(b) * 0.1
+    z = b * 0.25 + rng.standard_normal(b.size) * np.std(b) * 0.05
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a, dtype=np.float64).ravel()).cuda()
+    s = dict(n=len(ar), xyz=t(xyz), tq=t(tq), area=t(ar), b=t(b), z=t(z), x=t(x))
+    ws = WarmStart(hidden=hidden, layers=1, seed=0)
+    theta = W.init_params(hidden, 1, 8, seed=4)
+    ws.set_params(theta)
+    nbr = ws.graph_dev(s)[0].astype(np.int64)
+    xr, loss_ref, cache = W.forward(theta, hidden, 1, 8, xyz.reshape(-1, 3), tq.reshape(-1, 3), ar,
+                                    b, nbr, target=x, z=z)
+    g_ref = W.backward(cache, hidden, 1, 8, nbr)
+    loss, g = ws.loss_grad_dev(s)
+    assert abs(loss - loss_ref) <= 1e-4 * abs(loss_ref)
+    o = 0
+    for name, shp in W.param_shapes(hidden, 1, 8):
+        k = int(np.prod(shp))
+        d = np.abs(g[o:o + k] - g_ref[o:o + k]).max()
+        assert d <= 2e-3 * (np.abs(g_ref[o:o + k]).max() + 1e-30), name
+        o += k
+    xp = torch.empty_like(s["b"])
+    ws.predict_dev(s, xp)
+    assert np.linalg.norm(xp.cpu().numpy() - xr) <= 5e-4 * np.linalg.norm(xr)
