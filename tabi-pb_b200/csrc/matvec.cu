@@ -913,7 +913,7 @@ void set_target_range(Handle& H, int t0, int t1, cudaStream_t s) {
   std::vector<int> big, small;
   for (int l = 0; l < T.nleaf; ++l) {
     const int c = T.leaves[l], b0 = T.ibeg[c], nm = T.num[c];
-    if (b0 >= t0 && b0 + nm <= t1) (2 * nm > 512 ? big : small).push_back(l);
+    if (b0 >= t0 && b0 + nm <= t1) (2 * nm > kSolveSmall ? big : small).push_back(l);
   }
   auto by_size = [&](int a, int b) { return T.num[T.leaves[a]] > T.num[T.leaves[b]]; };
   std::sort(big.begin(), big.end(), by_size);

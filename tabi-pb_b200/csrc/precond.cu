@@ -1109,13 +1109,11 @@ __global__ void lu_diaginv_kernel(const int2* __restrict__ blocks,  // (leaf, k0
 // order 6,912.  The others: one group and five tiles, so that three CTAs share
 // an SM (two CTAs with six tiles: 383 instead of 375 us for 807,640 unknowns in
 // blocks of ~300).  Taking two or three tiles per wait keeps fewer in flight: 607
-// and 643 instead of 573 us at order 2,464 (623 before), 170 and 174 instead of
-// 166 us for 800 MB.  Above order ~5,000 the chain's one SM is slower than the
-// form before, whose 512 threads kept 131 KB in flight (order 5,818: 2.97
-// against 2.81 ms, beside a factorisation of 131 GFLOP).
+// and 643 instead of 573 us at order 2,464 with L2 flushed (623 before), 170 and
+// 174 instead of 166 us for 800 MB.  Blocks whose factors stay in L2, or of an odd
+// number of faces each: solve_rows_kernel.
 constexpr int kTile = kDB * kDB, kDRing = 3, kRingBig = 9, kRingSmall = 5;
 constexpr int kRingHuge = 6, kSolveHuge = 6912;  // blocks above this order
-constexpr int kSolveSmall = 512;     // largest order of the lists' small class
 constexpr int kMaxSolveLeaf = 5760;  // faces
 
 // threads and shared memory of solve_kernel<G, RING> for a block of the given order
@@ -1292,6 +1290,151 @@ __global__ void __launch_bounds__(solve_threads(G), (G == 1 ? 3 : 1)) solve_kern
   for (int i = tid; i < n; i += solve_threads(G)) {
     z[ib + i] = vec[i];
     z[N + ib + i] = vec[n + i];
+  }
+}
+
+// The same substitution with the factors read where they are used: per step the first
+// warp forms y_t = Dinv r_t, and 512 threads update the rows below (above) with the
+// step's 32 columns, each thread a row, the first row's values loaded while y_t is
+// formed.  Every step's loads wait for its barrier, but a 32 x 32 tile costs a fifth
+// of the streamed form's instructions, which bound that form once the factors come
+// from L2, and its loads are whole rows of columns, where the streamed 16-byte
+// copies straddle sectors in the columns of an odd number of faces.  Per apply, this
+// form and the streamed one: blocks of up to 530 unknowns, 8 MB in all, 37 and 41 us;
+// up to 938, 24 MB, 91 and 101; up to 1,598, 59 MB, 239 and 250; one of 2,464, 48 MB,
+// 426 and 479; up to 1,250, 69 MB, 147 and 166; up to 858, 93 MB, 105 and 86.  One
+// block of an odd number of faces: order 3,502 984 and 1,110 us, 5,818 2,844 and
+// 2,957, 7,002 3,973 and 4,275, 8,002 5,774 and 5,590; of an even number: 3,500
+// 985 and 947.
+constexpr int kRowThreads = 512;
+constexpr int64_t kRowBytes = 68 << 20;  // factors that stay in L2 between applies
+constexpr int kRowOrder = 7500;          // blocks of odd face counts
+constexpr size_t row_bytes(int order) {
+  return sizeof(double) * (2 * (size_t)order + kDB + 2 * kTile);
+}
+
+__global__ void __launch_bounds__(kRowThreads, 1) solve_rows_kernel(
+    const int2* __restrict__ leaf_rng, const int64_t* __restrict__ blk_off,
+    const int64_t* __restrict__ dinv_off, const int* __restrict__ leaf_list,
+    const double* __restrict__ lu, const double* __restrict__ dinv,
+    const int* __restrict__ perm, int N, const double* __restrict__ r,
+    double* __restrict__ z) {
+  extern __shared__ __align__(16) double sm[];
+  int leaf = leaf_list[blockIdx.x];
+  int2 lr = leaf_rng[leaf];
+  const int n = lr.y, m = 2 * n, ib = lr.x;
+  double* xs = sm;             // forward sweep: running; backward: results
+  double* fin = sm + m;        // forward sweep: results; backward: running
+  double* ys = sm + 2 * m;     // [32] the step's y
+  const double* A = lu + blk_off[leaf];
+  const double* Di = dinv + dinv_off[leaf];
+  const int* pm = perm + 2 * ib;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int i = tid; i < m; i += kRowThreads) {
+    int src = pm[i];
+    xs[i] = (src < n) ? r[ib + src] : r[N + ib + src - n];
+  }
+  // the inverse diagonal block of sweep step t (L blocks 0..nblk-1, then U
+  // blocks nblk-1..0), staged into shared memory one step ahead by cp.async
+  const int nblk = (m + kDB - 1) / kDB;
+  double* dbuf = ys + kDB;  // [2][kDB * kDB]
+  auto stage = [&](int t, int buf) {
+    if (t >= 2 * nblk) return;
+    const int b = t < nblk ? t : 2 * nblk - 1 - t;
+    const double* src = Di + (size_t)b * 2 * kDB * kDB + (t < nblk ? 0 : kDB * kDB);
+    for (int e = 2 * tid; e < kDB * kDB; e += 2 * kRowThreads) {
+      const unsigned d = (unsigned)__cvta_generic_to_shared(dbuf + buf * kDB * kDB + e);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src + e));
+    }
+    asm volatile("cp.async.commit_group;\n" ::);
+  };
+  // step t: y = Dinv * run[k0 .. k0+nb), res[k0 ..] = y, run[i] -= A[i, k0 ..
+  // k0+nb) y for the rows [i0, i1); the next step's block is copied while the
+  // rows are updated.  Four partial sums per dot product keep the dependent
+  // FMA chains 8 deep.
+  // y = Dinv * run[k0 .. k0+nb) for lane `lane`, four partial sums
+  auto diag = [&](int t, int k0, int nb, const double* run) {
+    const double* Dblk = dbuf + (t & 1) * kDB * kDB;
+    double v0 = 0.0, v1 = 0.0, v2 = 0.0, v3 = 0.0;
+    if (nb == kDB) {  // run + k0 is 16-byte aligned: paired loads
+      const double2* r2 = reinterpret_cast<const double2*>(run + k0);
+#pragma unroll
+      for (int q = 0; q < kDB; q += 4) {
+        const double2 ra = r2[q / 2], rb = r2[q / 2 + 1];
+        v0 = fma(Dblk[q * kDB + lane], ra.x, v0);
+        v1 = fma(Dblk[(q + 1) * kDB + lane], ra.y, v1);
+        v2 = fma(Dblk[(q + 2) * kDB + lane], rb.x, v2);
+        v3 = fma(Dblk[(q + 3) * kDB + lane], rb.y, v3);
+      }
+    } else {
+      for (int q = 0; q < nb; ++q) v0 = fma(Dblk[q * kDB + lane], run[k0 + q], v0);
+    }
+    return (v0 + v1) + (v2 + v3);
+  };
+  // run[i] -= A[i, k0 .. k0+nb) y for row i, tq preloaded when `have`
+  auto row = [&](int k0, int nb, int i, const double* y, double (&tq)[kDB], bool have,
+                 double* run) {
+    const double* a = A + (size_t)k0 * m + i;
+    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+    if (nb == kDB) {
+      if (!have) {
+#pragma unroll
+        for (int q = 0; q < kDB; ++q) tq[q] = a[(size_t)q * m];
+      }
+      const double2* y2 = reinterpret_cast<const double2*>(y);
+#pragma unroll
+      for (int q = 0; q < kDB; q += 4) {
+        const double2 ya = y2[q / 2], yb = y2[q / 2 + 1];
+        s0 = fma(tq[q], ya.x, s0);
+        s1 = fma(tq[q + 1], ya.y, s1);
+        s2 = fma(tq[q + 2], yb.x, s2);
+        s3 = fma(tq[q + 3], yb.y, s3);
+      }
+    } else {
+      for (int q = 0; q < nb; ++q) s0 = fma(a[(size_t)q * m], y[q], s0);
+    }
+    run[i] -= (s0 + s1) + (s2 + s3);
+  };
+  auto step = [&](int t, int k0, int nb, double* run, double* res, int i0, int i1) {
+    double tq[kDB];
+    // warp 0 forms y and shares it through shared memory (one more barrier,
+    // against 16 warps each reading the 8 KB block); the first row's panel
+    // values are loaded meanwhile
+    const int ifirst = i0 + tid;
+    const bool pre = ifirst < i1 && nb == kDB;
+    if (pre) {
+      const double* a = A + (size_t)k0 * m + ifirst;
+#pragma unroll
+      for (int q = 0; q < kDB; ++q) tq[q] = a[(size_t)q * m];
+    }
+    if (warp == 0) {
+      const double v = diag(t, k0, nb, run);
+      ys[lane] = v;
+      if (lane < nb) res[k0 + lane] = v;
+    }
+    stage(t + 1, (t + 1) & 1);
+    __syncthreads();
+    for (int i = ifirst; i < i1; i += kRowThreads) row(k0, nb, i, ys, tq, pre && i == ifirst, run);
+    asm volatile("cp.async.wait_group 0;\n" ::);
+    __syncthreads();
+  };
+  stage(0, 0);
+  asm volatile("cp.async.wait_group 0;\n" ::);
+  __syncthreads();
+  // L y = P r: running values in xs, y in fin
+  for (int k0 = 0, t = 0; k0 < m; k0 += kDB, ++t) {
+    const int nb = min(kDB, m - k0);
+    step(t, k0, nb, xs, fin, k0 + nb, m);
+  }
+  // U x = y: running values in fin, x in xs
+  for (int b = nblk - 1, t = nblk; b >= 0; --b, ++t) {
+    const int k0 = b * kDB;
+    const int nb = min(kDB, m - k0);
+    step(t, k0, nb, fin, xs, 0, k0);
+  }
+  for (int i = tid; i < n; i += kRowThreads) {
+    z[ib + i] = xs[i];
+    z[N + ib + i] = xs[n + i];
   }
 }
 
@@ -2016,11 +2159,20 @@ void build_precond(Handle& H, cudaStream_t s) {
   launch_assemble(H, d_tiles.p, (int)tiles.len, s);
   TABI_CUDA(cudaMemsetAsync(d_info.p, 0, sizeof(int) * nl, s));
   // apply lists (they depend on the leaf sizes only, so they are built while
-  // the assembly runs): blocks of order > 512 get two groups of warps, the others
-  // one group, on the side stream (see solve_kernel); largest first in each
+  // the assembly runs): blocks of order > kSolveSmall and the others, on the side
+  // stream (see solve_kernel); largest first in each
   {
     std::vector<int> big, small;
-    for (int l = 0; l < nl; ++l) (2 * rng[l].y > 512 ? big : small).push_back(l);
+    for (int l = 0; l < nl; ++l) (2 * rng[l].y > kSolveSmall ? big : small).push_back(l);
+    int64_t bytes = 0;
+    int order = 0;
+    bool odd = true;
+    for (int l : big) {
+      bytes += (int64_t)sizeof(double) * 4 * rng[l].y * rng[l].y;
+      order = std::max(order, 2 * rng[l].y);
+      odd &= (rng[l].y & 1) != 0;
+    }
+    T.solve_rows = bytes <= kRowBytes || (odd && order <= kRowOrder);
     std::sort(big.begin(), big.end(), [&](int a, int b) { return rng[a].y > rng[b].y; });
     std::sort(small.begin(), small.end(), [&](int a, int b) { return rng[a].y > rng[b].y; });
     T.n_solve_big = (int)big.size();
@@ -2508,21 +2660,25 @@ void msolve_dev(Handle& H, const double* r, double* z, cudaStream_t s) {
     TABI_CUDA(cudaEventRecord(H.ev_fork, s));
     TABI_CUDA(cudaStreamWaitEvent(s2, H.ev_fork, 0));
   }
-  auto launch = [&](auto* kernel, int G, size_t smem, int count, const int* leaves,
+  auto launch = [&](auto* kernel, int threads, size_t smem, int count, const int* leaves,
                     cudaStream_t st) {
     if (count == 0) return;
     raise_smem_limit((const void*)kernel, smem);
     TABI_K(K_SOLVE, st);
-    kernel<<<count, solve_threads(G), smem, st>>>(T.d_leaf_rng.p, T.d_blk_off.p, T.d_dinv_off.p,
+    kernel<<<count, threads, smem, st>>>(T.d_leaf_rng.p, T.d_blk_off.p, T.d_dinv_off.p,
                                                   leaves, T.d_lu.p, T.d_dinv.p, T.d_lu_perm.p, n,
                                                   r, z);
   };
   const int order = 2 * T.max_leaf;
-  if (order <= kSolveHuge)
-    launch(solve_kernel<2, kRingBig>, 2, solve_bytes(2, kRingBig, order), nbig, list, s);
+  if (T.solve_rows)
+    launch(solve_rows_kernel, kRowThreads, row_bytes(order), nbig, list, s);
+  else if (order <= kSolveHuge)
+    launch(solve_kernel<2, kRingBig>, solve_threads(2), solve_bytes(2, kRingBig, order), nbig,
+           list, s);
   else  // the vector (92 KB for the largest leaf) leaves room for fewer tiles
-    launch(solve_kernel<2, kRingHuge>, 2, solve_bytes(2, kRingHuge, order), nbig, list, s);
-  launch(solve_kernel<1, kRingSmall>, 1,
+    launch(solve_kernel<2, kRingHuge>, solve_threads(2), solve_bytes(2, kRingHuge, order), nbig,
+           list, s);
+  launch(solve_kernel<1, kRingSmall>, solve_threads(1),
          solve_bytes(1, kRingSmall, std::min(order, kSolveSmall)), nsmall, list + nbig, s2);
   if (fork) {
     TABI_CUDA(cudaEventRecord(H.ev_join, s2));

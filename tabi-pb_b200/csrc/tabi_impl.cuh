@@ -204,6 +204,9 @@ struct PinVec {
 constexpr int kFarThreads = 64;
 __host__ __device__ constexpr int far_pair(int order) { return order >= 6 ? 2 : 1; }
 
+// largest order of a leaf block in the preconditioner apply's small class
+constexpr int kSolveSmall = 512;
+
 // Work item of the interaction kernels: node and a chunk of its entry list.
 struct WorkItem {
   int node;
@@ -272,6 +275,7 @@ struct Tree {
   DBuf<double> d_dinv;           // per 32-row block: L^{-1}, U^{-1} (32 x 32 each)
   DBuf<int> d_lu_perm;           // per leaf row permutation of all pivots
   int n_solve_big = 0, n_solve_small = 0;
+  bool solve_rows = false;  // the big ones by solve_rows_kernel
   int max_leaf = 0;
   // mixed precision: leaf ids on the device; each face relative to its leaf
   // centre as FP32 hi + lo (with its area in lpos.w) and its normal in FP32

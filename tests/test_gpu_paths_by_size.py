@@ -209,3 +209,38 @@ def test_network_products(gpu_lib, level, hidden):
     xp = torch.empty_like(s["b"])
     ws.predict_dev(s, xp)
     assert np.linalg.norm(xp.cpu().numpy() - xr) <= 5e-4 * np.linalg.norm(xr)
+
+
+# one block of order > 512: the row form (factors below 64 MB, or an odd number of
+# faces up to order 7,500) and the streamed one, full and partial last steps.  B z = r
+# with B as LEAFMATVECpara assembles it, as in test_gpu_kernel_edges.py.
+@pytest.mark.parametrize("faces", [257, 272, 399, 416, 1447, 1448, 1450, 1456, 1465, 3749, 3751])
+def test_forms_of_the_block_apply(gpu_lib, faces):
+    kappa, eps = 0.1257, EPS1 / EPS0
+    case = born_case(4, radius=6.0)
+    case["nvert"] = np.ascontiguousarray(case["nvert"][:faces])
+    s, g = _solver(case, kappa=kappa, iprcd=1, maxparnode=4000)
+    with s:
+        n, o = s.nface, s.orderarr - 1
+        assert n == faces and s.leaves()[1].size == 1
+        r = np.random.default_rng(faces).normal(size=2 * n)
+        z = s.msolve(r)
+        xyz, nrm, ar = (np.asarray(v).reshape(n, -1)[o] for v in g[:3])
+    for i in range(0, n, 500):
+        j = min(n, i + 500)
+        d = xyz[None] - xyz[i:j, None]
+        rs = np.sqrt((d ** 2).sum(-1))
+        own = rs == 0
+        rs[own] = 1.0
+        g0, e = 1 / (4 * np.pi * rs), np.exp(-kappa * rs)
+        v, v0 = nrm[None], nrm[i:j, None]
+        c, c0, vv = (v * d).sum(-1) / rs, (v0 * d).sum(-1) / rs, (v * v0).sum(-1)
+        t1, t2 = g0 / rs, (1 + kappa * rs) * e
+        g3 = (vv - 3 * c0 * c) / rs * t1
+        k1, k2 = c * t1 * (1 - eps * t2), g0 * (1 - e)
+        k3, k4 = g3 * (t2 - 1) - kappa ** 2 * c0 * c * e * g0, c0 * t1 * (1 - t2 / eps)
+        a = np.where(own, 0.0, ar.ravel()[None])
+        y1 = .5 * (1 + eps) * z[i:j] - (k1 * a) @ z[:n] - (k3 * a) @ z[n:]
+        y2 = .5 * (1 + 1 / eps) * z[n + i:n + j] - (k2 * a) @ z[:n] - (k4 * a) @ z[n:]
+        assert np.abs(y1 - r[i:j]).max() <= 1e-10
+        assert np.abs(y2 - r[n + i:n + j]).max() <= 1e-10
