@@ -204,6 +204,8 @@ struct PinVec {
 constexpr int kFarThreads = 64;
 __host__ __device__ constexpr int far_pair(int order) { return order >= 6 ? 2 : 1; }
 
+constexpr int kSMs = 148;  // B200
+
 // largest order of a leaf block in the preconditioner apply's small class
 constexpr int kSolveSmall = 512;
 

@@ -680,8 +680,8 @@ void build_lists(Handle& H, cudaStream_t s) {
   // summation order.
   T.near_split = 1;
   if (H.prm.precision == TABI_PREC_FP64)
-    while (T.near_split < 16 && tn * T.near_split < 148LL * 8 * 128 &&
-           (pairs >= 16 * T.near_split * tn || tn * T.near_split < 148LL * 128))
+    while (T.near_split < 16 && tn * T.near_split < 8LL * kSMs * 128 &&
+           (pairs >= 16 * T.near_split * tn || tn * T.near_split < kSMs * 128LL))
       T.near_split *= 2;
   const int near_chunk = 128 / T.near_split;
   T.far_work.clear();

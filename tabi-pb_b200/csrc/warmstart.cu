@@ -931,7 +931,7 @@ void gemm(int M, int N, int Kd, const float* A, int lda, const __nv_bfloat16* W,
   // blocks of rows on, 64 from 37, else 32 (a prediction at H = 160: 1,112 panels 637,
   // 528 and 511 us, 5,436 panels 696, 636 and 639; 597 and 689 with 64 x 64 tiles)
   const int rows = ceil_div(M, kGM);
-  with_tile(rows >= 148 ? N : rows >= 37 ? std::min(N, 64) : 32, [&](auto t) {
+  with_tile(rows >= kSMs ? N : rows >= kSMs / 4 ? std::min(N, 64) : 32, [&](auto t) {
     constexpr int T = decltype(t)::value;
     dim3 grid(ceil_div(M, kGM), ceil_div(N, 16 * T));
     ws_gemm_kernel<T, TB, EPI><<<grid, 256, 0, s>>>(M, N, Kd, A, lda, W, ldw, bias, C, ldc, P,
@@ -1106,8 +1106,8 @@ void WsNet::graph(const WsInput& in, cudaStream_t s) {
 }
 
 void WsNet::dw(int M, int Kd, int N, const float* A, const float* D, float* g, cudaStream_t s) {
-  // rows per chunk: two blocks for each of 148 SMs, between 64 and 1,024
-  const int chunk = std::min(1024, std::max(64, ceil_div(ceil_div(M, 296), kGK) * kGK));
+  // rows per chunk: two blocks for each SM, between 64 and 1,024
+  const int chunk = std::min(1024, std::max(64, ceil_div(ceil_div(M, 2 * kSMs), kGK) * kGK));
   const int nch = ceil_div(M, chunk);
   part.alloc((size_t)nch * Kd * N);
   auto launch = [&](auto t) {
