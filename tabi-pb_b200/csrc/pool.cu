@@ -43,6 +43,7 @@ namespace {
 // per context: device blocks and page-locked blocks kept, resource bundles kept
 constexpr size_t kMaxDevice = size_t(4) << 30, kMaxPinned = size_t(256) << 20;
 constexpr size_t kMaxRes = 16;
+constexpr size_t kMaxStep = size_t(32) << 20;  // largest rounding of a block's size
 
 thread_local int tl_idle = 0;
 
@@ -95,9 +96,11 @@ MemPool::Block MemPool::get(size_t bytes, bool pinned) {
       return b;
     }
   }
-  // sizes in steps of an eighth of their magnitude, so that they meet again
+  // sizes in steps of an eighth of their magnitude, so that they meet again, but of
+  // at most 32 MiB: a large molecule's blocks together must not outgrow the memory
+  // that their exact sizes would fit
   size_t step = 4096;
-  while (16 * step < bytes) step *= 2;
+  while (16 * step < bytes && step < kMaxStep) step *= 2;
   b.bytes = (bytes + step - 1) / step * step;
   auto alloc = [&] {
     return pinned ? cudaMallocHost(&b.p, b.bytes) : cudaMalloc(&b.p, b.bytes);

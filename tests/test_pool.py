@@ -140,6 +140,14 @@ int main() {
   cur = first;
   CHECK(MemPool::get(MB, false).p == b.p);
   MemPool::put(b);
+  // a large block is rounded up by little: ten of them fit where their sizes do
+  MemPool::release();
+  limit = used + 10 * (size_t(17) * GB + 32 * MB);
+  v.clear();
+  for (int k = 0; k < 10; ++k) v.push_back(MemPool::get(17 * GB + 8 * k + 1, false));
+  for (auto& x : v) CHECK(x.bytes <= 17 * GB + 32 * MB);
+  for (auto& x : v) MemPool::put(x);
+  limit = 64 * GB;
   // bundles of streams and events: the last one back is the next one out
   HandleRes r = HandleRes::get();
   const int n = objects;
