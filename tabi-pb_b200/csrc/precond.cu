@@ -1110,8 +1110,8 @@ __global__ void lu_diaginv_kernel(const int2* __restrict__ blocks,  // (leaf, k0
 // an SM (two CTAs with six tiles: 383 instead of 375 us for 807,640 unknowns in
 // blocks of ~300).  Taking two or three tiles per wait keeps fewer in flight: 607
 // and 643 instead of 573 us at order 2,464 with L2 flushed (623 before), 170 and
-// 174 instead of 166 us for 800 MB.  Blocks whose factors stay in L2, or of an odd
-// number of faces each: solve_rows_kernel.
+// 174 instead of 166 us for 800 MB.  Blocks whose factors stay in L2, and lone ones
+// of an odd number of faces: solve_rows_kernel.
 constexpr int kTile = kDB * kDB, kDRing = 3, kRingBig = 9, kRingSmall = 5;
 constexpr int kRingHuge = 6, kSolveHuge = 6912;  // blocks above this order
 constexpr int kMaxSolveLeaf = 5760;  // faces
@@ -1299,16 +1299,21 @@ __global__ void __launch_bounds__(solve_threads(G), (G == 1 ? 3 : 1)) solve_kern
 // formed.  Every step's loads wait for its barrier, but a 32 x 32 tile costs a fifth
 // of the streamed form's instructions, which bound that form once the factors come
 // from L2, and its loads are whole rows of columns, where the streamed 16-byte
-// copies straddle sectors in the columns of an odd number of faces.  Per apply, this
-// form and the streamed one: blocks of up to 530 unknowns, 8 MB in all, 37 and 41 us;
-// up to 938, 24 MB, 91 and 101; up to 1,598, 59 MB, 239 and 250; one of 2,464, 48 MB,
-// 426 and 479; up to 1,250, 69 MB, 147 and 166; up to 858, 93 MB, 105 and 86.  One
-// block of an odd number of faces: order 3,502 984 and 1,110 us, 5,818 2,844 and
-// 2,957, 7,002 3,973 and 4,275, 8,002 5,774 and 5,590; of an even number: 3,500
-// 985 and 947.
+// copies straddle sectors in the columns of an odd number of faces.
+//
+// Taken where the factors of all leaves stay in L2 even beside two more handles at
+// work (kRowBytes), us per apply of this form and the streamed one, one handle and
+// three in turn: 10 MB in blocks of up to 558 unknowns 41.4, 44.5 and 14.8, 15.5;
+// 20 MB, one block of 978, 97, 106 and 35.4, 36.3; not at 25 MB, blocks up to 754,
+// 66, 69 and 31, 25; 39 MB, up to 844, 76, 78 and 37, 29; 96 MB, up to 664, 75, 55
+// and 36, 28.  And for a lone block (there is nothing beside it to fill an SM) up to
+// kLoneBytes, order 2,000 302, 333 and 121, 113, 2,464 427, 478 and 189, 162, or of an
+// odd number of faces up to kLoneOrder: order 2,502 476, 587 and 206, 199; 3,502
+// 991, 1,111 and 372, 372; 7,002 4,040, 4,287 and 1,339, 1,428; beyond, 8,002 5,774,
+// 5,590; an even number, 2,900 680, 661 and 266, 222.
 constexpr int kRowThreads = 512;
-constexpr int64_t kRowBytes = 68 << 20;  // factors that stay in L2 between applies
-constexpr int kRowOrder = 7500;          // blocks of odd face counts
+constexpr int64_t kRowBytes = 20 << 20, kLoneBytes = 56 << 20;
+constexpr int kLoneOrder = 7500;
 constexpr size_t row_bytes(int order) {
   return sizeof(double) * (2 * (size_t)order + kDB + 2 * kTile);
 }
@@ -2164,15 +2169,9 @@ void build_precond(Handle& H, cudaStream_t s) {
   {
     std::vector<int> big, small;
     for (int l = 0; l < nl; ++l) (2 * rng[l].y > kSolveSmall ? big : small).push_back(l);
-    int64_t bytes = 0;
-    int order = 0;
-    bool odd = true;
-    for (int l : big) {
-      bytes += (int64_t)sizeof(double) * 4 * rng[l].y * rng[l].y;
-      order = std::max(order, 2 * rng[l].y);
-      odd &= (rng[l].y & 1) != 0;
-    }
-    T.solve_rows = bytes <= kRowBytes || (odd && order <= kRowOrder);
+    const int64_t bytes = (int64_t)sizeof(double) * off;  // of all factors
+    T.solve_rows = nl > 1 ? bytes <= kRowBytes
+                          : bytes <= kLoneBytes || (rng[0].y % 2 && 2 * rng[0].y <= kLoneOrder);
     std::sort(big.begin(), big.end(), [&](int a, int b) { return rng[a].y > rng[b].y; });
     std::sort(small.begin(), small.end(), [&](int a, int b) { return rng[a].y > rng[b].y; });
     T.n_solve_big = (int)big.size();

@@ -211,10 +211,10 @@ def test_network_products(gpu_lib, level, hidden):
     assert np.linalg.norm(xp.cpu().numpy() - xr) <= 5e-4 * np.linalg.norm(xr)
 
 
-# one block of order > 512: the row form (factors below 64 MB, or an odd number of
+# one block of order > 512: the row form (factors up to 56 MiB, or an odd number of
 # faces up to order 7,500) and the streamed one, full and partial last steps.  B z = r
 # with B as LEAFMATVECpara assembles it, as in test_gpu_kernel_edges.py.
-@pytest.mark.parametrize("faces", [257, 272, 399, 416, 1447, 1448, 1450, 1456, 1465, 3749, 3751])
+@pytest.mark.parametrize("faces", [257, 272, 399, 416, 1354, 1356, 1447, 1448, 1450, 1456, 3749, 3751])
 def test_forms_of_the_block_apply(gpu_lib, faces):
     kappa, eps = 0.1257, EPS1 / EPS0
     case = born_case(4, radius=6.0)
